@@ -41,7 +41,7 @@ def reference_lib():
     on a host without them the prebuilt library that travelled with the tree is used."""
     so = os.path.join(ORACLE, "_ref", "libapcref.so")
     if not os.path.exists(so):
-        if not os.path.isdir(REFERENCE_SRC):
+        if not os.path.exists(os.path.join(REFERENCE_SRC, "octree.cpp")):
             pytest.skip("reference sources and prebuilt oracle/_ref both absent")
         _make("ref")
     return so
