@@ -84,6 +84,7 @@ template int apc_ensure<float>(apc_context *, float **, size_t, size_t *);
 template int apc_ensure<int>(apc_context *, int **, size_t, size_t *);
 template int apc_ensure<uint32_t>(apc_context *, uint32_t **, size_t, size_t *);
 template int apc_ensure<uint64_t>(apc_context *, uint64_t **, size_t, size_t *);
+template int apc_ensure<unsigned char>(apc_context *, unsigned char **, size_t, size_t *);
 
 int apc_read_errors(apc_context *c, int *flags) {
   APC_CUDA_TRY(c, cudaMemcpyAsync(c->h_pinned + 1, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->s));

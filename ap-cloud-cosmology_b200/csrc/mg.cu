@@ -20,8 +20,8 @@
 //     Rows sum to zero except the Dirichlet pin's aggregate, so the constant mode is
 //     reproduced exactly on every level.
 //   * Damped Jacobi smoothing on ELL operators, over-scaled coarse corrections; the
-//     levels of <= 1024 nodes in one single-block kernel; an explicit dense inverse (FP64,
-//     formed on the host) on the coarsest level of <= 64 nodes.
+//     coarse levels on one thread-block cluster; an explicit dense inverse (formed in
+//     FP64) on the coarsest level of <= 64 nodes.
 //   * Flexible GMRES with classical Gram-Schmidt (optionally a second, re-orthogonalising
 //     sweep), right preconditioned, so the residual it monitors is the true residual of
 //     the correction equation.  The SpMV is fused with the first dot-product pass.  The
@@ -935,15 +935,10 @@ static inline int tail_lanes(int n, int w, int threads) {
   return g;
 }
 
-// the graph path's tail kernel: 512 threads leave 128 registers a thread for the batched
+// the graph path's tail kernel, for levels that do not fit the cluster kernel's shared
+// memory (rows of hundreds of slots): 512 threads leave 128 registers a thread for the batched
 // row loads (a 1024-thread block has 64)
 constexpr int kTailThreads = 512;
-// the staged tail: its loads hit shared memory, so short batches suffice and the block can
-// take 1024 threads (64 registers), one round for levels of up to 1024 rows
-constexpr int kTailSmemThreads = 1024;
-template <class V>
-constexpr int kTailSmemBatch = 4;
-
 // sum_j a_ij xj(j) for every row of a tail level, L.g lanes per row; emit(i, sum) runs on
 // the group's first lane.  The trip count is the same for the whole block (shuffles).
 template <class V, int B, class XJ, class F>
@@ -1069,128 +1064,357 @@ __global__ void __launch_bounds__(kTailThreads) vcycle_tail(TailArgs<V> A) {
   tail_body<V, RowBatch<V>::n>(A);
 }
 
-constexpr size_t kTailSmemMax = 227 * 1024;  // dynamic shared memory a block may opt into
+constexpr size_t kSmemMax = 227 * 1024;  // dynamic shared memory a block may opt into
 
-// The tail with every level staged in shared memory (the levels are constant for a solve
-// and, at a few hundred rows, take tens of KB): each launch copies the tail's matrices,
-// maps and the first level's right-hand side in, runs the same body on the copies, and
-// writes the first level's solution back.  Staging turns each phase's gathers from L2
-// round trips into shared-memory loads.  The layout is tail_smem_bytes's.
-__host__ __device__ inline size_t tail_align(size_t b) { return (b + 15) & ~(size_t)15; }
-
-template <class V>
-__host__ __device__ inline size_t tail_smem_bytes(const TailArgs<V> &A) {
-  size_t b = tail_align(sizeof(TailArgs<V>));
-  for (int k = 0; k < A.nl; ++k) {
-    const size_t n = (size_t)A.L[k].n, nw = n * (size_t)A.L[k].w;
-    b += tail_align(nw * sizeof(int)) + tail_align(nw * sizeof(V)) + tail_align(n * sizeof(V));  // col, val, dinv
-    if (k + 1 < A.nl) b += tail_align(n * sizeof(int));                                          // agg
-    if (k > 0) b += tail_align(n * sizeof(int)) + tail_align((size_t)A.L[k - 1].n * sizeof(int)); // mptr, mem
-    b += 4 * tail_align(n * sizeof(V));                                                          // x, x2, b, r
-  }
-  const size_t nk = (size_t)A.L[A.nl - 1].n;
-  return b + tail_align(nk * nk * sizeof(V));  // the coarsest inverse
-}
-
-// Block-wide asynchronous copy of `bytes` (a multiple of 4) from global to shared memory:
-// 16-byte cp.async where both addresses allow it, 4-byte otherwise.  Completion is waited
-// for by stage_wait.
-__device__ __forceinline__ void stage_copy(void *dst, const void *src, size_t bytes) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  const char *sp = static_cast<const char *>(src);
-  size_t done = 0;
-  if (((reinterpret_cast<uintptr_t>(src) | d) & 15) == 0) {
-    const size_t n16 = bytes / 16;
-    for (size_t k = threadIdx.x; k < n16; k += blockDim.x)
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d + (unsigned)(16 * k)), "l"(sp + 16 * k)
-                   : "memory");
-    done = n16 * 16;
-  }
-  for (size_t k = done / 4 + threadIdx.x; k < bytes / 4; k += blockDim.x)
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d + (unsigned)(4 * k)), "l"(sp + 4 * k)
-                 : "memory");
-}
-
-__device__ __forceinline__ void stage_wait() {
-  asm volatile("cp.async.commit_group;\n" ::: "memory");
-  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-  __syncthreads();
-}
+// ---- the coarse end of the V-cycle on one thread-block cluster ----
+// Every level from the first whose share fits shared memory down to the coarsest runs in
+// one launch of kClBlocks blocks on as many SMs.  Each block holds its rows of every level's
+// matrix and its own copy of the level's vectors; the lane group that finishes a row
+// stores it to every block's copy through distributed shared memory, so the next phase's
+// gathers are local.  Phases are separated by the hardware cluster barrier (0.25 us, where a
+// dependent launch costs 4-5 us whatever the level's size).  The restriction, the coarse
+// level's first sweep and the prolongation need no phase of their own: every block does them
+// for all rows on its own copies.  Per level that leaves four barriers: two pre-smoothing
+// sweeps in one pass, the residual, and two post-smoothing sweeps.
+// A block's share (matrix, maps, 16-bit indices) is packed once per hierarchy (cl_pack) into
+// one contiguous image, so that a launch stages it with 16-byte asynchronous copies.
+// What bounds it is the chain of phases, ~0.7 us each.  At 128^3 (levels of 4111, 527, 78 and 20
+// rows) it takes 25 us where the one-block tail and the 4111-row level's kernels took 44; with
+// levels that did not fit one block's shared memory (559 rows x 55 slots) 27 us instead of 100.
+constexpr int kClBlocks = 16;      // the largest (non-portable) cluster
+constexpr int kClThreads = 512;
+constexpr int kClLevels = 16;
 
 template <class V>
-__global__ void __launch_bounds__(kTailSmemThreads) vcycle_tail_smem(TailArgs<V> A) {
-  extern __shared__ __align__(16) unsigned char tsm[];
-  TailArgs<V> &S = *reinterpret_cast<TailArgs<V> *>(tsm);
-  unsigned char *p = tsm + tail_align(sizeof(TailArgs<V>));
+struct ClLevel {
+  int n, w, g;                // rows, slots, lanes per row (power of two)
+  size_t ld;
+  const int *col;
+  const V *val, *dinv;
+  const int *agg;             // node -> next coarser node
+  const int *mptr, *mem;      // members of the next coarser level's nodes on this one
+};
+template <class V>
+struct ClArgs {
+  int nl, sweeps;             // levels, the last one solved by its explicit inverse
+  V omega, alpha;
+  const V *inv, *b;
+  V *x;
+  unsigned char *img;         // the blocks' packed shares, `share` bytes each
+  unsigned share, total;      // bytes of a share; of the whole shared-memory layout
+  ClLevel<V> L[kClLevels];
+};
+
+__host__ __device__ inline unsigned tail_align(size_t b) { return (unsigned)((b + 15) & ~(size_t)15); }
+
+// a block's rows of a level of n rows, and the odd leading dimension of its staged slots (so
+// that lanes on neighbouring slots of a row fall in different banks)
+__host__ __device__ inline int cl_rows_per_block(int n) { return (n + kClBlocks - 1) / kClBlocks; }
+__host__ __device__ inline int cl_ld(int n) { return cl_rows_per_block(n) | 1; }
+
+// Byte offsets of level k in a block's shared memory; the same in every block.  The packed
+// share comes first (val .. mem of every level), the vectors after it.
+struct ClOffsets {
+  unsigned val;               // V [slot][row]; the coarsest level: [row][n] of the inverse
+  unsigned col;               // u16 [slot][row]
+  unsigned dinv;              // V: all rows (the top level: the block's)
+  unsigned agg, mptr, mem;    // u16
+  unsigned xa, xb;            // V: the level's vector, twice (all rows)
+  unsigned b;                 // V: the block's rows (the coarsest level: all rows)
+};
+
+template <class V>
+__host__ __device__ inline void cl_layout(const ClArgs<V> &A, ClOffsets *off, unsigned *share, unsigned *total) {
+  unsigned o = 0;
   auto take = [&](size_t bytes) {
-    unsigned char *q = p;
-    p += tail_align(bytes);
-    return q;
+    const unsigned p = o;
+    o += tail_align(bytes);
+    return p;
   };
-  const int t = threadIdx.x, T = blockDim.x;
-  if (t == 0) S = A;
-  __syncthreads();
-  for (int k = 0; k < A.nl; ++k) {
-    const TailLevel<V> &G = A.L[k];
-    const int n = G.n, w = G.w;
-    int *col = (int *)take((size_t)n * w * sizeof(int));
-    V *val = (V *)take((size_t)n * w * sizeof(V));
-    V *dinv = (V *)take((size_t)n * sizeof(V));
-    if (G.ld == (size_t)n) {
-      // coarse levels: the slot-major arrays are contiguous
-      stage_copy(col, G.col, (size_t)n * w * sizeof(int));
-      stage_copy(val, G.val, (size_t)n * w * sizeof(V));
-    } else {
-      for (int e = t; e < n * w; e += T) {
-        const int slot = e / n, i = e - slot * n;
-        const size_t at = (size_t)slot * G.ld + i;
-        col[e] = G.col[at];
-        val[e] = G.val[at];
+  for (int part = 0; part < 2; ++part) {
+    for (int k = 0; k < A.nl; ++k) {
+      const size_t n = (size_t)A.L[k].n, rows = (size_t)cl_rows_per_block(A.L[k].n);
+      const size_t sl = (size_t)cl_ld(A.L[k].n) * A.L[k].w;
+      const bool last = k + 1 == A.nl;
+      if (part == 0) {
+        const unsigned val = take((last ? rows * n : sl) * sizeof(V));
+        const unsigned col = take(last ? 0 : sl * sizeof(uint16_t));
+        const unsigned dinv = take(last ? 0 : (k == 0 ? rows : n) * sizeof(V));
+        const unsigned agg = take(last ? 0 : n * sizeof(uint16_t));
+        const unsigned mptr = take(last ? 0 : ((size_t)A.L[k + 1].n + 1) * sizeof(uint16_t));
+        const unsigned mem = take(last ? 0 : n * sizeof(uint16_t));
+        if (off) {
+          off[k].val = val;
+          off[k].col = col;
+          off[k].dinv = dinv;
+          off[k].agg = agg;
+          off[k].mptr = mptr;
+          off[k].mem = mem;
+        }
+      } else {
+        const unsigned xa = take(n * sizeof(V));
+        const unsigned xb = take(last ? 0 : n * sizeof(V));
+        const unsigned b = take((last ? n : rows) * sizeof(V));
+        if (off) {
+          off[k].xa = xa;
+          off[k].xb = xb;
+          off[k].b = b;
+        }
       }
     }
-    stage_copy(dinv, G.dinv, (size_t)n * sizeof(V));
-    int *agg = nullptr, *mptr = nullptr, *mem = nullptr;
-    if (k + 1 < A.nl) {
-      agg = (int *)take((size_t)n * sizeof(int));
-      stage_copy(agg, G.agg, (size_t)n * sizeof(int));
-    }
-    if (k > 0) {
-      const int nf = A.L[k - 1].n;
-      mptr = (int *)take((size_t)n * sizeof(int));
-      mem = (int *)take((size_t)nf * sizeof(int));
-      stage_copy(mptr, G.mptr, (size_t)n * sizeof(int));
-      stage_copy(mem, G.mem, (size_t)nf * sizeof(int));
-    }
-    V *x = (V *)take((size_t)n * sizeof(V));
-    V *x2 = (V *)take((size_t)n * sizeof(V));
-    V *b = (V *)take((size_t)n * sizeof(V));
-    V *r = (V *)take((size_t)n * sizeof(V));
-    if (k == 0) stage_copy(b, G.b, (size_t)n * sizeof(V));
-    if (t == 0) {
-      TailLevel<V> &D = S.L[k];
-      D.ld = (size_t)n;
-      D.col = col;
-      D.val = val;
-      D.dinv = dinv;
-      D.agg = agg;
-      D.mptr = mptr;
-      D.mem = mem;
-      D.x = x;
-      D.x2 = x2;
-      D.b = b;
-      D.r = r;
-    }
+    if (part == 0 && share) *share = o;
   }
-  {
-    const int nk = A.L[A.nl - 1].n;
-    V *inv = (V *)take((size_t)nk * nk * sizeof(V));
-    stage_copy(inv, A.inv, (size_t)nk * nk * sizeof(V));
-    if (t == 0) S.inv = inv;
+  if (total) *total = o;
+}
+
+// The static part of the kernel's shared memory (offsets, level sizes), with margin.
+constexpr unsigned kClStatic = 2048;
+
+// Whether the levels of A fit a cluster's shared memory: 16-bit indices, and the layout
+// within what a block may opt into.  Sets A.share and A.total.
+template <class V>
+static bool cl_fits(ClArgs<V> &A) {
+  size_t big = 0;
+  for (int k = 0; k < A.nl; ++k) {
+    if (A.L[k].n > 65535) return false;
+    big += (size_t)cl_ld(A.L[k].n) * A.L[k].w + (size_t)A.L[k].n;
   }
-  stage_wait();
-  tail_body<V, kTailSmemBatch<V>>(S);
+  if (big > (size_t)1 << 20) return false;  // far beyond shared memory: the sums stay small
+  cl_layout<V>(A, nullptr, &A.share, &A.total);
+  return A.total + kClStatic <= kSmemMax;
+}
+
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ unsigned cluster_rank() {
+  unsigned r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+
+__device__ __forceinline__ void remote_store(unsigned addr, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+__device__ __forceinline__ void remote_store(unsigned addr, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
+}
+
+// v to *p of every block of the cluster, the g lanes of a group taking the blocks in turn
+template <class V>
+__device__ __forceinline__ void cl_broadcast(V *p, V v, int sub, int g) {
+  const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+  for (int d = sub; d < kClBlocks; d += g) {
+    unsigned ra;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(d));
+    remote_store(ra, v);
+  }
+}
+
+// The block's share of every level, packed: block r of the grid writes block r's image.
+template <class V>
+__global__ void __launch_bounds__(kClThreads) cl_pack(const __grid_constant__ ClArgs<V> A) {
+  __shared__ ClOffsets off[kClLevels];
+  const int t = threadIdx.x, rank = blockIdx.x;
+  if (t == 0) cl_layout<V>(A, off, nullptr, nullptr);
   __syncthreads();
-  for (int i = t; i < A.L[0].n; i += T) A.L[0].x[i] = S.L[0].x[i];
+  unsigned char *img = A.img + (size_t)rank * A.share;
+  const int last = A.nl - 1;
+  for (int k = 0; k < A.nl; ++k) {
+    const ClLevel<V> &L = A.L[k];
+    const int n = L.n, R = cl_rows_per_block(n), ld = cl_ld(n), r0 = rank * R, rows = max(0, min(R, n - r0));
+    V *val = (V *)(img + off[k].val), *dinv = (V *)(img + off[k].dinv);
+    uint16_t *col = (uint16_t *)(img + off[k].col), *agg = (uint16_t *)(img + off[k].agg);
+    uint16_t *mptr = (uint16_t *)(img + off[k].mptr), *mem = (uint16_t *)(img + off[k].mem);
+    if (k == last) {
+      for (int e = t; e < rows * n; e += kClThreads) val[e] = A.inv[(size_t)r0 * n + e];
+      continue;
+    }
+    for (int e = t; e < ld * L.w; e += kClThreads) {
+      const int s = e / ld, i = e - s * ld;
+      const size_t at = (size_t)s * L.ld + r0 + i;
+      val[e] = i < rows ? L.val[at] : V(0);
+      col[e] = i < rows ? (uint16_t)L.col[at] : (uint16_t)0;
+    }
+    const int nc = A.L[k + 1].n;
+    for (int i = t; i < n; i += kClThreads) {
+      agg[i] = (uint16_t)L.agg[i];
+      mem[i] = (uint16_t)L.mem[i];
+      if (k > 0) dinv[i] = L.dinv[i];
+    }
+    if (k == 0)
+      for (int i = t; i < rows; i += kClThreads) dinv[i] = L.dinv[r0 + i];
+    for (int i = t; i <= nc; i += kClThreads) mptr[i] = (uint16_t)(i < nc ? L.mptr[i] : n);
+  }
+}
+
+// a level as the phases see it
+template <class V>
+struct ClView {
+  const V *val, *dinv;        // dinv: the block's rows
+  const uint16_t *col;
+  V *xa, *xb, *b;
+  int n, w, g, rows, r0, ld;
+};
+
+// v[i] = x[i] + om dinv_i (b_i - sum_k a_ik x(col_ik)) (RES: b_i - the sum) for the block's
+// rows of a level, g lanes per row, handed to out(row, value, lane of the group)
+template <bool RES, class V, class F>
+__device__ __forceinline__ void cl_rows(const ClView<V> &Q, const V *x, V om, F out) {
+  const int g = Q.g, sub = threadIdx.x & (g - 1), per = kClThreads / g, step = g * Q.ld;
+  for (int i0 = 0; i0 < Q.rows; i0 += per) {  // the same count for the whole block (shuffles)
+    const int i = i0 + (int)threadIdx.x / g;
+    const bool act = i < Q.rows;
+    V s = V(0), bi = V(0), xi = V(0), di = V(0);
+    if (act) {
+      bi = Q.b[i];
+      if (!RES) {
+        xi = x[Q.r0 + i];
+        di = Q.dinv[i];
+      }
+      const V *vp = Q.val + sub * Q.ld + i;
+      const uint16_t *cp = Q.col + sub * Q.ld + i;
+      int k = sub;
+      for (; k + 3 * g < Q.w; k += 4 * g, vp += 4 * step, cp += 4 * step) {
+        const V a0 = vp[0], a1 = vp[step], a2 = vp[2 * step], a3 = vp[3 * step];
+        const int c0 = cp[0], c1 = cp[step], c2 = cp[2 * step], c3 = cp[3 * step];
+        s += a0 * x[c0];
+        s += a1 * x[c1];
+        s += a2 * x[c2];
+        s += a3 * x[c3];
+      }
+      for (; k < Q.w; k += g, vp += step, cp += step) s += *vp * x[*cp];
+    }
+    for (int o = g >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (act) out(i, RES ? bi - s : xi + om * di * (bi - s), sub);
+  }
+}
+
+template <class V>
+__global__ void __launch_bounds__(kClThreads, 1) vcycle_cluster(const __grid_constant__ ClArgs<V> A) {
+  extern __shared__ __align__(16) unsigned char cl_smem[];
+  __shared__ ClOffsets off[kClLevels];
+  __shared__ int4 dim[kClLevels];  // n, w, g
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int rank = (int)cluster_rank();
+  const V om = A.omega, al = A.alpha;
+  const int sw = A.sweeps, last = A.nl - 1;
+  // ---- the block's share of every level ----
+  {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(cl_smem);
+    const unsigned char *src = A.img + (size_t)rank * A.share;
+    for (unsigned o = 16 * t; o < A.share; o += 16 * kClThreads)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d + o), "l"(src + o) : "memory");
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  }
+  if (t == 0) cl_layout<V>(A, off, nullptr, nullptr);
+  if (t >= 32 && t - 32 < A.nl) dim[t - 32] = make_int4(A.L[t - 32].n, A.L[t - 32].w, A.L[t - 32].g, 0);
+  __syncthreads();
+  auto ptr = [&](unsigned o) { return reinterpret_cast<V *>(cl_smem + o); };
+  auto idx = [&](unsigned o) { return reinterpret_cast<uint16_t *>(cl_smem + o); };
+  auto view = [&](int k) {
+    const ClOffsets o = off[k];
+    const int4 q = dim[k];
+    ClView<V> Q;
+    Q.n = q.x;
+    Q.w = q.y;
+    Q.g = q.z;
+    const int R = cl_rows_per_block(Q.n);
+    Q.r0 = rank * R;
+    Q.rows = max(0, min(R, Q.n - Q.r0));
+    Q.ld = R | 1;
+    Q.val = ptr(o.val);
+    Q.col = idx(o.col);
+    Q.dinv = ptr(o.dinv) + (k == 0 ? 0 : Q.r0);
+    Q.xa = ptr(o.xa);
+    Q.xb = ptr(o.xb);
+    Q.b = ptr(o.b);
+    return Q;
+  };
+  {
+    // the right-hand side, and the first sweep from zero for every row
+    const ClView<V> Q = view(0);
+    if (last == 0) {
+      for (int i = t; i < Q.n; i += kClThreads) Q.b[i] = A.b[i];
+    } else {
+      const V *dinv = A.L[0].dinv;
+#pragma unroll 4
+      for (int i = t; i < Q.n; i += kClThreads) {
+        const V bi = A.b[i];
+        Q.xb[i] = om * dinv[i] * bi;
+        if ((unsigned)(i - Q.r0) < (unsigned)Q.rows) Q.b[i - Q.r0] = bi;
+      }
+    }
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();
+  cluster_barrier();  // every block runs: its shared memory may be written from here on
+  // ---- down ----
+  // a level's iterate lies in xb after one sweep (from zero: no operator) and changes sides
+  // with each further one
+  for (int k = 0; k < last; ++k) {
+    const ClView<V> Q = view(k);
+    V *x = Q.xb, *y = Q.xa;
+    for (int q = 1; q < sw; ++q) {
+      cl_rows<false>(Q, x, om, [&](int i, V v, int sub) { cl_broadcast(y + Q.r0 + i, v, sub, Q.g); });
+      cluster_barrier();
+      V *z = x; x = y; y = z;
+    }
+    cl_rows<true>(Q, x, om, [&](int i, V v, int sub) { cl_broadcast(y + Q.r0 + i, v, sub, Q.g); });
+    cluster_barrier();
+    // the coarse right-hand side, in member order, and its first sweep
+    const ClView<V> C = view(k + 1);
+    const uint16_t *mptr = idx(off[k].mptr), *mem = idx(off[k].mem);
+    const V *dinv = ptr(off[k + 1].dinv);
+    for (int I = t; I < C.n; I += kClThreads) {
+      V s = V(0);
+      for (int q = mptr[I], e = mptr[I + 1]; q < e; ++q) s += y[mem[q]];
+      if (k + 1 == last) {
+        C.b[I] = s;
+      } else {
+        C.xb[I] = om * dinv[I] * s;
+        if ((unsigned)(I - C.r0) < (unsigned)C.rows) C.b[I - C.r0] = s;
+      }
+    }
+    __syncthreads();
+  }
+  // ---- the coarsest level: x = K^-1 b, a warp per row ----
+  const ClView<V> K = view(last);
+  for (int i = warp; i < K.rows; i += kClThreads / 32) {
+    V s = V(0);
+#pragma unroll 4
+    for (int j = lane; j < K.n; j += 32) s += K.val[i * K.n + j] * K.b[j];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (last == 0) {
+      if (lane == 0) A.x[K.r0 + i] = s;
+    } else {
+      cl_broadcast(K.xa + K.r0 + i, s, lane, 32);
+    }
+  }
+  if (last == 0) return;  // no remote access after the first barrier
+  cluster_barrier();
+  // ---- up ----
+  const V *xc = K.xa;
+  for (int k = last - 1; k >= 0; --k) {
+    const ClView<V> Q = view(k);
+    V *x = (sw & 1) ? Q.xb : Q.xa, *y = (sw & 1) ? Q.xa : Q.xb;
+    const uint16_t *agg = idx(off[k].agg);
+    for (int i = t; i < Q.n; i += kClThreads) x[i] += al * xc[agg[i]];
+    __syncthreads();
+    for (int q = 0; q < sw; ++q) {
+      if (k == 0 && q + 1 == sw) {
+        cl_rows<false>(Q, x, om, [&](int i, V v, int sub) {
+          if (sub == 0) A.x[Q.r0 + i] = v;
+        });
+      } else {
+        cl_rows<false>(Q, x, om, [&](int i, V v, int sub) { cl_broadcast(y + Q.r0 + i, v, sub, Q.g); });
+        cluster_barrier();
+      }
+      V *z = x; x = y; y = z;
+    }
+    xc = x;
+  }
 }
 // ---------------------------------------------- the whole solve as one persistent kernel
 //
@@ -1774,6 +1998,10 @@ struct MgHier {
   T *coarse_inv = nullptr;
   int coarse_n = 0;
   T *uval = nullptr;  // coarse rows before the ELL transpose
+  // the levels run by vcycle_cluster: from cl_first on (-1: none fit), their packed shares
+  ClArgs<T> cl{};
+  int cl_first = -1;
+  unsigned char *cl_img = nullptr;
   // FGMRES: basis V, preconditioned vectors Z, V-cycle in/out, correction
   T *V = nullptr, *Z = nullptr, *vin = nullptr, *vout = nullptr, *dvec = nullptr;
 };
@@ -1812,7 +2040,7 @@ struct MgWork {
   // checked after the next solve's readback
   int *cstat = nullptr;
   int *cstat_host = nullptr;
-  bool tail_smem_set = false;  // the staged tail kernels may take kTailSmemMax
+  bool cluster_set = false;  // vcycle_cluster may take kSmemMax and a 16-block cluster
   // the numeric build's per-level widths (device, and its pinned readback; [kMaxLevels + 1]
   // is the ELL overflow flag) and the ELL slots allocated per level (host, the widest seen)
   int *wdev = nullptr;
@@ -1866,7 +2094,7 @@ static void free_hier(apc_context *c, MgHier<T> &H) {
     apc_free(c, L.b);
     apc_free(c, L.r);
   }
-  void *p[] = {H.coarse_inv, H.uval, H.V, H.Z, H.vin, H.vout, H.dvec};
+  void *p[] = {H.coarse_inv, H.uval, H.cl_img, H.V, H.Z, H.vin, H.vout, H.dvec};
   for (void *q : p) apc_free(c, q);
 }
 
@@ -1977,6 +2205,51 @@ static int mg_structure(apc_context *c) {
   }
   S.nlev = lev + 1;
   S.gen = c->select_gen;
+  return APC_OK;
+}
+
+// The levels that vcycle_cluster runs (from the first that fits) and their packed shares,
+// on c->s after the hierarchy's operators and the coarsest inverse.
+template <class T>
+static int cluster_levels(apc_context *c, MgHier<T> &H) {
+  MgWork *m = c->mg;
+  H.cl_first = -1;
+  if (!m->cluster_set) {
+    for (const void *f : {(const void *)vcycle_cluster<float>, (const void *)vcycle_cluster<double>}) {
+      APC_CUDA_TRY(c, cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)(kSmemMax - kClStatic)));
+      APC_CUDA_TRY(c, cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    }
+    m->cluster_set = true;
+  }
+  for (int l = std::max(0, H.nlev - kClLevels); l < H.nlev; ++l) {
+    ClArgs<T> A{};
+    A.nl = H.nlev - l;
+    A.inv = H.coarse_inv;
+    for (int k = 0; k < A.nl; ++k) {
+      const MgLevel<T> &Q = H.lv[l + k];
+      ClLevel<T> &D = A.L[k];
+      D.n = Q.n;
+      D.w = Q.w;
+      D.ld = Q.ld;
+      D.col = Q.col;
+      D.val = Q.val;
+      D.dinv = Q.dinv;
+      D.agg = Q.agg;
+      D.mptr = k + 1 < A.nl ? H.lv[l + k + 1].mptr : nullptr;
+      D.mem = k + 1 < A.nl ? H.lv[l + k + 1].mem : nullptr;
+      D.g = tail_lanes(cl_rows_per_block(Q.n), Q.w, kClThreads);
+    }
+    if (!cl_fits(A)) continue;
+    APC_TRY(apc_ensure(c, &H.cl_img, (size_t)A.share * kClBlocks));
+    A.img = H.cl_img;
+    cl_pack<T><<<kClBlocks, kClThreads, 0, c->s>>>(A);
+    apc_count_launch(c);
+    APC_CUDA_TRY(c, cudaGetLastError());
+    H.cl = A;
+    H.cl_first = l;
+    break;
+  }
   return APC_OK;
 }
 
@@ -2097,13 +2370,6 @@ static int mg_build(apc_context *c) {
   }
   APC_TRY(apc_ensure(c, &H.coarse_inv, (size_t)n * n + 1));
   H.coarse_n = n;
-  if (!m->tail_smem_set) {
-    APC_CUDA_TRY(c, cudaFuncSetAttribute(vcycle_tail_smem<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kTailSmemMax));
-    APC_CUDA_TRY(c, cudaFuncSetAttribute(vcycle_tail_smem<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kTailSmemMax));
-    m->tail_smem_set = true;
-  }
   if (n <= kCoarseInvMax) {
     // on the device, in stream order: no host round trip; a singular operator is reported
     // by the solve that follows (check_coarse)
@@ -2120,7 +2386,7 @@ static int mg_build(apc_context *c) {
     apc_count_launch(c);
     APC_CUDA_TRY(c, cudaGetLastError());
     APC_CUDA_TRY(c, cudaMemcpyAsync(m->cstat_host, m->cstat, sizeof(int), cudaMemcpyDeviceToHost, c->s));
-    return APC_OK;
+    return cluster_levels(c, H);
   }
   // a stalled coarsening leaves more rows: on the host
   std::vector<int> col(K.ld * K.w);
@@ -2166,7 +2432,7 @@ static int mg_build(apc_context *c) {
                                   c->s));
   APC_CUDA_TRY(c, apc_stream_wait(c));
   if (m->cstat_host) *m->cstat_host = 0;
-  return APC_OK;
+  return cluster_levels(c, H);
 }
 
 // After a host wait that follows the hierarchy build in stream order: the device-side
@@ -2192,8 +2458,32 @@ static void vcycle(apc_context *c, cudaStream_t s, int l, const T *b, T *x) {
   // solve from 48 to 29 FGMRES iterations
   const T omega = (T)(c->cfg.mg_omega > 0 ? c->cfg.mg_omega : 0.95);
   const T alpha = (T)(c->cfg.mg_alpha > 0 ? c->cfg.mg_alpha : 1.8);
+  if (l == H.cl_first) {
+    // this level and every coarser one on one cluster
+    ClArgs<T> A = H.cl;
+    A.sweeps = sweeps;
+    A.omega = omega;
+    A.alpha = alpha;
+    A.b = b;
+    A.x = x;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(kClBlocks);
+    cfg.blockDim = dim3(kClThreads);
+    cfg.dynamicSmemBytes = A.total;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kClBlocks;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, vcycle_cluster<T>, A);  // an error is read after the capture
+    apc_count_launch(c);
+    return;
+  }
   if (n <= kTail || l == H.nlev - 1) {
-    // this level and every coarser one in a single block
+    // levels that do not fit a cluster (rows of hundreds of slots): a single block
     TailArgs<T> A{};
     A.nl = std::min(H.nlev - l, kTailLevels);
     A.inv = H.coarse_inv;
@@ -2216,17 +2506,9 @@ static void vcycle(apc_context *c, cudaStream_t s, int l, const T *b, T *x) {
       D.b = k == 0 ? const_cast<T *>(b) : Q.b;
       D.x2 = Q.x2;
       D.r = Q.r;
+      D.g = tail_lanes(Q.n, Q.w, kTailThreads);
     }
-    // staged in shared memory when the tail's levels fit (they do at 128^3: ~90 KB in FP32)
-    const size_t tb = tail_smem_bytes(A);
-    const bool staged = tb <= kTailSmemMax;
-    const int threads = staged ? kTailSmemThreads : kTailThreads;
-    // wide rows get several lanes while the block has lanes to spare
-    for (int k = 0; k < A.nl; ++k) A.L[k].g = tail_lanes(A.L[k].n, A.L[k].w, threads);
-    if (staged)
-      vcycle_tail_smem<T><<<1, threads, tb, s>>>(A);
-    else
-      vcycle_tail<T><<<1, threads, 0, s>>>(A);
+    vcycle_tail<T><<<1, kTailThreads, 0, s>>>(A);
     apc_count_launch(c);
     return;
   }

@@ -1,0 +1,86 @@
+"""The V-cycle's coarse levels on a thread-block cluster: the potential solve meets its stopping
+test, in few iterations, for hierarchies at the edges of what the cluster kernel takes - one
+level (the dense solve alone), levels of fewer rows than blocks, a whole hierarchy in the
+cluster, grid levels above it - at every sweep parity and in each precision.
+
+The residual is formed here in FP64 from the assembled matrix.  The solver stops at
+rtol ||D^-1 b|| = 1e-10 of its own FP64 residual; evaluating it here in another order moves it
+by a few ulp of ||D^-1 A|| ||x||, 1e-12 of ||D^-1 b|| at these sizes, so 1.05e-10 holds.  A
+V-cycle that is wrong on some level still lets FGMRES converge, but more slowly, so where the
+Krylov vectors are FP64 the iteration count is compared with the persistent solve's
+(mixed_solve_graphs = 0), whose V-cycle is the same operator in other code: rounding moves the
+count by at most two.  (The FP32-Krylov path's count follows the rounding of its corrections:
+its graph and persistent forms differ by tens of iterations on the largest box here.)
+"""
+import numpy as np
+import pytest
+
+from apcloud import binding, ics
+
+pytestmark = pytest.mark.gpu
+
+BOXES = {
+    "lattice4": ("zel", 4, 2e-2),      # 8 cells: one level
+    "lattice8": ("zel", 8, 1e-9),      # every particle in a cell of its own: 512 cells and deeper
+    "lattice17": ("zel", 17, None),
+    "ball1500": ("ball", 1500, None),  # uneven rows, few per block
+    "ball20k": ("ball", 20011, None),
+    "lattice40": ("zel", 40, 1e-5),    # grid levels above the cluster
+}
+
+
+def _box(kind, size, gfd_c):
+    if kind == "ball":
+        rho = size / (4.0 / 3.0 * np.pi * 0.3 ** 3)
+        return ics.uniform_ball(size, 0.3, seed=3), gfd_c or 8.0 ** (5.0 / 3.0) * rho ** (-2.0 / 3.0)
+    p = ics.zeldovich(size, -2.0, 0.25, 0.05, 1.0, 0.0, seed=4)
+    return p, gfd_c or 1.28 * 8.0 ** (5.0 / 3.0) * size ** -2.0
+
+
+C_POT = 1.5 / 0.05
+
+
+def _solve(parts, c, depth, precision, sweeps, graphs=1):
+    prec = {"mixed": binding.APC_PREC_MIXED, "fp64mg": binding.APC_PREC_FP64_MULTIGRID,
+            "vcycle32": binding.APC_PREC_MIXED_VCYCLE}[precision]
+    g = binding.GpuPath(parts, depth, c, precision=prec, mg_sweeps=sweeps, solve_graphs=graphs)
+    g.select()
+    g.solve(1.0 / parts.n, C_POT, -1.0)
+    return g
+
+
+@pytest.fixture(scope="module", params=sorted(BOXES))
+def box(request, gpu_lib):
+    """(particles, gfd_c, depth, cells, potential matrix) of a box."""
+    parts, c = _box(*BOXES[request.param])
+    depth = 8 if request.param == "lattice8" else 21
+    g = _solve(parts, c, depth, "mixed", 2)
+    cells, mat = g.cells(), g.matrix(1)
+    g.close()
+    return parts, c, depth, cells, mat
+
+
+@pytest.mark.parametrize("sweeps", [1, 2, 3])
+@pytest.mark.parametrize("precision", ["mixed", "fp64mg", "vcycle32"])
+def test_potential_residual(box, precision, sweeps):
+    parts, c, depth, cells, (ptr, col, val) = box
+    g = _solve(parts, c, depth, precision, sweeps)
+    st, f = g.solve_stats(), g.fields()
+    g.close()
+    if precision != "mixed":
+        g = _solve(parts, c, depth, "fp64mg", sweeps, graphs=0)
+        its = g.solve_stats()["potential_its"]
+        g.close()
+    m = cells.m
+    row = np.repeat(np.arange(m), np.diff(ptr))
+    v = cells.h[:m] ** 3
+    b = (f.density - np.sum(f.density * v) / np.sum(v)) * C_POT
+    ax = np.bincount(row, weights=val * f.potential[col], minlength=m)
+    d = np.zeros(m)
+    d[row[row == col]] = val[row == col]
+    d[d == 0.0] = 1.0
+    bn = np.linalg.norm(b / d)
+    assert st["potential_reason"] in (2, 3)
+    if bn > 1e-12 * C_POT / np.abs(d).max():  # equal densities: the right-hand side is rounding alone
+        assert np.linalg.norm((b - ax) / d) <= 1.05e-10 * bn
+        assert precision == "mixed" or abs(st["potential_its"] - its) <= 2
