@@ -119,8 +119,6 @@ struct apc_context {
   int *cell_of = nullptr;  // sorted particle -> cell
   uint64_t *full_keys = nullptr, *full_keys_alt = nullptr;  // fully sorted key copies (diagnostics)
   uint32_t *full_ids = nullptr, *full_ids_alt = nullptr;
-  double *gfd_scr_d = nullptr;  // GFD search: per-warp sort lists longer than a warp
-  int *gfd_scr_i = nullptr;
   int *gfd_qr = nullptr;         // GFD: cells queued for the Householder pass
   double *adj_ckpt = nullptr, *adj_tape = nullptr;  // trajectory VJP: checkpoints, Hessian tape
   double last_c_pot = 0.0, last_c_field = 0.0;       // constants of the last apc_solve

@@ -53,10 +53,9 @@ struct GfdParams {
   const int *count, *type, *nb24, *nnb;
   int *st_idx;
   double *gx;  // per cell the 9 x lm least-squares operator X
-  double *scr_d;  // per search warp: kListCap sort keys and indices (lists over 32)
-  int *scr_i;
   int *qr_list, *qr_count;  // cells for the Householder pass
   int *chunk_next;          // the search's next unclaimed cell (zeroed before its launch)
+  int chunk;                // cells per claim, <= kChunk
   int *ell_col;
   double *a1, *a2, *rhs;
   size_t ld;  // ELL leading dimension (row capacity)
@@ -127,18 +126,24 @@ struct __align__(16) WarpSmem {
   int bidx[8][kBucketCap];
 };
 
-// The search handles kChunk consecutive cells per warp: their lists (at most 32
-// candidates each, the usual case) are staged here, then lane q sorts cell q's list
-// sequentially.  Rows are padded to 33 entries so that lanes at the same position fall
-// in different banks.  12 cells per warp keep a block's shared memory at 28 KB, so 8
-// blocks (32 warps) fit on an SM; at 128^3 this measured faster than 8 or 16 cells.
+// A warp takes up to kChunk consecutive cells and stages their candidate lists here, one
+// after the other; when the pool or the chunk is full, lane q sorts the q-th list
+// sequentially.  A list starts an odd number of entries after the one before it, so that
+// lanes at the same position of lists of equal length fall in different banks.  Lists have 24
+// entries on a lattice and up to 10 lm (at most kListCap) where the tree is uneven: one
+// pool for every length keeps the long ones out of global memory, where one lane's sort
+// took 20-50 us per list while the rest of its warp waited (late 128^3 state, 9 % of the
+// cells: search 1.10 ms; 4k ball, 55 %: 0.46 ms).  12 cells per warp keep a block's shared
+// memory at 27 KB, so 8 blocks (32 warps) fit on an SM; at 128^3 this measured faster than 8
+// or 16 cells.
 constexpr int kChunk = 12;
-constexpr int kStageLd = 33;
+constexpr int kPool = 384;
+static_assert(kPool >= kListCap + 1, "the longest list fits an empty pool");
 struct SortStage {
-  double key[kChunk][kStageLd];
-  int idx[kChunk][kStageLd];
+  double key[kPool];
+  int idx[kPool];
   int nn[kChunk][8];
-  int staged[kChunk];
+  int off[kChunk], cell[kChunk];
 };
 
 // Least squares, per warp: a slice of the dynamic shared memory laid out as
@@ -255,14 +260,30 @@ __device__ void reference_sort(double *key, int *idx, const int *nn, int l, int 
   aquicksort(key, idx, 0, l - 1, lm);
 }
 
+// The staged lists: lane q sorts the q-th (reference_sort), then the warp writes the first
+// lm candidates of each with coalesced stores.
+__device__ __forceinline__ void sort_staged(const GfdParams &P, SortStage &T, int staged, int lane) {
+  if (lane < staged) {
+    int l = 0;
+#pragma unroll
+    for (int o = 0; o < 8; ++o) l += T.nn[lane][o];
+    reference_sort(T.key + T.off[lane], T.idx + T.off[lane], T.nn[lane], l, P.lm);
+  }
+  __syncwarp();
+  for (int t = lane; t < staged * P.lm; t += 32) {
+    const int q = t / P.lm, j = t - q * P.lm;
+    P.st_idx[(size_t)T.cell[q] * P.lm + j] = T.idx[T.off[q] + j];
+  }
+  __syncwarp();
+}
+
 // Phase 1: the neighbour search and the reference's sort; the first lm candidates go to
-// st_idx.  A warp takes kChunk consecutive cells.  For each in turn the whole warp finds
-// the candidates (rings of Neigh24 lists, discovery order kept per octant); a list of at
-// most 32 candidates is staged in shared memory.  Then lane q runs cell q's sort
-// (reference_sort), and the warp writes the chunk's stencils with coalesced stores.
-// Longer lists are sorted at once by lane 0 in a global scratch slice.  A cell whose
-// search fails raises its flag and gets its own index in every slot, so that phase 2
-// stays in bounds (the step then fails).
+// st_idx.  A warp takes P.chunk consecutive cells: 12 where that leaves every warp work, fewer
+// on small cell sets (one per warp up to 32 cells per SM), whose time is that of one warp's
+// cells in series.  For each in turn the whole warp finds the candidates (rings of Neigh24
+// lists, discovery order kept per octant) and stages the list in shared memory (SortStage).
+// A cell whose search fails raises its flag and gets its own index in every slot, so that
+// phase 2 stays in bounds (the step then fails).
 __global__ void __launch_bounds__(32 * kSearchWarps, 8) gfd_search(GfdParams P) {
   __shared__ WarpSmem smem[kSearchWarps];
   __shared__ SortStage stage[kSearchWarps];
@@ -270,15 +291,15 @@ __global__ void __launch_bounds__(32 * kSearchWarps, 8) gfd_search(GfdParams P) 
   WarpSmem &S = smem[w];
   SortStage &T = stage[w];
   const int lm = P.lm;
-  const int gw = blockIdx.x * kSearchWarps + w;
   // chunks are claimed from a counter: late in a run the cost per cell varies widely along
   // the Morton order, and a fixed assignment left warps with runs of costly cells
   for (;;) {
     int c0 = 0;
-    if (lane == 0) c0 = atomicAdd(P.chunk_next, kChunk);
+    if (lane == 0) c0 = atomicAdd(P.chunk_next, P.chunk);
     c0 = __shfl_sync(0xffffffffu, c0, 0);
     if (c0 >= P.m) break;
-    const int nq = min(kChunk, P.m - c0);
+    const int nq = min(P.chunk, P.m - c0);
+    int staged = 0, fill = 0;  // lists in the pool, entries they take
     // the next cell's Neigh24 row is loaded while the current cell is searched
     int cnt_next = P.nnb[c0];
     int m_next = lane < cnt_next ? P.nb24[24 * (size_t)c0 + lane] : -1;
@@ -379,7 +400,6 @@ __global__ void __launch_bounds__(32 * kSearchWarps, 8) gfd_search(GfdParams P) 
       if (few || !ok || l > P.sort_cap) {
         if (lane == 0) {
           atomicOr(P.err, few ? DERR_STENCIL_FEW : DERR_STENCIL_MANY);
-          T.staged[q] = 0;
         }
         if (lane < lm) P.st_idx[(size_t)i0 * lm + lane] = i0;
         __syncwarp();
@@ -387,77 +407,45 @@ __global__ void __launch_bounds__(32 * kSearchWarps, 8) gfd_search(GfdParams P) 
       }
       // ---- the list in bucket order, keyed by the squared distances (recomputed from
       //      the indices by the same operations as at discovery) ----
+      if (fill + l > kPool) {
+        sort_staged(P, T, staged, lane);
+        staged = 0;
+        fill = 0;
+      }
       {
         int v = 0;
 #pragma unroll
         for (int o = 0; o < 8; ++o)
           if (lane == o) v = nn[o];
-        if (lane < 8) T.nn[q][lane] = v;
-        __syncwarp();
-      }
-      if (l <= 32) {
-        int e = lane, m = i0;
-        double d2 = 0.0;
-        if (lane < l) {
-          int b = 0;
-#pragma unroll
-          for (int o = 0; o < 8; ++o) {
-            if (b == o && e >= nn[o]) {
-              e -= nn[o];
-              b = o + 1;
-            }
-          }
-          m = S.bidx[b][e];
-          double wx, wy, wz;
-          offset_of(P, m, i0, wx, wy, wz);
-          d2 = sq3(wx, wy, wz);
-          T.key[q][lane] = d2;
-          T.idx[q][lane] = m;
-        }
-        if (lane == 0) T.staged[q] = l;
-      } else {
-        // a longer list: the warp writes it in bucket order to this warp's slice of a global
-        // scratch list, 32 entries at a time; lane 0 sorts it now
-        double *ldist = P.scr_d + (size_t)gw * kListCap;
-        int *lidx = P.scr_i + (size_t)gw * kListCap;
-        int pre[9];
-        pre[0] = 0;
-#pragma unroll
-        for (int o = 0; o < 8; ++o) pre[o + 1] = pre[o] + nn[o];
-        for (int p = lane; p < l; p += 32) {
-          int b = 0, base = 0;
-#pragma unroll
-          for (int o = 1; o < 8; ++o)
-            if (p >= pre[o]) {
-              b = o;
-              base = pre[o];
-            }
-          const int m = S.bidx[b][p - base];
-          double wx, wy, wz;
-          offset_of(P, m, i0, wx, wy, wz);
-          ldist[p] = sq3(wx, wy, wz);
-          lidx[p] = m;
-        }
-        __threadfence_block();
-        __syncwarp();
+        if (lane < 8) T.nn[staged][lane] = v;
         if (lane == 0) {
-          reference_sort(ldist, lidx, T.nn[q], l, lm);
-          T.staged[q] = 0;
+          T.off[staged] = fill;
+          T.cell[staged] = i0;
         }
-        __threadfence_block();
-        __syncwarp();
-        if (lane < lm) P.st_idx[(size_t)i0 * lm + lane] = lidx[lane];
       }
+      int pre[9];
+      pre[0] = 0;
+#pragma unroll
+      for (int o = 0; o < 8; ++o) pre[o + 1] = pre[o] + nn[o];
+      for (int p = lane; p < l; p += 32) {
+        int b = 0, base = 0;
+#pragma unroll
+        for (int o = 1; o < 8; ++o)
+          if (p >= pre[o]) {
+            b = o;
+            base = pre[o];
+          }
+        const int m = S.bidx[b][p - base];
+        double wx, wy, wz;
+        offset_of(P, m, i0, wx, wy, wz);
+        T.key[fill + p] = sq3(wx, wy, wz);
+        T.idx[fill + p] = m;
+      }
+      ++staged;
+      fill += l | 1;
       __syncwarp();
     }
-    // ---- the staged lists: lane q sorts cell q's, then coalesced stores of the chunk ----
-    if (lane < nq && T.staged[lane] > 0) reference_sort(T.key[lane], T.idx[lane], T.nn[lane], T.staged[lane], lm);
-    __syncwarp();
-    for (int t = lane; t < nq * lm; t += 32) {
-      const int q = t / lm;
-      if (T.staged[q] > 0) P.st_idx[(size_t)c0 * lm + t] = T.idx[q][t - q * lm];
-    }
-    __syncwarp();
+    if (staged > 0) sort_staged(P, T, staged, lane);
   }
 }
 
@@ -833,12 +821,10 @@ int apc_gfd_assemble(apc_context *c, double c_dens, int (*during)(apc_context *)
   P.ell_col = c->ell_col; P.a1 = c->a1; P.a2 = c->a2; P.rhs = c->rhs;
   P.ld = ld;
   P.err = c->d_err;
+  const int swarps = apc_sm_count(c) * 8 * kSearchWarps;  // the search's resident warps
+  P.chunk = std::max(1, std::min(kChunk, (M + swarps - 1) / swarps));
   const int sblocks =
-      std::max(1, std::min((M + kSearchWarps * kChunk - 1) / (kSearchWarps * kChunk), apc_sm_count(c) * 8));
-  APC_TRY(apc_ensure(c, &c->gfd_scr_d, (size_t)sblocks * kSearchWarps * kListCap, nullptr));
-  APC_TRY(apc_ensure(c, &c->gfd_scr_i, (size_t)sblocks * kSearchWarps * kListCap, nullptr));
-  P.scr_d = c->gfd_scr_d;
-  P.scr_i = c->gfd_scr_i;
+      std::max(1, std::min((M + kSearchWarps * P.chunk - 1) / (kSearchWarps * P.chunk), swarps / kSearchWarps));
   APC_TRY(apc_ensure(c, &c->gfd_qr, (size_t)M + 1, nullptr));
   P.qr_list = c->gfd_qr;
   P.qr_count = c->counters + 112;
