@@ -29,6 +29,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "apc_internal.cuh"
 
@@ -221,7 +222,8 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_kernel(GmresArgs<T> A) {
   bool guess_zero = true;
   double ttol = 0.0, rnorm0 = 0.0, res = 0.0;
   if (threadIdx.x == 0) s_res = 0.0;
-  if (!grid_sync(A.bar, nb, A.err)) return;
+  unsigned epoch = 0;
+  if (!grid_sync(A.bar, nb, epoch, A.err)) return;
 
   while (!reason) {
     // ---- initial residual: u0 = D^-1 (b - A x) ----
@@ -246,7 +248,7 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_kernel(GmresArgs<T> A) {
       const double v = block_sum(nrm, sm_red);
       if (threadIdx.x == 0) put_partial(partB, 0, v);
     }
-    if (!grid_sync(A.bar, nb, A.err)) return;
+    if (!grid_sync(A.bar, nb, epoch, A.err)) return;
     gather_partials(partB, nb, 1, sh);
     __syncthreads();
     const double beta = sqrt(sh[0]);
@@ -279,7 +281,7 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_kernel(GmresArgs<T> A) {
       }
       __syncthreads();
       block_dots(w, A.U, A.un, r0, r1, it + 1, sm_red, partA);
-      if (!grid_sync(A.bar, nb, A.err)) return;
+      if (!grid_sync(A.bar, nb, epoch, A.err)) return;
       gather_partials(partA, nb, it + 1, sh);
       __syncthreads();
       if ((int)threadIdx.x <= it) {
@@ -299,7 +301,7 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_kernel(GmresArgs<T> A) {
       if (REORTH) {
         __syncthreads();
         block_dots(w, A.U, A.un, r0, r1, it + 1, sm_red, partB);
-        if (!grid_sync(A.bar, nb, A.err)) return;
+        if (!grid_sync(A.bar, nb, epoch, A.err)) return;
         gather_partials(partB, nb, it + 1, sh);
         __syncthreads();
         if ((int)threadIdx.x <= it) {
@@ -317,13 +319,13 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_kernel(GmresArgs<T> A) {
         }
         const double v = block_sum(nr, sm_red);
         if (threadIdx.x == 0) put_partial(partA, kNormSlot, v);
-        if (!grid_sync(A.bar, nb, A.err)) return;
+        if (!grid_sync(A.bar, nb, epoch, A.err)) return;
         gather_partials(partA + (size_t)kNormSlot * kMaxBlocks, nb, 1, sh);
         __syncthreads();
       } else {
         const double v = block_sum(nr, sm_red);
         if (threadIdx.x == 0) put_partial(partB, 0, v);
-        if (!grid_sync(A.bar, nb, A.err)) return;
+        if (!grid_sync(A.bar, nb, epoch, A.err)) return;
         gather_partials(partB, nb, 1, sh);
         __syncthreads();
       }
@@ -405,9 +407,370 @@ __global__ void __launch_bounds__(kThreads, 1) gmres_kernel(GmresArgs<T> A) {
       break;
     }
     guess_zero = false;
-    if (!grid_sync(A.bar, nb, A.err)) return;
+    if (!grid_sync(A.bar, nb, epoch, A.err)) return;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
+    *A.out_its = its;
+    *A.out_reason = reason;
+    *A.out_rnorm = res;
+  }
+}
+
+// ------------------------------------------------------------ the kernel on clusters
+//
+// The same solve, bit for bit, for matrices of up to a few tens of thousands of rows.  The
+// persistent kernel above gives every 1024 rows one block, so such a matrix kept a few SMs
+// busy: 18 gathers of 1024 rows are 10 us of one SM's gather rate, and 4 and 20 blocks took
+// 31 and 22 us per iteration (4,096 and 20,350 rows).  Here a cluster of K blocks shares the
+// rows of one such block:
+//   - a block keeps its rows' matrix (values, columns) and their slice of the basis in
+//     shared memory; only the gathered vector goes through L2;
+//   - four warps per 32 rows split the basis vectors of the dot products, eight at a time,
+//     by a transposing shuffle reduction (9 exchanges for 8 sums instead of 40);
+//   - per-warp sums go to the cluster's first block through distributed shared memory, which
+//     adds them in warp order and publishes them; then every block waits for all clusters
+//     (with one cluster, for its own blocks);
+//   - the norm's sum, the Givens rotation and the stopping test run in one warp while the rows'
+//     threads already gather the next product.
+// Each sum is formed by the additions of the persistent kernel in the same order: rows in its
+// blocks and warps, the xor tree of 32 lanes, warps in turn, blocks in turn.  The Givens
+// rotations of the new column run beside the Gram-Schmidt update.
+constexpr int kCgMaxClusters = 148;
+constexpr int kCgSmemMax = 225 * 1024;  // beside its few static words
+
+struct CgArgs {
+  GmresArgs<double> g;
+  int nvb, rpb;               // blocks of the persistent kernel, rows of each
+  int K;                      // blocks per cluster
+  unsigned o_u, o_col, o_red, o_nrm, o_hh, o_small;  // byte offsets in shared memory (values at 0)
+};
+
+// xor-tree sums over the warp of eight values: on return the sum of value j is in the lanes
+// with (lane >> 2) == j, formed by the offsets 16, 8, 4, 2, 1 in turn
+__device__ __forceinline__ double warp_sum8(double (&v)[8], int lane) {
+  const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const double keep = b4 ? v[4 + i] : v[i], send = b4 ? v[i] : v[4 + i];
+    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const double keep = b3 ? v[2 + i] : v[i], send = b3 ? v[i] : v[2 + i];
+    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+  }
+  const double keep = b2 ? v[1] : v[0], send = b2 ? v[0] : v[1];
+  double s = keep + __shfl_xor_sync(0xffffffffu, send, 4);
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  s += __shfl_xor_sync(0xffffffffu, s, 1);
+  return s;
+}
+
+__device__ __forceinline__ double xor_sum(double t) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  return t;
+}
+
+// slots whose gathers are issued together: a whole row of 18 where registers allow it (9 there
+// take 10.3 us per iteration at 4,096 rows instead of 8.0)
+template <int THREADS>
+constexpr int kCgBatch = THREADS == 256 ? 18 : (THREADS == 512 ? 9 : 6);
+
+// SMEM_U: the rows' slice of the basis lies in shared memory too; a basis too long for that
+// (restart 200 on 128 rows per block) is read from L2.
+template <int THREADS, bool SMEM_U>
+__global__ void __launch_bounds__(THREADS, 1) gmres_cluster(const __grid_constant__ CgArgs C) {
+  extern __shared__ __align__(16) unsigned char cg_smem[];
+  const GmresArgs<double> &A = C.g;
+  const int K = C.K, m = A.restart, vw = 32 / K, R = 32 * vw;  // 32-row warps, row slots
+  double *val = reinterpret_cast<double *>(cg_smem);           // [slot][row]
+  int *col = reinterpret_cast<int *>(cg_smem + C.o_col);
+  double *red = reinterpret_cast<double *>(cg_smem + C.o_red); // first block: [warp][vector]
+  double *nrm = reinterpret_cast<double *>(cg_smem + C.o_nrm); // first block: 1024 rows
+  double *small = reinterpret_cast<double *>(cg_smem + C.o_small);
+  double *cc = small, *ss = cc + (m + 1), *grs = ss + (m + 1), *scale = grs + (m + 2), *coef = scale + (m + 2),
+         *sh = coef + (m + 2), *hcol = sh + (m + 2), *wrow = hcol + (m + 2);
+  __shared__ double s_wsum[32];
+  __shared__ double s_res;
+  __shared__ int s_flow[2], s_go;
+
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nwarp = THREADS / 32;
+  const int crank = (int)cluster_rank(), vb = blockIdx.x / K;
+  const int part = warp / vw, vwl = warp - part * vw;  // the warp's share of the vectors, its rows
+  const bool lead = crank == 0;
+  // the rows, as the persistent kernel's block vb and its warps hold them
+  const int r0 = min(A.n, vb * C.rpb), r1 = min(A.n, r0 + C.rpb);
+  const int per = (r1 - r0 + 31) / 32;
+  const int vwarp = crank * vw + vwl;
+  const int row = r0 + vwarp * per + lane, slot = vwl * 32 + lane;
+  const bool owner = part == 0, act = lane < per && row < r1;
+  const bool own = owner && act;
+  double *const U = SMEM_U ? reinterpret_cast<double *>(cg_smem + C.o_u) + slot : A.U + row;  // the row's
+  const size_t us = SMEM_U ? (size_t)R : A.un;                                                // u_j at U[j us]
+  const int parts = nwarp / vw;
+  const int hld = m + 1;
+  double *HH = m <= 31 ? reinterpret_cast<double *>(cg_smem + C.o_hh)
+                       : A.hh + (size_t)blockIdx.x * (size_t)hld * m;
+  double *partA = A.part, *partB = A.part + (size_t)kSlots * kMaxBlocks;
+  unsigned target = 0;
+  const unsigned ncl = (unsigned)C.nvb;
+
+  // after a cluster's sums are published by its first block (or nothing is): every block
+  // waits for all clusters.  On a time-out the cluster's blocks meet once more, so that none
+  // of them is gone while another still stores to its shared memory.
+  auto all_clusters = [&]() -> bool {
+    if (ncl == 1) {
+      cluster_barrier();
+      return true;
+    }
+    target += ncl;
+    if (lead) __syncthreads();
+    if (t == 0) {
+      if (lead) grid_arrive(A.bar);
+      s_go = grid_wait(A.bar, target, A.err, kSpinLimit);
+    }
+    __syncthreads();
+    if (s_go) return true;
+    cluster_barrier();
+    return false;
+  };
+  // the sum of nrm over the persistent kernel's block, published in slot 0 of B
+  auto publish_norm = [&]() {
+    cluster_barrier();
+    if (lead) {
+      for (int wv = warp; wv < 32; wv += nwarp) {
+        const double v = xor_sum(nrm[wv * 32 + lane]);
+        if (lane == 0) s_wsum[wv] = v;
+      }
+      __syncthreads();
+      if (warp == 0) {
+        const double v = xor_sum(s_wsum[lane]);
+        if (lane == 0) partB[vb] = v;
+      }
+    }
+  };
+  auto gather_dots = [&](int nv) {
+    for (int j0 = 8 * warp; j0 < nv; j0 += 8 * nwarp) {
+      double v[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v[q] = 0.0;
+      for (int b = lane; b < C.nvb; b += 32)
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          if (j0 + q < nv) v[q] += __ldcg(partA + (size_t)(j0 + q) * kMaxBlocks + b);
+      const double sum = warp_sum8(v, lane);
+      const int j = j0 + (lane >> 2);
+      if ((lane & 3) == 0 && j < nv) {
+        const double h = sum * scale[j];  // <v_j, w>
+        hcol[j] = h;
+        coef[j] = h * scale[j];           // weight on u_j
+      }
+    }
+    __syncthreads();
+  };
+  // by one warp; every lane gets the norm's square
+  auto gather_norm = [&]() {
+    double v = 0.0;
+    for (int b = lane; b < C.nvb; b += 32) v += __ldcg(partB + b);
+    return xor_sum(v);
+  };
+
+  double di = 1.0, bi = 0.0, xi = 0.0;
+  if (act)
+    for (int k = part; k < A.w; k += parts) {
+      const size_t at = (size_t)k * A.ld + row;
+      val[k * R + slot] = A.val[at];
+      col[k * R + slot] = A.col[at];
+    }
+  if (own) {
+    const double d = A.val[row];
+    di = d == 0.0 ? 1.0 : 1.0 / d;
+    bi = A.b[row];
+    A.x[row] = 0.0;
+  }
+  for (int i = t; i < 1024; i += THREADS) nrm[i] = 0.0;
+  int its = 0, reason = 0, itcount = 0;
+  bool guess_zero = true;
+  double ttol = 0.0, rnorm0 = 0.0, res = 0.0;
+  if (t == 0) s_res = 0.0;
+  __syncthreads();
+  cluster_barrier();  // every block of the cluster runs
+  if (!all_clusters()) return;
+
+  auto spmv = [&](const double *v) {
+    constexpr int B = kCgBatch<THREADS>;
+    double s = 0.0;
+    for (int k = 0; k < A.w; k += B) {
+      double x[B];
+#pragma unroll
+      for (int u = 0; u < B; ++u)
+        if (k + u < A.w) x[u] = __ldcg(v + col[(k + u) * R + slot]);
+#pragma unroll
+      for (int u = 0; u < B; ++u)
+        if (k + u < A.w) s += val[(k + u) * R + slot] * x[u];
+    }
+    return s;
+  };
+
+  while (!reason) {
+    // ---- initial residual: u0 = D^-1 (b - A x) ----
+    if (own) {
+      double r = bi;
+      if (!guess_zero) r -= spmv(A.x);
+      const double u = di * r;
+      A.U[row] = u;
+      if (SMEM_U) U[0] = u;
+      remote_store(cluster_addr(nrm + (row - r0), 0), u * u);
+    }
+    publish_norm();
+    if (!all_clusters()) return;
+    const double beta = sqrt(gather_norm());
+    if (t == 0) {
+      scale[0] = beta != 0.0 ? 1.0 / beta : 1.0;
+      grs[0] = beta;
+    }
+    res = beta;
+    if (res == 0.0) {
+      reason = KSP_CONVERGED_ATOL;
+      break;
+    }
+    reason = converged_default(its, res, A.rtol, A.atol, A.dtol, ttol, rnorm0);
+    int it = 0;
+    __syncthreads();
+    double av = 0.0;  // the row of A u_it
+    if (own && !reason) av = spmv(A.U);
+    while (!reason && it < m && its < A.max_it) {
+      // ---- w = D^-1 A v_it and the cluster's dots with u_0..u_it ----
+      double w = 0.0;
+      if (own) {
+        w = di * scale[it] * av;
+        wrow[slot] = w;
+      }
+      __syncthreads();
+      {
+        const double wv = act ? wrow[slot] : 0.0;
+        for (int j0 = 8 * part; j0 <= it; j0 += 8 * parts) {
+          double v[8];
+#pragma unroll
+          for (int q = 0; q < 8; ++q) v[q] = act && j0 + q <= it ? wv * U[(j0 + q) * us] : 0.0;
+          const double sum = warp_sum8(v, lane);
+          const int j = j0 + (lane >> 2);
+          if ((lane & 3) == 0 && j <= it) remote_store(cluster_addr(red + vwarp * (m + 1) + j, 0), sum);
+        }
+      }
+      cluster_barrier();
+      if (lead && t <= it) {
+        double s = 0.0;
+#pragma unroll
+        for (int wv = 0; wv < 32; ++wv) s += red[wv * (m + 1) + t];
+        partA[(size_t)t * kMaxBlocks + vb] = s;
+      }
+      if (!all_clusters()) return;
+      gather_dots(it + 1);
+      // ---- w -= sum_j h_j v_j and its norm; beside it the earlier rotations of the column ----
+      if (own) {
+        double x = w;
+#pragma unroll 8
+        for (int j = 0; j <= it; ++j) x = x - coef[j] * U[j * us];
+        A.U[(size_t)(it + 1) * A.un + row] = x;
+        if (SMEM_U) U[(it + 1) * us] = x;
+        remote_store(cluster_addr(nrm + (row - r0), 0), x * x);
+      } else if (t == THREADS - 32) {
+        double *hh = hcol;
+        for (int j = 1; j <= it; ++j) {
+          const double t0 = hh[j - 1];
+          hh[j - 1] = cc[j - 1] * t0 + ss[j - 1] * hh[j];
+          hh[j] = cc[j - 1] * hh[j] - ss[j - 1] * t0;
+        }
+      }
+      publish_norm();
+      if (!all_clusters()) return;
+      // ---- Hessenberg / Givens (KSPGMRESUpdateHessenberg), every block alike, by the last
+      //      warp; beside it the rows' threads gather the next product ----
+      if (own && it + 1 < m) av = spmv(A.U + (size_t)(it + 1) * A.un);
+      const double nsq = warp == nwarp - 1 ? gather_norm() : 0.0;
+      if (t == THREADS - 32) {
+        const double tt = sqrt(nsq);
+        scale[it + 1] = tt != 0.0 ? 1.0 / tt : 1.0;
+        double *hh = hcol;
+        hh[it + 1] = tt;
+        double hapbnd = fabs(tt / grs[it]);
+        if (hapbnd > 1e-30) hapbnd = 1e-30;
+        const int hapend = tt < hapbnd;
+        int rs = 0;
+        double rr = s_res;
+        if (!hapend) {
+          const double q = sqrt(hh[it] * hh[it] + hh[it + 1] * hh[it + 1]);
+          if (q == 0.0) {
+            rs = KSP_DIVERGED_NULL;
+          } else {
+            cc[it] = hh[it] / q;
+            ss[it] = hh[it + 1] / q;
+            grs[it + 1] = -(ss[it] * grs[it]);
+            grs[it] = cc[it] * grs[it];
+            hh[it] = cc[it] * hh[it] + ss[it] * hh[it + 1];
+            rr = fabs(grs[it + 1]);
+          }
+        } else {
+          rr = 0.0;
+        }
+        s_flow[0] = rs;
+        s_flow[1] = hapend;
+        s_res = rr;
+      }
+      __syncthreads();
+      for (int j = t; j <= it; j += THREADS) HH[(size_t)it * hld + j] = hcol[j];
+      const int rs = s_flow[0], hapend = s_flow[1];
+      if (!rs) res = s_res;
+      ++it;
+      ++its;
+      if (rs) {
+        reason = rs;
+        break;
+      }
+      reason = converged_default(its, res, A.rtol, A.atol, A.dtol, ttol, rnorm0);
+      if (hapend) {
+        if (!reason) reason = KSP_DIVERGED_BREAKDOWN;
+        break;
+      }
+    }
+    // ---- KSPGMRESBuildSoln: back substitution, x += sum_j y_j v_j ----
+    const int last = it - 1;
+    if (last >= 0) {
+      __syncthreads();  // the last column is in HH
+      if (t == 0) {
+        double *y = sh;
+        const double hl = HH[(size_t)last * hld + last];
+        y[last] = hl != 0.0 ? grs[last] / hl : 0.0;
+        for (int ii = 1; ii <= last; ++ii) {
+          const int k = last - ii;
+          double s = grs[k];
+          for (int j = k + 1; j <= last; ++j) s -= HH[(size_t)j * hld + k] * y[j];
+          const double hkk = HH[(size_t)k * hld + k];
+          y[k] = hkk != 0.0 ? s / hkk : 0.0;
+        }
+        for (int j = 0; j <= last; ++j) coef[j] = y[j] * scale[j];
+      }
+      __syncthreads();
+      if (own) {
+        double s = 0.0;
+#pragma unroll 8
+        for (int j = 0; j <= last; ++j) s = s + coef[j] * U[j * us];
+        xi = xi + s;
+        A.x[row] = xi;
+      }
+    }
+    itcount += it;
+    if (itcount >= A.max_it) {
+      if (!reason) reason = KSP_DIVERGED_ITS;
+      break;
+    }
+    guess_zero = false;
+    cluster_barrier();
+    if (!all_clusters()) return;
+  }
+  if (blockIdx.x == 0 && t == 0) {
     *A.out_its = its;
     *A.out_reason = reason;
     *A.out_rnorm = res;
@@ -439,7 +802,8 @@ __global__ void zero_f64(int n, double *x) {
 // leaves without arriving (a flag that nothing sets), so the wait must run out.
 __global__ void bounded_wait_probe(GridBar *bar, int *err, long long limit) {
   if (blockIdx.x == 1) return;
-  grid_sync(bar, 2u, err, limit);
+  unsigned epoch = 0;
+  grid_sync(bar, 2u, epoch, err, limit);
 }
 
 }  // namespace
@@ -456,6 +820,7 @@ struct KrylovWork {
   float *a32 = nullptr;
   double *hh = nullptr;  // per-block Hessenberg slices of the large-restart kernel
   size_t hh_bytes = 0;
+  bool cg_set = false;  // gmres_cluster may take kCgSmemMax and clusters of 16
   int cap_n = 0;
   int occ64[2] = {0, 0}, occ32[2] = {0, 0};
 };
@@ -473,6 +838,88 @@ void apc_krylov_free(apc_context *c) {
   apc_free(c, k->hh);
   delete k;
   c->kw = nullptr;
+}
+
+// The solve on clusters (gmres_cluster) where it applies: `blocks` blocks of the persistent
+// kernel of at most 1024 rows, each taken by a cluster of the largest K whose shared memory
+// and co-residency allow it, at least 2, with the basis in shared memory if it fits for any
+// K.  *done says whether it was launched.  More rows keep the persistent kernel, whose blocks
+// then fill the SMs.  Measured, us per iteration, persistent kernel (with the same grid barrier)
+// and clusters: 4,096 rows 16.1 and 8.0, 20,322 rows 19.4 and 11.5, 32,768 rows 16.3 and 11.2.
+static int launch_gmres_cluster(apc_context *c, const GmresArgs<double> &g, int blocks, bool *done) {
+  KrylovWork *k = c->kw;
+  const int m = g.restart, rpb = (g.n + blocks - 1) / blocks;
+  *done = false;
+  if (rpb > 1024 || blocks > kCgMaxClusters) return APC_OK;
+  void (*const kern[2][3])(CgArgs) = {
+      {gmres_cluster<256, true>, gmres_cluster<512, true>, gmres_cluster<1024, true>},
+      {gmres_cluster<256, false>, gmres_cluster<512, false>, gmres_cluster<1024, false>}};
+  if (!k->cg_set) {
+    for (auto &fs : kern)
+      for (auto f : fs) {
+        APC_CUDA_TRY(c, cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kCgSmemMax));
+        APC_CUDA_TRY(c, cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+      }
+    k->cg_set = true;
+  }
+  for (int q = 0; q < 7; ++q) {  // 16, 8, 4 with the basis in shared memory; 16, 8, 4, 2 without
+    const int in_l2 = q >= 3, K = 16 >> (in_l2 ? q - 3 : q), v = std::min(in_l2 ? q - 3 : q, 2);
+    const size_t R = 1024 / (size_t)K, M = (size_t)m;
+    CgArgs C{};
+    C.g = g;
+    C.nvb = blocks;
+    C.rpb = rpb;
+    C.K = K;
+    size_t o = 0;
+    auto take = [&](size_t bytes) {
+      const size_t p = o;
+      o += (bytes + 15) & ~(size_t)15;
+      return (unsigned)p;
+    };
+    take((size_t)g.w * R * sizeof(double));
+    C.o_u = take(in_l2 ? 0 : (M + 1) * R * sizeof(double));
+    C.o_col = take((size_t)g.w * R * sizeof(int));
+    C.o_red = take(32 * (M + 1) * sizeof(double));
+    C.o_nrm = take(1024 * sizeof(double));
+    C.o_hh = take(m <= 31 ? (M + 1) * M * sizeof(double) : 0);
+    C.o_small = take((7 * (M + 2) + R) * sizeof(double));
+    if (o > kCgSmemMax) continue;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks * K);
+    cfg.blockDim = dim3(std::min(1024, 4096 / K));
+    cfg.dynamicSmemBytes = o;
+    cfg.stream = c->s;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = K;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeCooperative;
+    at[1].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int ncl = 0;
+    if (cudaOccupancyMaxActiveClusters(&ncl, kern[in_l2][v], &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      continue;
+    }
+    if (ncl < blocks) continue;
+    if (m > 31) {
+      const size_t hb = sizeof(double) * (size_t)blocks * K * (M + 1) * M;
+      if (hb > k->hh_bytes) {
+        apc_free(c, k->hh);
+        k->hh = nullptr;
+        APC_TRY(apc_alloc(c, (void **)&k->hh, hb));
+        k->hh_bytes = hb;
+      }
+      C.g.hh = k->hh;
+    }
+    cfg.numAttrs = 2;
+    APC_CUDA_TRY(c, cudaLaunchKernelEx(&cfg, kern[in_l2][v], C));
+    *done = true;
+    return APC_OK;
+  }
+  return APC_OK;
 }
 
 template <class T, bool RE>
@@ -540,7 +987,10 @@ static int launch_gmres(apc_context *c, int n, const T *val, const T *b, T *x, i
   a.out_rnorm = k->dres;
   void *args[] = {&a};
   APC_CUDA_TRY(c, cudaEventRecord(c->kev[0], c->s));
-  APC_CUDA_TRY(c, cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(kThreads), args, 0, c->s));
+  bool on_clusters = false;
+  if constexpr (std::is_same_v<T, double> && !RE) APC_TRY(launch_gmres_cluster(c, a, blocks, &on_clusters));
+  if (!on_clusters)
+    APC_CUDA_TRY(c, cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(kThreads), args, 0, c->s));
   APC_CUDA_TRY(c, cudaEventRecord(c->kev[1], c->s));
   apc_count_launch(c);
   int hi[2];

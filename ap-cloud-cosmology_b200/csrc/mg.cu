@@ -1184,31 +1184,10 @@ static bool cl_fits(ClArgs<V> &A) {
   return A.total + kClStatic <= kSmemMax;
 }
 
-__device__ __forceinline__ void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ unsigned cluster_rank() {
-  unsigned r;
-  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-
-__device__ __forceinline__ void remote_store(unsigned addr, float v) {
-  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
-}
-__device__ __forceinline__ void remote_store(unsigned addr, double v) {
-  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
-}
-
 // v to *p of every block of the cluster, the g lanes of a group taking the blocks in turn
 template <class V>
 __device__ __forceinline__ void cl_broadcast(V *p, V v, int sub, int g) {
-  const unsigned a = (unsigned)__cvta_generic_to_shared(p);
-  for (int d = sub; d < kClBlocks; d += g) {
-    unsigned ra;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(d));
-    remote_store(ra, v);
-  }
+  for (int d = sub; d < kClBlocks; d += g) remote_store(cluster_addr(p, d), v);
 }
 
 // The block's share of every level, packed: block r of the grid writes block r's image.
@@ -1492,9 +1471,10 @@ struct Grp {
   int rank, size;
   GridBar *bar;
   int *err;
+  mutable unsigned epoch;  // arrivals awaited at bar so far
 };
 
-__device__ __forceinline__ bool gsync(const Grp &g) { return grid_sync(g.bar, (unsigned)g.size, g.err); }
+__device__ __forceinline__ bool gsync(const Grp &g) { return grid_sync(g.bar, (unsigned)g.size, g.epoch, g.err); }
 
 __device__ __forceinline__ double p_block_sum(double v, double *red) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1923,7 +1903,7 @@ __device__ bool solve_body(const PSolveArgs<T> &A, const Grp &g, PShared &sh, do
 template <class T>
 __global__ void __launch_bounds__(kPT, 1) ir_solve_persistent(PSolveArgs<T> A) {
   __shared__ PShared sh;
-  const Grp g{(int)blockIdx.x, (int)gridDim.x, A.bar, A.err};
+  const Grp g{(int)blockIdx.x, (int)gridDim.x, A.bar, A.err, 0u};
   solve_body(A, g, sh, A.part);
 }
 
@@ -1938,7 +1918,7 @@ __global__ void __launch_bounds__(kPT, 1) ir_solve_batched(const PSolveArgs<T> *
   __shared__ PShared sh;
   __shared__ PSolveArgs<T> A;
   const int grp = blockIdx.x / gsize;
-  const Grp g{(int)(blockIdx.x % gsize), gsize, bars + grp, err};
+  const Grp g{(int)(blockIdx.x % gsize), gsize, bars + grp, err, 0u};
   double *part = parts + (size_t)grp * kPSlots * kPMaxBlocks;
   for (;;) {
     if (g.rank == 0 && threadIdx.x == 0) slot[grp] = atomicAdd(queue, 1);

@@ -299,7 +299,7 @@ int apc_device_code_version(int device, int *binary_version, int *ptx_version);
 
 /* Self-check of the library's bounded device waits (the grid barrier of the persistent
  * GMRES kernel).  Two blocks are launched on `device`; one leaves without arriving at
- * the barrier, so the other's wait runs out after spin_limit polls (each a ~64 ns sleep;
+ * the barrier, so the other's wait runs out after spin_limit polls (each a ~0.7 us read;
  * 1 <= spin_limit <= 2^24) and it raises the error and abort flags and returns, as the
  * solver kernels do.  Returns APC_ERR_TIMEOUT when the wait gave up (the designed
  * outcome), APC_OK if the barrier completed.  The device stays usable either way. */
