@@ -57,6 +57,8 @@ struct apc_context {
   cudaEvent_t cs_ev = nullptr, vel_ev = nullptr;  // c->s before the upload; upload done
   bool vel_caller_order = false;  // pvx.. hold the caller's order (a fresh upload), not the sorted one
   cudaMemPool_t pool = nullptr;  // the device's stream-ordered pool (all device buffers)
+  std::vector<char *> slabs;     // small buffers are cut from these (apc_alloc)
+  size_t slab_used = 0;          // bytes taken from the last one
   std::string err;
   int64_t launches = 0;
   bool have_particles = false, have_cells = false, have_fields = false;
