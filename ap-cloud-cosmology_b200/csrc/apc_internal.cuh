@@ -91,24 +91,22 @@ struct apc_context {
   int lcap = 0;                  // leaf hash capacity
   uint64_t *l_keys = nullptr;
   int *l_vals = nullptr;
-  int op_cap = 0;                // opened list capacity
   uint64_t *op_code = nullptr;   // opened nodes: td in BFS order, then balance events in order
   int *op_base = nullptr;        // temp index of the node's first child
   int *op_first = nullptr, *op_count = nullptr;  // particle range (all opened nodes)
   int n_open_td = 0, n_open = 0;
-  std::vector<int> td_level_off;  // [level] -> offset of level's td-opened nodes; size depth+2
-  uint64_t *req_key = nullptr, *req_key_alt = nullptr;  // balance requests: first-requester key
-  uint32_t *req_idx = nullptr, *req_idx_alt = nullptr;  //                   sort payload
-  uint64_t *req_code = nullptr;                         //                   requested cell
-  int *req_pos = nullptr;        // scan output of per-(node, octant) flags
+  int *r_list = nullptr;         // used slots of the two request tables
+  bool r_dirty = true;           // the request tables may hold entries
+  uint32_t *child_words = nullptr;  // one bit per child: two levels in turn, the leaves
+  int *leaf_base = nullptr;      // leaves before each word of the last
+  uint64_t *child_range = nullptr;  // particle range of a level's children (two ints each)
+  unsigned char *tree_out = nullptr;   // sizes of the tree, grid barrier, request counts
   long long maxnc_state = 10000; // temp-node budget, doubled like Mover::maxnc (mover.cpp:36-41)
   int *counters = nullptr;       // small device counters
   int *d_err = nullptr;          // device error flags
   int *h_pinned = nullptr;       // pinned host mirror for small readbacks
   int *scan_tmp = nullptr;
   int scan_tmp_cap = 0;
-  int *flags = nullptr;          // per-(opened node, octant) flags / scan
-  int flags_cap = 0;
   std::vector<int> numnodes;     // octree level sizes of the last build
 
   // ---- cells (Computational_particle) in the reference's output order ----

@@ -177,9 +177,9 @@ void free_all(apc_context *c) {
   void *ptrs[] = {c->px, c->py, c->pz, c->pvx, c->pvy, c->pvz, c->pax, c->pay, c->paz, c->pid,
                   c->qx, c->qy, c->qz, c->qvx, c->qvy, c->qvz, c->qid, c->keys, c->keys_alt, c->perm,
                   c->perm_alt, c->sort_hist, c->reduce_buf, c->h_keys, c->h_vals, c->r_keys, c->r_vals,
-                  c->l_keys, c->l_vals, c->op_code, c->op_base, c->op_first, c->op_count, c->req_key,
-                  c->req_key_alt, c->req_idx, c->req_idx_alt, c->req_code, c->req_pos, c->counters,
-                  c->d_err, c->scan_tmp, c->flags, c->cx, c->cy, c->cz, c->ch, c->cfirst, c->ccount,
+                  c->l_keys, c->l_vals, c->op_code, c->op_base, c->op_first, c->op_count, c->r_list,
+                  c->child_words, c->leaf_base, c->child_range, c->tree_out, c->counters,
+                  c->d_err, c->scan_tmp, c->cx, c->cy, c->cz, c->ch, c->cfirst, c->ccount,
                   c->ctype, c->ccode, c->nb24, c->nnb, c->cell_of, c->st_idx, c->st_dist, c->gfd_x,
                   c->ell_col, c->a1, c->a2, c->a1f, c->a2f, c->a1d, c->a2d, c->rhs, c->bcrhs, c->density, c->potential,
                   c->deriv, c->adj_ckpt, c->adj_tape, c->gfd_qr, c->full_keys, c->full_keys_alt, c->full_ids, c->full_ids_alt, c->warm_keys, c->warm_rho,
@@ -489,12 +489,6 @@ int apc_select(apc_context *c, int *n_cells) {
   c->step_open = true;
   APC_CUDA_TRY(c, cudaMemsetAsync(c->d_err, 0, sizeof(int), c->s));
   APC_TRY(apc_octree_build(c));
-  int derr = 0;
-  APC_TRY(apc_read_errors(c, &derr));
-  if (derr & DERR_NOT_FINITE) {
-    c->err = "non-finite particle coordinates";
-    return APC_ERR_NOT_FINITE;
-  }
   int rc = apc_selection(c);
   if (rc == APC_RETRY_FULL_SORT) {
     // the tree went deeper than the sort: sort by every bit and select again
@@ -503,9 +497,7 @@ int apc_select(apc_context *c, int *n_cells) {
     APC_TRY(apc_octree_build(c));
     rc = apc_selection(c);
   }
-  APC_TRY(rc);
-  APC_CUDA_TRY(c, cudaEventRecord(c->ev[1], c->s));
-  APC_CUDA_TRY(c, apc_event_wait(c->ev[1]));
+  APC_TRY(rc);  // its last read of the error flags came after ev[1]
   // the velocity upload ran beside the selection: once a phase call returns, the caller's
   // arrays are no longer read, as with the positions
   if (c->vel_caller_order) APC_CUDA_TRY(c, apc_event_wait(c->vel_ev));

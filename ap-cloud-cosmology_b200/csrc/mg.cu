@@ -2159,7 +2159,7 @@ static int mg_structure(apc_context *c) {
     if (lev == 0) {
       // parent codes of cells at level <= D have at most 3 D - 2 significant bits; the
       // deepest cell level is one below the deepest top-down opened level
-      const int deepest = (int)c->td_level_off.size();
+      const int deepest = c->levels_hint + 2;
       const int bits = std::min(64, 3 * deepest + 1);
       APC_TRY(apc_radix_sort_u64(c, m->pkey, m->pidx, m->pkey_alt, m->pidx_alt, nf, 0, bits, &alt));
     }

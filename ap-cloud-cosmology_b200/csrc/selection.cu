@@ -27,11 +27,17 @@
 // x+, x-, y+, y-, z+, z-.  A neighbour is one same-or-coarser cell or the 4 finer
 // cells on the shared face.
 //
+// The tree (top-down levels, balance sweeps, numbering of the leaves) is one cooperative
+// kernel, select_tree: its phases are separated by the bounded grid barrier (1.2 us) where
+// launches with a host read of each level's size took 20-30 us per level and sweep.  The host
+// reads the sizes once, sizes the cell arrays and queues the output kernels.
+//
 // Location code of a cell at level L with Morton prefix P: (1 << 3L) | P.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 
 #include "apc_internal.cuh"
 
@@ -73,62 +79,6 @@ __device__ __forceinline__ void cell_range(const uint64_t *keys, int n, int dept
   *count = b - a;
 }
 
-// ------------------------------------------------------------------ top-down
-
-__global__ void td_root(uint64_t *op_code, int *op_base, int *op_first, int *op_count, int n,
-                        uint64_t *hkeys, int *hvals, int hcap, int *err) {
-  op_code[0] = 1ull;
-  op_base[0] = 1;
-  op_first[0] = 0;
-  op_count[0] = n;
-  bool fresh;
-  int s = hash_insert(hkeys, hcap, 1ull, &fresh);
-  if (s < 0) atomicOr(err, DERR_HASH_FULL);
-  else hvals[s] = 0;
-}
-
-// children of the opened nodes [off, off+cnt) of level L: particle ranges and the
-// refinement test n*h^2 > c (octree.cpp:1165-1183)
-__global__ void td_expand(const uint64_t *__restrict__ keys, int depth, int L, int off, int cnt,
-                          const int *__restrict__ op_first, const int *__restrict__ op_count,
-                          double hchild, double c, int maxdepth, int *__restrict__ flags,
-                          int *__restrict__ cfirst, int *__restrict__ ccount) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 8 * cnt) return;
-  const int o = off + (t >> 3), ch = t & 7;
-  const int lo = op_first[o], hi = lo + op_count[o];
-  const int shift = 3 * (depth - L - 1);
-  const int a = lower_digit(keys, lo, hi, shift, ch);
-  const int b = lower_digit(keys, a, hi, shift, ch + 1);
-  const int np = b - a;
-  double temp = 1.0 * np;
-  temp = __dmul_rn(temp, hchild);
-  temp = __dmul_rn(temp, hchild);
-  flags[t] = (temp > c) && (L + 1 < maxdepth);
-  cfirst[t] = a;
-  ccount[t] = np;
-}
-
-__global__ void td_compact(int off, int cnt, int off_next, const int *__restrict__ flags,
-                           const int *__restrict__ pos, const int *__restrict__ cfirst,
-                           const int *__restrict__ ccount, uint64_t *op_code, int *op_base,
-                           int *op_first, int *op_count, uint64_t *hkeys, int *hvals, int hcap,
-                           int *err) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 8 * cnt || !flags[t]) return;
-  const int o = off + (t >> 3);
-  const int q = off_next + pos[t];
-  const uint64_t code = (op_code[o] << 3) | (uint64_t)(t & 7);
-  op_code[q] = code;
-  op_base[q] = 1 + 8 * q;
-  op_first[q] = cfirst[t];
-  op_count[q] = ccount[t];
-  bool fresh;
-  int s = hash_insert(hkeys, hcap, code, &fresh);
-  if (s < 0) atomicOr(err, DERR_HASH_FULL);
-  else hvals[s] = q;
-}
-
 // ------------------------------------------------------------------ balance
 
 __device__ __forceinline__ bool neighbour_code(uint64_t code, int L, int di, int bc, uint64_t *out) {
@@ -156,96 +106,390 @@ __device__ __forceinline__ bool neighbour_code(uint64_t code, int L, int di, int
   return true;
 }
 
-// sweep ln: every node of level ln (children of opened nodes of level ln-1) requests the
-// opening of the coarse cells that break 2:1 across its six faces
-__global__ void bal_requests(int ln, int td_a, int td_b, int bal_a, int bal_b, int bc,
-                             const uint64_t *__restrict__ op_code, const int *__restrict__ op_base,
-                             const uint64_t *__restrict__ hkeys, int hcap, uint64_t *rkeys,
-                             unsigned long long *rvals, int rcap, int *err) {
-  const int ntd = td_b - td_a, nbal = bal_b - bal_a;
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 8 * (ntd + nbal)) return;
-  const int r = t >> 3, ch = t & 7;
-  const int o = r < ntd ? td_a + r : bal_a + (r - ntd);
-  const uint64_t pcode = op_code[o];
+// ------------------------------------------------------------------ the tree
+
+constexpr int kTreeThreads = 512;
+constexpr int kTreeWarps = kTreeThreads / 32;
+constexpr int kTreeLevels = 24;
+
+// what the host reads back: the sizes, and why the kernel stopped early
+enum : int { TREE_FULL = 1, TREE_DEEPER = 2 };
+struct TreeOut {
+  int stop;                 // TREE_* bits: a table was full, the sort was too shallow
+  int maxlev;               // level of the last temp node (octree.cpp:1792 ml)
+  int n_open_td, n_open;    // opened nodes: top-down, all
+  int nc;                   // leaves of top-down opened nodes (Type 0 cells)
+};
+
+struct TreeArgs {
+  const uint64_t *keys;
+  int n, depth, sorted_levels, bc;
+  double h0, c;
+  uint64_t *hkeys;          // opened-node hash
+  int *hvals;
+  int hcap;                 // at most hcap / 2 nodes are opened
+  uint64_t *rkeys[2];       // balance requests: two tables, used in turn, empty between selections
+  unsigned long long *rvals[2];
+  int *rlist[2];            // their used slots
+  int rcap;
+  uint64_t *op_code;
+  int *op_base, *op_first, *op_count;
+  uint32_t *words[2];       // one bit per child, in child order
+  int2 *crange;             // particle range of each child of the level in hand
+  uint32_t *leaf;           // one bit per child of every opened node: a leaf
+  int *leaf_base;           // leaves before each word
+  int *nreq;                // requests of each sweep, zeroed before the launch
+  TreeOut *out;
+  GridBar *bar;
+  int *err;
+};
+
+// first index in [lo, hi) whose digit ((key >> shift) & 7) >= d, by a warp: 32 probes a round
+__device__ __forceinline__ int warp_lower_digit(const uint64_t *keys, int lo, int hi, int shift, int d, int lane) {
+  while (hi - lo > 0) {
+    const int step = (hi - lo + 31) / 32;
+    const int p = min(lo + lane * step, hi - 1);  // probes ascend, the first is lo
+    const bool below = (int)((keys[p] >> shift) & 7ull) < d;
+    const int k = __popc(__ballot_sync(0xffffffffu, below));  // a prefix of the lanes is below
+    if (k == 0) return lo;
+    const int nlo = min(lo + (k - 1) * step, hi - 1) + 1;
+    const int nhi = k < 32 ? min(lo + k * step, hi) : hi;
+    lo = nlo;
+    hi = max(nlo, nhi);
+  }
+  return lo;
+}
+
+// sum over the block of v, in every thread
+__device__ __forceinline__ int tree_block_sum(int v, int *sm) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  v = __reduce_add_sync(0xffffffffu, v);
+  __syncthreads();
+  if (lane == 0) sm[warp] = v;
+  __syncthreads();
+  return __reduce_add_sync(0xffffffffu, lane < kTreeWarps ? sm[lane] : 0);
+}
+
+// exclusive sum over the block's threads; *total is the block's sum
+__device__ __forceinline__ int tree_block_scan(int v, int *sm, int *total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int incl = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  __syncthreads();
+  if (lane == 31) sm[warp] = incl;
+  __syncthreads();
+  const int w = lane < kTreeWarps ? sm[lane] : 0;
+  *total = __reduce_add_sync(0xffffffffu, w);
+  return incl - v + __reduce_add_sync(0xffffffffu, lane < warp ? w : 0);
+}
+
+// One sweep ln's requests by one (opened node, child) pair: the child, a node of level ln,
+// requests the opening of the coarse cells that break 2:1 across its six faces.
+__device__ __forceinline__ void request_openings(const TreeArgs &A, int ln, int o, int ch, int tab) {
+  const uint64_t pcode = A.op_code[o];
   if (code_level(pcode) != ln - 1) return;
   const uint64_t code = (pcode << 3) | (uint64_t)ch;
-  const unsigned long long tidx = (unsigned long long)(op_base[o] + ch);
+  const unsigned long long tidx = (unsigned long long)(A.op_base[o] + ch);
   for (int di = 0; di < 6; ++di) {
     uint64_t nc;
-    if (!neighbour_code(code, ln, di, bc, &nc)) continue;
-    if (ln >= 2 && hash_find(hkeys, hcap, nc >> 6) >= 0) continue;  // leaf at level >= ln-1
+    if (!neighbour_code(code, ln, di, A.bc, &nc)) continue;
+    if (ln >= 2 && hash_find(A.hkeys, A.hcap, nc >> 6) >= 0) continue;  // leaf at level >= ln-1
     int lstar = 0;
     for (int l = ln - 3; l >= 0; --l)
-      if (hash_find(hkeys, hcap, nc >> (3 * (ln - l))) >= 0) { lstar = l; break; }
+      if (hash_find(A.hkeys, A.hcap, nc >> (3 * (ln - l))) >= 0) { lstar = l; break; }
     for (int l = lstar + 1; l <= ln - 2; ++l) {
       const uint64_t target = nc >> (3 * (ln - l));
       const unsigned long long key = (tidx << 8) | ((unsigned long long)di << 5) | (unsigned long long)l;
       bool fresh;
-      int s = hash_insert(rkeys, rcap, target, &fresh);
-      if (s < 0) { atomicOr(err, DERR_HASH_FULL); continue; }
-      atomicMin(&rvals[s], key);
+      const int s = hash_insert(A.rkeys[tab], A.rcap, target, &fresh);
+      if (s < 0) {
+        atomicOr(A.err, DERR_HASH_FULL);
+        continue;
+      }
+      if (fresh) {
+        const int q = atomicAdd(&A.nreq[ln], 1);
+        if (q < A.rcap / 2) A.rlist[tab][q] = s;
+      }
+      atomicMin(&A.rvals[tab][s], key);
     }
   }
 }
 
-__global__ void bal_collect(const uint64_t *__restrict__ rkeys, const unsigned long long *__restrict__ rvals,
-                            int rcap, int *count, uint64_t *out_key, uint32_t *out_idx,
-                            uint64_t *out_code) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= rcap) return;
-  uint64_t k = rkeys[s];
-  if (!k) return;
-  int q = atomicAdd(count, 1);
-  out_key[q] = rvals[s];
-  out_idx[q] = (uint32_t)q;
-  out_code[q] = k;
+__device__ __forceinline__ void open_node(const TreeArgs &A, int q, uint64_t code, int base, int first, int count) {
+  A.op_code[q] = code;
+  A.op_base[q] = base;
+  A.op_first[q] = first;
+  A.op_count[q] = count;
+  bool fresh;
+  const int s = hash_insert(A.hkeys, A.hcap, code, &fresh);
+  if (s < 0) atomicOr(A.err, DERR_HASH_FULL);
+  else A.hvals[s] = q;
 }
 
-__global__ void bal_commit(int nreq, int n_open, int child_base0, const uint32_t *__restrict__ order,
-                           const uint64_t *__restrict__ codes, const uint64_t *__restrict__ keys,
-                           int n, int depth, uint64_t *op_code, int *op_base, int *op_first,
-                           int *op_count, uint64_t *hkeys, int *hvals, int hcap, int *err) {
-  int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= nreq) return;
-  const int q = n_open + r;
-  const uint64_t code = codes[order[r]];
-  op_code[q] = code;
-  op_base[q] = child_base0 + 8 * r;
-  int f, cnt;
-  cell_range(keys, n, depth, code, &f, &cnt);
-  op_first[q] = f;
-  op_count[q] = cnt;
-  bool fresh;
-  int s = hash_insert(hkeys, hcap, code, &fresh);
-  if (s < 0) atomicOr(err, DERR_HASH_FULL);
-  else hvals[s] = q;
+// The opened nodes of the octree (top-down refinement, then the 2:1 balance) in the
+// reference's temp-node order, and the numbering of their leaves.  The root is open (the host
+// tests it).  Every block takes the same branches: the counts it branches on are read after a
+// barrier.  What bounds it is the chain of ~4 barriers and dependent key probes per level.
+__global__ void __launch_bounds__(kTreeThreads) select_tree(const __grid_constant__ TreeArgs A) {
+  __shared__ int sm[kTreeWarps], off_s[kTreeLevels + 1], s_base[kTreeThreads];
+  __shared__ uint32_t s_word[kTreeThreads];
+  __shared__ unsigned long long s_key[kTreeThreads];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int G = gridDim.x, b = blockIdx.x;
+  const int gthreads = G * kTreeThreads, gt = b * kTreeThreads + t;
+  const int gwarps = G * kTreeWarps, gwarp = b * kTreeWarps + warp;
+  unsigned epoch = 0;
+  int stop = 0;
+
+  // the bits of words [0, nwords) before the block's share [w0, w1), and in all
+  auto share = [&](const uint32_t *words, int nwords, int &w0, int &w1, int &before, int &total) {
+    const int per = (nwords + G - 1) / G;
+    w0 = min(nwords, b * per);
+    w1 = min(nwords, w0 + per);
+    int lo = 0, all = 0;
+    for (int w = t; w < nwords; w += kTreeThreads) {
+      const int p = __popc(__ldcg(words + w));
+      all += p;
+      if (w < w0) lo += p;
+    }
+    before = tree_block_sum(lo, sm);
+    total = tree_block_sum(all, sm);
+  };
+  auto finish = [&](int maxlev, int n_open_td, int n_open) {
+    if (b == 0 && t == 0) {
+      A.out->stop = stop;
+      A.out->maxlev = maxlev;
+      A.out->n_open_td = n_open_td;
+      A.out->n_open = n_open;
+    }
+  };
+
+  if (b == 0) {
+    if (t == 0) {
+      open_node(A, 0, 1ull, 1, 0, A.n);
+      A.words[0][0] = 0u;
+    }
+  }
+  if (t == 0) {
+    off_s[0] = 0;
+    off_s[1] = 1;
+  }
+  if (!grid_sync(A.bar, G, epoch, A.err)) return;
+
+  // ---- top-down, level by level ----
+  int off = 0, cnt = 1, n_open = 1, maxlev = 0, cur = 0;
+  double hchild = A.h0;
+  for (int L = 0; L < A.depth && cnt > 0; ++L) {
+    // children at level L + 1 need the particles sorted by that many levels of key bits
+    if (L + 1 > A.sorted_levels) {
+      stop |= TREE_DEEPER;
+      break;
+    }
+    maxlev = L + 1;
+    hchild *= 0.5;  // exact: h0 2^-(L + 1)
+    const int m8 = 8 * cnt, shift = 3 * (A.depth - L - 1);
+    uint32_t *words = A.words[cur];
+    const bool deeper = L + 1 < A.depth;
+    // particle ranges of the children and the refinement test n h^2 > c (octree.cpp:1165-1183)
+    auto opens = [&](int np) {
+      double v = 1.0 * np;
+      v = __dmul_rn(v, hchild);
+      v = __dmul_rn(v, hchild);
+      return v > A.c && deeper;
+    };
+    if (m8 <= gwarps) {
+      // few children with long ranges: a warp per child (words zeroed beforehand)
+      for (int q = gwarp; q < m8; q += gwarps) {
+        const int o = off + (q >> 3), ch = q & 7;
+        const int lo = A.op_first[o], hi = lo + A.op_count[o];
+        const int a = warp_lower_digit(A.keys, lo, hi, shift, ch, lane);
+        const int e = ch == 7 ? hi : warp_lower_digit(A.keys, a, hi, shift, ch + 1, lane);
+        if (lane == 0) {
+          A.crange[q] = make_int2(a, e - a);
+          if (opens(e - a)) atomicOr(words + (q >> 5), 1u << (q & 31));
+        }
+      }
+    } else {
+      const int rounds = (m8 + gthreads - 1) / gthreads;
+      for (int r = 0; r < rounds; ++r) {
+        const int q = r * gthreads + gt;  // a warp's lanes share a word
+        const bool act = q < m8;
+        int a = 0, hi = 0;
+        if (act) {
+          const int o = off + (q >> 3);
+          const int lo = A.op_first[o];
+          hi = lo + A.op_count[o];
+          a = lower_digit(A.keys, lo, hi, shift, q & 7);
+        }
+        const int nxt = __shfl_down_sync(0xffffffffu, a, 1);
+        const int np = ((q & 7) == 7 ? hi : nxt) - a;
+        const bool f = act && opens(np);
+        if (f) A.crange[q] = make_int2(a, np);
+        const unsigned bal = __ballot_sync(0xffffffffu, f);
+        if (lane == 0 && act) words[q >> 5] = bal;
+      }
+    }
+    if (!grid_sync(A.bar, G, epoch, A.err)) return;
+    // the opened children in order: their place is the number of opened children before them
+    const int nwords = (m8 + 31) / 32, off_next = off + cnt;
+    int w0, w1, before, total;
+    share(words, nwords, w0, w1, before, total);
+    if (2ll * (off_next + total) > A.hcap) {
+      stop |= TREE_FULL;
+      break;
+    }
+    for (int wb = w0; wb < w1; wb += kTreeThreads) {
+      const uint32_t word = wb + t < w1 ? __ldcg(words + wb + t) : 0u;
+      int sum;
+      const int ex = tree_block_scan(__popc(word), sm, &sum);
+      s_base[t] = before + ex;
+      s_word[t] = word;
+      __syncthreads();
+      const int items = min(kTreeThreads, w1 - wb) * 32;
+      for (int i = t; i < items; i += kTreeThreads) {
+        const uint32_t wd = s_word[i >> 5];
+        if (!((wd >> (i & 31)) & 1u)) continue;
+        const int q = wb * 32 + i, o = off + (q >> 3);
+        const int at = off_next + s_base[i >> 5] + __popc(wd & ((1u << (i & 31)) - 1u));
+        const int2 rg = A.crange[q];
+        open_node(A, at, (A.op_code[o] << 3) | (uint64_t)(q & 7), 1 + 8 * at, rg.x, rg.y);
+      }
+      before += sum;
+      __syncthreads();
+    }
+    cur ^= 1;
+    if (8 * total <= gwarps)
+      for (int w = gt; w < (8 * total + 31) / 32; w += gthreads) A.words[cur][w] = 0u;
+    off = off_next;
+    cnt = total;
+    n_open = off + cnt;
+    if (t == 0 && L + 2 <= kTreeLevels) off_s[L + 2] = n_open;
+    if (!grid_sync(A.bar, G, epoch, A.err)) return;
+  }
+  const int n_open_td = n_open, child_base = 1 + 8 * n_open_td;
+
+  // ---- bottom-up 2:1 balance, sweeps ln = maxlev .. 2 ----
+  int tab = 0, dirty[2] = {0, 0};
+  for (int ln = maxlev; ln > 1 && !stop; --ln) {
+    const int td_a = off_s[ln - 1], ntd = off_s[ln] - td_a, nbal = n_open - n_open_td;
+    for (int q = gt; q < 8 * (ntd + nbal); q += gthreads) {
+      const int r = q >> 3;
+      request_openings(A, ln, r < ntd ? td_a + r : n_open_td + (r - ntd), q & 7, tab);
+    }
+    if (!grid_sync(A.bar, G, epoch, A.err)) return;
+    const int nreq = __ldcg(A.nreq + ln);
+    if (nreq == 0) continue;
+    if (nreq > A.rcap / 2 || 2ll * (n_open + nreq) > A.hcap) {
+      stop |= TREE_FULL;
+      break;
+    }
+    // a request's place is its rank by first requester: few requests (a percent of the cells
+    // at most in the collapse runs), so each counts the smaller keys
+    const int *list = A.rlist[tab];
+    const unsigned long long *vals = A.rvals[tab];
+    const int rounds = (nreq + gthreads - 1) / gthreads;
+    for (int r = 0; r < rounds; ++r) {
+      if (r * gthreads + b * kTreeThreads >= nreq) continue;  // no request of this block's
+      const int i = r * gthreads + gt;
+      const int slot = i < nreq ? __ldcg(list + i) : 0;
+      const unsigned long long key = i < nreq ? __ldcg(vals + slot) : 0ull;
+      int rank = 0;
+      for (int j0 = 0; j0 < nreq; j0 += kTreeThreads) {
+        __syncthreads();
+        if (j0 + t < nreq) s_key[t] = __ldcg(vals + __ldcg(list + j0 + t));
+        __syncthreads();
+        const int jn = min(kTreeThreads, nreq - j0);
+        for (int j = 0; j < jn; ++j) rank += s_key[j] < key ? 1 : 0;
+      }
+      if (i < nreq) {
+        const uint64_t code = A.rkeys[tab][slot];
+        int f, cn;
+        cell_range(A.keys, A.n, A.depth, code, &f, &cn);
+        open_node(A, n_open + rank, code, child_base + 8 * (n_open - n_open_td + rank), f, cn);
+      }
+    }
+    n_open += nreq;
+    dirty[tab] = nreq;
+    // the other table's entries of the sweep before are no longer read: empty it
+    tab ^= 1;
+    for (int i = gt; i < dirty[tab]; i += gthreads) {
+      const int slot = __ldcg(A.rlist[tab] + i);
+      A.rkeys[tab][slot] = 0ull;
+      A.rvals[tab][slot] = ~0ull;
+    }
+    dirty[tab] = 0;
+    if (!grid_sync(A.bar, G, epoch, A.err)) return;
+  }
+  tab ^= 1;  // the last table used
+  for (int i = gt; i < dirty[tab] && !stop; i += gthreads) {
+    const int slot = __ldcg(A.rlist[tab] + i);
+    A.rkeys[tab][slot] = 0ull;
+    A.rvals[tab][slot] = ~0ull;
+  }
+  if (stop) {
+    finish(maxlev, n_open_td, n_open);
+    return;
+  }
+
+  // ---- the leaves: unopened children of opened nodes ----
+  const int m8 = 8 * n_open, nwords = (m8 + 31) / 32;
+  for (int r = 0; r < (m8 + gthreads - 1) / gthreads; ++r) {
+    const int q = r * gthreads + gt;
+    const bool f = q < m8 && hash_find(A.hkeys, A.hcap, (A.op_code[q >> 3] << 3) | (uint64_t)(q & 7)) < 0;
+    const unsigned bal = __ballot_sync(0xffffffffu, f);
+    if (lane == 0 && q < m8) A.leaf[q >> 5] = bal;
+  }
+  if (!grid_sync(A.bar, G, epoch, A.err)) return;
+  int w0, w1, before, total;
+  share(A.leaf, nwords, w0, w1, before, total);
+  const int split = 8 * n_open_td;  // children of top-down opened nodes
+  if (b == 0 && t == 0 && (split >> 5) >= nwords) A.out->nc = total;
+  for (int wb = w0; wb < w1; wb += kTreeThreads) {
+    const uint32_t word = wb + t < w1 ? __ldcg(A.leaf + wb + t) : 0u;
+    int sum;
+    const int ex = tree_block_scan(__popc(word), sm, &sum);
+    if (wb + t < w1) {
+      A.leaf_base[wb + t] = before + ex;
+      if (wb + t == split >> 5) A.out->nc = before + ex + __popc(word & ((1u << (split & 31)) - 1u));
+    }
+    before += sum;
+  }
+  finish(maxlev, n_open_td, n_open);
 }
 
 // ------------------------------------------------------------------ output
 
-__global__ void leaf_flags(int n_open, const uint64_t *__restrict__ op_code,
-                           const uint64_t *__restrict__ hkeys, int hcap, int *flags) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 8 * n_open) return;
-  const uint64_t child = (op_code[t >> 3] << 3) | (uint64_t)(t & 7);
-  flags[t] = hash_find(hkeys, hcap, child) < 0;
-}
-
 // cell centre by replaying the reference's parent-centre +- h/4 recursion from the root
 // (octree.cpp:1233-1235 and siblings), so that every rounding step is the same
-__global__ void leaf_emit(int n_open, int n_open_td, const int *__restrict__ flags,
-                          const int *__restrict__ pos, const uint64_t *__restrict__ op_code,
-                          const uint64_t *__restrict__ keys, int n, int depth, double cx0,
+__global__ void leaf_emit(int n_open, int n_open_td, const uint32_t *__restrict__ leaf,
+                          const int *__restrict__ leaf_base, const uint64_t *__restrict__ op_code,
+                          const int *__restrict__ op_first, const int *__restrict__ op_count,
+                          const uint64_t *__restrict__ keys, int depth, double cx0,
                           double cy0, double cz0, double hx0, double hy0, double hz0, double h0,
                           double *cx, double *cy, double *cz, double *ch, int *cfirst, int *ccount,
                           int *ctype, uint64_t *ccode, uint64_t *lkeys, int *lvals, int lcap,
                           int *err) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 8 * n_open || !flags[t]) return;
-  const int i = pos[t];
-  const uint64_t code = (op_code[t >> 3] << 3) | (uint64_t)(t & 7);
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  // the child's first particle, searched in its parent's range; its end is the next child's
+  const bool in = t < 8 * n_open;
+  const uint64_t code = in ? (op_code[t >> 3] << 3) | (uint64_t)(t & 7) : 8ull;
   const int L = code_level(code);
+  int f = 0, end = 0;
+  if (in) {
+    f = op_first[t >> 3];
+    end = f + op_count[t >> 3];
+    f = lower_digit(keys, f, end, 3 * (depth - L), t & 7);
+  }
+  const int next = __shfl_down_sync(0xffffffffu, f, 1);
+  if (!in) return;
+  const uint32_t word = leaf[t >> 5];
+  if (!((word >> (t & 31)) & 1u)) return;
+  const int i = leaf_base[t >> 5] + __popc(word & ((1u << (t & 31)) - 1u));
+  const int c = ((t & 7) == 7 ? end : next) - f;
   double x = cx0, y = cy0, z = cz0;
   for (int l = 0; l < L; ++l) {
     const unsigned dgt = (unsigned)((code >> (3 * (L - 1 - l))) & 7ull);
@@ -258,8 +502,6 @@ __global__ void leaf_emit(int n_open, int n_open_td, const int *__restrict__ fla
   cy[i] = y;
   cz[i] = z;
   ch[i] = ldexp(h0, -L);
-  int f, c;
-  cell_range(keys, n, depth, code, &f, &c);
   cfirst[i] = f;
   ccount[i] = c;
   ctype[i] = (t >> 3) < n_open_td ? 0 : -1;
@@ -322,41 +564,6 @@ int grid_for(long long n) { return (int)std::max<long long>(1, (n + kT - 1) / kT
 
 }  // namespace
 
-static int read_int(apc_context *c, const int *dev, int *host) {
-  APC_CUDA_TRY(c, cudaMemcpyAsync(c->h_pinned, dev, sizeof(int), cudaMemcpyDeviceToHost, c->s));
-  APC_CUDA_TRY(c, apc_stream_wait(c));
-  *host = c->h_pinned[0];
-  return APC_OK;
-}
-
-static int ensure_open_cap(apc_context *c, long long need) {
-  if (need <= c->op_cap) return APC_OK;
-  long long cap = std::max<long long>(need, 2ll * c->op_cap);
-  // grow preserving contents
-  uint64_t *nc = nullptr;
-  int *nb = nullptr, *nf = nullptr, *nn = nullptr;
-  APC_TRY(apc_alloc(c, (void **)&nc, sizeof(uint64_t) * cap));
-  APC_TRY(apc_alloc(c, (void **)&nb, sizeof(int) * cap));
-  APC_TRY(apc_alloc(c, (void **)&nf, sizeof(int) * cap));
-  APC_TRY(apc_alloc(c, (void **)&nn, sizeof(int) * cap));
-  if (c->op_cap > 0) {
-    APC_CUDA_TRY(c, cudaMemcpyAsync(nc, c->op_code, sizeof(uint64_t) * c->op_cap, cudaMemcpyDeviceToDevice, c->s));
-    APC_CUDA_TRY(c, cudaMemcpyAsync(nb, c->op_base, sizeof(int) * c->op_cap, cudaMemcpyDeviceToDevice, c->s));
-    APC_CUDA_TRY(c, cudaMemcpyAsync(nf, c->op_first, sizeof(int) * c->op_cap, cudaMemcpyDeviceToDevice, c->s));
-    APC_CUDA_TRY(c, cudaMemcpyAsync(nn, c->op_count, sizeof(int) * c->op_cap, cudaMemcpyDeviceToDevice, c->s));
-    apc_free(c, c->op_code);
-    apc_free(c, c->op_base);
-    apc_free(c, c->op_first);
-    apc_free(c, c->op_count);
-  }
-  c->op_code = nc;
-  c->op_base = nb;
-  c->op_first = nf;
-  c->op_count = nn;
-  c->op_cap = (int)cap;
-  return APC_OK;
-}
-
 static int ensure_hash(apc_context *c, uint64_t **keys, void **vals, size_t val_size, int *cap, int want) {
   if (want > *cap) {
     apc_free(c, *keys);
@@ -370,143 +577,131 @@ static int ensure_hash(apc_context *c, uint64_t **keys, void **vals, size_t val_
   return APC_OK;
 }
 
-// One attempt at the whole selection with the current hash capacities.
+// The selection's buffers for tables of `want` slots.  The request tables hold one entry per
+// coarse cell to be opened, a small part of the opened nodes.
+static int ensure_tree(apc_context *c, int want) {
+  if (!c->tree_out)
+    APC_TRY(apc_alloc(c, (void **)&c->tree_out, sizeof(TreeOut) + sizeof(GridBar) + kTreeLevels * sizeof(int)));
+  if (want <= c->hcap) return APC_OK;
+  APC_TRY(ensure_hash(c, &c->h_keys, (void **)&c->h_vals, sizeof(int), &c->hcap, want));
+  const size_t open = (size_t)want / 2, rcap = std::max<size_t>(1 << 16, (size_t)want / 4);
+  APC_TRY(apc_ensure(c, &c->op_code, open));
+  APC_TRY(apc_ensure(c, &c->op_base, open));
+  APC_TRY(apc_ensure(c, &c->op_first, open));
+  APC_TRY(apc_ensure(c, &c->op_count, open));
+  APC_TRY(apc_ensure(c, &c->r_keys, 2 * rcap));
+  APC_TRY(apc_ensure(c, &c->r_vals, 2 * rcap));
+  APC_TRY(apc_ensure(c, &c->r_list, rcap));
+  APC_TRY(apc_ensure(c, &c->child_words, 3 * (open / 4)));
+  APC_TRY(apc_ensure(c, &c->leaf_base, open / 4));
+  APC_TRY(apc_ensure(c, &c->child_range, 8 * open));
+  c->rcap = (int)rcap;
+  c->r_dirty = true;
+  return APC_OK;
+}
+
+// One attempt at the whole selection with the current table capacities.
 static int select_once(apc_context *c, int *hash_full) {
   const int n = c->n, D = c->cfg.depth;
   const double cc = c->cfg.gfd_c;
   *hash_full = 0;
-  APC_CUDA_TRY(c, cudaMemsetAsync(c->d_err, 0, sizeof(int), c->s));
-  APC_CUDA_TRY(c, cudaMemsetAsync(c->h_keys, 0, sizeof(uint64_t) * c->hcap, c->s));
 
   // ---- level 0 (octree.cpp:1114-1160, 1165-1183) ----
   double temp = 1.0 * n;
   temp = temp * c->h0;
   temp = temp * c->h0;
-  const bool root_open = n > 0 && temp > cc && 0 < D;
-  c->td_level_off.assign(1, 0);
-  APC_TRY(ensure_open_cap(c, 1024));
-  int n_open = 0;
-  if (root_open) {
-    td_root<<<1, 1, 0, c->s>>>(c->op_code, c->op_base, c->op_first, c->op_count, n, c->h_keys,
-                               c->h_vals, c->hcap, c->d_err);
-    apc_count_launch(c);
-    n_open = 1;
-  }
-  c->td_level_off.push_back(n_open);
-
-  // ---- top-down, level by level ----
-  int maxlev = 0;  // level of the last temp node (octree.cpp:1792 ml)
-  for (int L = 0; L < D; ++L) {
-    const int off = c->td_level_off[L], cnt = c->td_level_off[L + 1] - off;
-    if (cnt == 0) break;
-    // children at level L + 1 need the particles sorted by that many levels of key bits
-    if (L + 1 > c->sorted_levels) return APC_RETRY_FULL_SORT;
-    maxlev = L + 1;
-    const long long m8 = 8ll * cnt;
-    APC_TRY(apc_ensure(c, &c->flags, (size_t)(3 * m8 + 1), nullptr));
-    int *flg = c->flags, *cf = c->flags + m8, *cn = c->flags + 2 * m8;
-    APC_TRY(apc_ensure(c, &c->scan_tmp, 16, nullptr));
-    const double hchild = ldexp(c->h0, -(L + 1));
-    td_expand<<<grid_for(m8), kT, 0, c->s>>>(c->keys, D, L, off, cnt, c->op_first, c->op_count,
-                                              hchild, cc, D, flg, cf, cn);
-    apc_count_launch(c);
-    APC_CUDA_TRY(c, cudaGetLastError());
-    int *pos = nullptr;
-    APC_TRY(apc_ensure(c, &c->req_pos, (size_t)m8 + 1, nullptr));
-    pos = c->req_pos;
-    APC_TRY(apc_exclusive_scan(c, flg, pos, (int)m8, c->counters));
-    int total = 0;
-    APC_TRY(read_int(c, c->counters, &total));
-    const int off_next = off + cnt;
-    APC_TRY(ensure_open_cap(c, (long long)off_next + total + 1));
-    if (total > 0) {
-      td_compact<<<grid_for(m8), kT, 0, c->s>>>(off, cnt, off_next, flg, pos, cf, cn, c->op_code,
-                                                 c->op_base, c->op_first, c->op_count, c->h_keys,
-                                                 c->h_vals, c->hcap, c->d_err);
-      apc_count_launch(c);
-    }
-    c->td_level_off.push_back(off_next + total);
-  }
-  const int n_open_td = c->td_level_off.back();
-  c->n_open_td = n_open_td;
-  c->levels_hint = maxlev;
-  n_open = n_open_td;
-  const int child_base_bal = 1 + 8 * n_open_td;  // j after the top-down sweep
-
-  // ---- bottom-up 2:1 balance, sweeps ln = maxlev .. 2 ----
-  int n_events = 0;
-  for (int ln = maxlev; ln > 1; --ln) {
-    const int lv = ln - 1;
-    const int td_a = lv < (int)c->td_level_off.size() - 1 ? c->td_level_off[lv] : n_open_td;
-    const int td_b = lv < (int)c->td_level_off.size() - 1 ? c->td_level_off[lv + 1] : n_open_td;
-    const int bal_a = n_open_td, bal_b = n_open;
-    const long long nthreads = 8ll * ((td_b - td_a) + (bal_b - bal_a));
-    if (nthreads == 0) continue;
-    APC_CUDA_TRY(c, cudaMemsetAsync(c->r_keys, 0, sizeof(uint64_t) * c->rcap, c->s));
-    APC_CUDA_TRY(c, cudaMemsetAsync(c->r_vals, 0xff, sizeof(uint64_t) * c->rcap, c->s));
-    bal_requests<<<grid_for(nthreads), kT, 0, c->s>>>(ln, td_a, td_b, bal_a, bal_b, c->cfg.bc, c->op_code,
-                                                      c->op_base, c->h_keys, c->hcap, c->r_keys,
-                                                      (unsigned long long *)c->r_vals, c->rcap, c->d_err);
-    apc_count_launch(c);
-    APC_CUDA_TRY(c, cudaGetLastError());
-    APC_CUDA_TRY(c, cudaMemsetAsync(c->counters, 0, sizeof(int), c->s));
-    APC_TRY(apc_ensure(c, &c->req_key, (size_t)c->rcap, nullptr));
-    APC_TRY(apc_ensure(c, &c->req_key_alt, (size_t)c->rcap, nullptr));
-    APC_TRY(apc_ensure(c, &c->req_idx, (size_t)c->rcap, nullptr));
-    APC_TRY(apc_ensure(c, &c->req_idx_alt, (size_t)c->rcap, nullptr));
-    APC_TRY(apc_ensure(c, &c->req_code, (size_t)c->rcap, nullptr));
-    bal_collect<<<grid_for(c->rcap), kT, 0, c->s>>>(c->r_keys, (const unsigned long long *)c->r_vals,
-                                                     c->rcap, c->counters, c->req_key, c->req_idx,
-                                                     c->req_code);
-    apc_count_launch(c);
-    int nreq = 0;
-    APC_TRY(read_int(c, c->counters, &nreq));
-    if (nreq == 0) continue;
-    bool alt = false;
-    APC_TRY(apc_radix_sort_u64(c, c->req_key, c->req_idx, c->req_key_alt, c->req_idx_alt, nreq, 0, 40, &alt));
-    const uint32_t *order = alt ? c->req_idx_alt : c->req_idx;
-    APC_TRY(ensure_open_cap(c, (long long)n_open + nreq + 1));
-    bal_commit<<<grid_for(nreq), kT, 0, c->s>>>(nreq, n_open, child_base_bal + 8 * n_events, order,
-                                                c->req_code, c->keys, n, D, c->op_code, c->op_base,
-                                                c->op_first, c->op_count, c->h_keys, c->h_vals,
-                                                c->hcap, c->d_err);
-    apc_count_launch(c);
-    APC_CUDA_TRY(c, cudaGetLastError());
-    n_open += nreq;
-    n_events += nreq;
-    if (2ll * n_open > c->hcap) { *hash_full = 1; return APC_OK; }
-  }
-  c->n_open = n_open;
-  // a full hash table is read with the output's errors below: every probe is bounded, so
-  // the output pass runs safely on an incomplete table, and the selection is then redone
-  int derr = 0;
-
-  // ---- output cells ----
-  if (n_open == 0) {
+  if (!(n > 0 && temp > cc && 0 < D)) {
     // the root is the only cell (octree.cpp:1785-1788 leaf[0] = 1)
-    APC_TRY(apc_ensure(c, &c->cx, 1, nullptr));
+    int derr = 0;
+    APC_TRY(apc_read_errors(c, &derr));
+    if (derr & DERR_NOT_FINITE) {
+      c->err = "non-finite particle coordinates";
+      return APC_ERR_NOT_FINITE;
+    }
     c->nc = 1;
     c->nv = 0;
     c->nb = 0;
     return APC_ERR_UNSUPPORTED;
   }
-  const long long m8 = 8ll * n_open;
-  APC_TRY(apc_ensure(c, &c->flags, (size_t)m8 + 1, nullptr));
-  APC_TRY(apc_ensure(c, &c->req_pos, (size_t)m8 + 1, nullptr));
-  leaf_flags<<<grid_for(m8), kT, 0, c->s>>>(n_open, c->op_code, c->h_keys, c->hcap, c->flags);
+  TreeArgs A{};
+  A.keys = c->keys;
+  A.n = n;
+  A.depth = D;
+  A.sorted_levels = c->sorted_levels;
+  A.bc = c->cfg.bc;
+  A.h0 = c->h0;
+  A.c = cc;
+  A.hkeys = c->h_keys;
+  A.hvals = c->h_vals;
+  A.hcap = c->hcap;
+  for (int k = 0; k < 2; ++k) {
+    A.rkeys[k] = c->r_keys + (size_t)k * c->rcap;
+    A.rvals[k] = (unsigned long long *)c->r_vals + (size_t)k * c->rcap;
+    A.rlist[k] = c->r_list + (size_t)k * (c->rcap / 2);
+  }
+  A.rcap = c->rcap;
+  A.op_code = c->op_code;
+  A.op_base = c->op_base;
+  A.op_first = c->op_first;
+  A.op_count = c->op_count;
+  const size_t nw = (size_t)c->hcap / 8;  // words for the children of hcap / 2 nodes
+  A.words[0] = c->child_words;
+  A.words[1] = c->child_words + nw;
+  A.leaf = c->child_words + 2 * nw;
+  A.leaf_base = c->leaf_base;
+  A.crange = (int2 *)c->child_range;
+  A.out = (TreeOut *)c->tree_out;
+  A.bar = (GridBar *)(c->tree_out + sizeof(TreeOut));
+  A.nreq = (int *)(c->tree_out + sizeof(TreeOut) + sizeof(GridBar));
+  A.err = c->d_err;
+  if (c->r_dirty) {
+    APC_CUDA_TRY(c, cudaMemsetAsync(c->r_keys, 0, sizeof(uint64_t) * 2 * c->rcap, c->s));
+    APC_CUDA_TRY(c, cudaMemsetAsync(c->r_vals, 0xff, sizeof(uint64_t) * 2 * c->rcap, c->s));
+  }
+  APC_CUDA_TRY(c, cudaMemsetAsync(c->tree_out, 0, sizeof(TreeOut) + sizeof(GridBar) + kTreeLevels * sizeof(int), c->s));
+  APC_CUDA_TRY(c, cudaMemsetAsync(c->h_keys, 0, sizeof(uint64_t) * c->hcap, c->s));
+  // a block for every 2048 particles (about as many children of opened nodes as threads)
+  const int blocks = std::max(1, std::min(apc_sm_count(c), n / 2048));
+  void *args[] = {&A};
+  APC_CUDA_TRY(c, cudaLaunchCooperativeKernel((const void *)select_tree, dim3(blocks), dim3(kTreeThreads), args, 0,
+                                              c->s));
   apc_count_launch(c);
-  APC_TRY(apc_exclusive_scan(c, c->flags, c->req_pos, (int)m8, c->counters));
-  int M = 0, nc = 0;
-  // the cell count and the computational-cell count in one round trip
-  APC_CUDA_TRY(c, cudaMemcpyAsync(c->h_pinned, c->counters, sizeof(int), cudaMemcpyDeviceToHost, c->s));
-  if (8ll * n_open_td < m8)
-    APC_CUDA_TRY(c, cudaMemcpyAsync(c->h_pinned + 3, c->req_pos + 8ll * n_open_td, sizeof(int),
-                                    cudaMemcpyDeviceToHost, c->s));
+  // the sizes and the error flags in one round trip (pinned words 20 ..)
+  static_assert(sizeof(TreeOut) <= 20 * sizeof(int), "the pinned words reserved for it");
+  APC_CUDA_TRY(c, cudaMemcpyAsync(c->h_pinned + 20, c->tree_out, sizeof(TreeOut), cudaMemcpyDeviceToHost, c->s));
+  APC_CUDA_TRY(c, cudaMemcpyAsync(c->h_pinned + 1, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->s));
+  c->r_dirty = true;  // until the kernel is known to have emptied the request tables
   APC_CUDA_TRY(c, apc_stream_wait(c));
-  M = c->h_pinned[0];
-  nc = (8ll * n_open_td < m8) ? c->h_pinned[3] : M;
-  c->nc = nc;
-  c->nv = M - nc;
+  TreeOut T;
+  memcpy(&T, c->h_pinned + 20, sizeof(T));
+  int derr = c->h_pinned[1];
+  if (derr & DERR_SORT) {
+    c->err = "radix sort: a tile's look-back wait ran past its bound";
+    return APC_ERR_TIMEOUT;
+  }
+  if (derr & DERR_NOT_FINITE) {
+    c->err = "non-finite particle coordinates";
+    return APC_ERR_NOT_FINITE;
+  }
+  if (derr & DERR_KRYLOV) {
+    c->err = "selection kernel grid barrier timed out";
+    return APC_ERR_TIMEOUT;
+  }
+  if (T.stop & TREE_DEEPER) return APC_RETRY_FULL_SORT;
+  if ((T.stop & TREE_FULL) || (derr & DERR_HASH_FULL)) {
+    *hash_full = 1;
+    return APC_OK;
+  }
+  c->r_dirty = false;
+  const int n_open = T.n_open, n_open_td = T.n_open_td;
+  c->n_open_td = n_open_td;
+  c->n_open = n_open;
+  c->levels_hint = T.maxlev;
+
+  // ---- output cells: of the 8 children of each opened node all but the other opened nodes ----
+  const int M = 7 * n_open + 1;
+  c->nc = T.nc;
+  c->nv = M - T.nc;
   c->nb = 0;
   // capacities for cells
   const size_t mc = (size_t)M + 1;
@@ -523,20 +718,17 @@ static int select_once(apc_context *c, int *hash_full) {
   const int want_l = next_pow2(2ll * M + 1024);
   APC_TRY(ensure_hash(c, &c->l_keys, (void **)&c->l_vals, sizeof(int), &c->lcap, want_l));
   APC_CUDA_TRY(c, cudaMemsetAsync(c->l_keys, 0, sizeof(uint64_t) * c->lcap, c->s));
-  leaf_emit<<<grid_for(m8), kT, 0, c->s>>>(n_open, n_open_td, c->flags, c->req_pos, c->op_code, c->keys, n,
-                                            D, c->cx0, c->cy0, c->cz0, c->hx0, c->hy0, c->hz0, c->h0,
-                                            c->cx, c->cy, c->cz, c->ch, c->cfirst, c->ccount, c->ctype,
-                                            c->ccode, c->l_keys, c->l_vals, c->lcap, c->d_err);
+  leaf_emit<<<grid_for(8ll * n_open), kT, 0, c->s>>>(n_open, n_open_td, A.leaf, A.leaf_base, c->op_code, c->op_first,
+                                                     c->op_count, c->keys, D, c->cx0, c->cy0, c->cz0, c->hx0, c->hy0,
+                                                     c->hz0, c->h0, c->cx, c->cy, c->cz, c->ch, c->cfirst, c->ccount,
+                                                     c->ctype, c->ccode, c->l_keys, c->l_vals, c->lcap, c->d_err);
   neigh24_build<<<grid_for(M), kT, 0, c->s>>>(M, c->cfg.bc, c->ccode, c->h_keys, c->hcap, c->l_keys,
                                                c->l_vals, c->lcap, c->nb24, c->nnb, c->d_err);
   apc_count_launch(c, 2);
   APC_CUDA_TRY(c, cudaGetLastError());
+  APC_CUDA_TRY(c, cudaEventRecord(c->ev[1], c->s));
   APC_TRY(apc_read_errors(c, &derr));
   if (derr & DERR_HASH_FULL) { *hash_full = 1; return APC_OK; }
-  if (derr & DERR_NOT_FINITE) {
-    c->err = "non-finite particle coordinates";
-    return APC_ERR_NOT_FINITE;
-  }
   if (derr & DERR_NEIGH) {
     c->err = c->cfg.bc == 1 ? "2:1 face neighbour missing in the selected cell set"
                              : "non-periodic boundary cells are not supported";
@@ -550,8 +742,8 @@ int apc_selection(apc_context *c) {
   // on overflow (the device reports a full table instead of probing without bound)
   int want_h = next_pow2(std::max<long long>(1 << 16, (long long)c->n / 2));
   for (int attempt = 0; attempt < 8; ++attempt) {
-    APC_TRY(ensure_hash(c, &c->h_keys, (void **)&c->h_vals, sizeof(int), &c->hcap, want_h));
-    APC_TRY(ensure_hash(c, &c->r_keys, (void **)&c->r_vals, sizeof(uint64_t), &c->rcap, want_h));
+    APC_TRY(ensure_tree(c, want_h));
+    if (attempt > 0) APC_CUDA_TRY(c, cudaMemsetAsync(c->d_err, 0, sizeof(int), c->s));
     int full = 0;
     int rc = select_once(c, &full);
     if (rc != APC_OK) return rc;
@@ -573,7 +765,7 @@ int apc_selection(apc_context *c) {
       }
       return APC_OK;
     }
-    want_h *= 2;
+    want_h = 2 * c->hcap;
   }
   c->err = "selection hash tables kept overflowing";
   return APC_ERR_OUT_OF_MEMORY;
