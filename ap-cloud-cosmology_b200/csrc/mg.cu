@@ -1269,29 +1269,18 @@ __device__ __forceinline__ void cl_rows(const ClView<V> &Q, const V *x, V om, F 
   }
 }
 
+// What the phases of a block need: the layout of its shared memory and its rank.
 template <class V>
-__global__ void __launch_bounds__(kClThreads, 1) vcycle_cluster(const __grid_constant__ ClArgs<V> A) {
-  extern __shared__ __align__(16) unsigned char cl_smem[];
-  __shared__ ClOffsets off[kClLevels];
-  __shared__ int4 dim[kClLevels];  // n, w, g
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const int rank = (int)cluster_rank();
-  const V om = A.omega, al = A.alpha;
-  const int sw = A.sweeps, last = A.nl - 1;
-  // ---- the block's share of every level ----
-  {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(cl_smem);
-    const unsigned char *src = A.img + (size_t)rank * A.share;
-    for (unsigned o = 16 * t; o < A.share; o += 16 * kClThreads)
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d + o), "l"(src + o) : "memory");
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-  }
-  if (t == 0) cl_layout<V>(A, off, nullptr, nullptr);
-  if (t >= 32 && t - 32 < A.nl) dim[t - 32] = make_int4(A.L[t - 32].n, A.L[t - 32].w, A.L[t - 32].g, 0);
-  __syncthreads();
-  auto ptr = [&](unsigned o) { return reinterpret_cast<V *>(cl_smem + o); };
-  auto idx = [&](unsigned o) { return reinterpret_cast<uint16_t *>(cl_smem + o); };
-  auto view = [&](int k) {
+struct ClCtx {
+  unsigned char *smem;
+  const ClOffsets *off;
+  const int4 *dim;            // n, w, g of each level
+  int rank, last, sweeps;
+  V om, al;
+
+  __device__ __forceinline__ V *ptr(unsigned o) const { return reinterpret_cast<V *>(smem + o); }
+  __device__ __forceinline__ uint16_t *idx(unsigned o) const { return reinterpret_cast<uint16_t *>(smem + o); }
+  __device__ __forceinline__ ClView<V> view(int k) const {
     const ClOffsets o = off[k];
     const int4 q = dim[k];
     ClView<V> Q;
@@ -1309,30 +1298,42 @@ __global__ void __launch_bounds__(kClThreads, 1) vcycle_cluster(const __grid_con
     Q.xb = ptr(o.xb);
     Q.b = ptr(o.b);
     return Q;
-  };
-  {
-    // the right-hand side, and the first sweep from zero for every row
-    const ClView<V> Q = view(0);
-    if (last == 0) {
-      for (int i = t; i < Q.n; i += kClThreads) Q.b[i] = A.b[i];
-    } else {
-      const V *dinv = A.L[0].dinv;
-#pragma unroll 4
-      for (int i = t; i < Q.n; i += kClThreads) {
-        const V bi = A.b[i];
-        Q.xb[i] = om * dinv[i] * bi;
-        if ((unsigned)(i - Q.r0) < (unsigned)Q.rows) Q.b[i - Q.r0] = bi;
-      }
-    }
   }
+};
+
+// Queue the copies of the block's packed share into shared memory (cl_staged waits for them)
+// and set up the layout.
+template <class V>
+__device__ __forceinline__ void cl_stage(const ClArgs<V> &A, unsigned char *smem, ClOffsets *off, int4 *dim, int rank) {
+  const int t = threadIdx.x;
+  const unsigned d = (unsigned)__cvta_generic_to_shared(smem);
+  const unsigned char *src = A.img + (size_t)rank * A.share;
+  for (unsigned o = 16 * t; o < A.share; o += 16 * kClThreads)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d + o), "l"(src + o) : "memory");
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+  if (t == 0) cl_layout<V>(A, off, nullptr, nullptr);
+  if (t >= 32 && t - 32 < A.nl) dim[t - 32] = make_int4(A.L[t - 32].n, A.L[t - 32].w, A.L[t - 32].g, 0);
+  __syncthreads();
+}
+__device__ __forceinline__ void cl_staged() {
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
   __syncthreads();
-  cluster_barrier();  // every block runs: its shared memory may be written from here on
+}
+
+// One V-cycle by the cluster.  The caller has put the right-hand side of the block's rows in
+// the top level's b and the first sweep (omega D^-1 b) of all rows in its xb; with one level,
+// the whole right-hand side in b.  The result goes to `out` in global memory (the block's
+// rows), or, with out == nullptr, to every block's copy: the buffer returned, after a barrier.
+template <class V>
+__device__ __forceinline__ V *cl_vcycle(const ClCtx<V> &X, V *out) {
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int sw = X.sweeps, last = X.last;
+  const V om = X.om, al = X.al;
   // ---- down ----
   // a level's iterate lies in xb after one sweep (from zero: no operator) and changes sides
   // with each further one
   for (int k = 0; k < last; ++k) {
-    const ClView<V> Q = view(k);
+    const ClView<V> Q = X.view(k);
     V *x = Q.xb, *y = Q.xa;
     for (int q = 1; q < sw; ++q) {
       cl_rows<false>(Q, x, om, [&](int i, V v, int sub) { cl_broadcast(y + Q.r0 + i, v, sub, Q.g); });
@@ -1342,9 +1343,9 @@ __global__ void __launch_bounds__(kClThreads, 1) vcycle_cluster(const __grid_con
     cl_rows<true>(Q, x, om, [&](int i, V v, int sub) { cl_broadcast(y + Q.r0 + i, v, sub, Q.g); });
     cluster_barrier();
     // the coarse right-hand side, in member order, and its first sweep
-    const ClView<V> C = view(k + 1);
-    const uint16_t *mptr = idx(off[k].mptr), *mem = idx(off[k].mem);
-    const V *dinv = ptr(off[k + 1].dinv);
+    const ClView<V> C = X.view(k + 1);
+    const uint16_t *mptr = X.idx(X.off[k].mptr), *mem = X.idx(X.off[k].mem);
+    const V *dinv = X.ptr(X.off[k + 1].dinv);
     for (int I = t; I < C.n; I += kClThreads) {
       V s = V(0);
       for (int q = mptr[I], e = mptr[I + 1]; q < e; ++q) s += y[mem[q]];
@@ -1358,33 +1359,33 @@ __global__ void __launch_bounds__(kClThreads, 1) vcycle_cluster(const __grid_con
     __syncthreads();
   }
   // ---- the coarsest level: x = K^-1 b, a warp per row ----
-  const ClView<V> K = view(last);
+  const ClView<V> K = X.view(last);
   for (int i = warp; i < K.rows; i += kClThreads / 32) {
     V s = V(0);
 #pragma unroll 4
     for (int j = lane; j < K.n; j += 32) s += K.val[i * K.n + j] * K.b[j];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (last == 0) {
-      if (lane == 0) A.x[K.r0 + i] = s;
+    if (last == 0 && out) {
+      if (lane == 0) out[K.r0 + i] = s;
     } else {
       cl_broadcast(K.xa + K.r0 + i, s, lane, 32);
     }
   }
-  if (last == 0) return;  // no remote access after the first barrier
+  if (last == 0 && out) return nullptr;
   cluster_barrier();
   // ---- up ----
-  const V *xc = K.xa;
+  V *xc = K.xa;
   for (int k = last - 1; k >= 0; --k) {
-    const ClView<V> Q = view(k);
+    const ClView<V> Q = X.view(k);
     V *x = (sw & 1) ? Q.xb : Q.xa, *y = (sw & 1) ? Q.xa : Q.xb;
-    const uint16_t *agg = idx(off[k].agg);
+    const uint16_t *agg = X.idx(X.off[k].agg);
     for (int i = t; i < Q.n; i += kClThreads) x[i] += al * xc[agg[i]];
     __syncthreads();
     for (int q = 0; q < sw; ++q) {
-      if (k == 0 && q + 1 == sw) {
+      if (out && k == 0 && q + 1 == sw) {
         cl_rows<false>(Q, x, om, [&](int i, V v, int sub) {
-          if (sub == 0) A.x[Q.r0 + i] = v;
+          if (sub == 0) out[Q.r0 + i] = v;
         });
       } else {
         cl_rows<false>(Q, x, om, [&](int i, V v, int sub) { cl_broadcast(y + Q.r0 + i, v, sub, Q.g); });
@@ -1394,7 +1395,350 @@ __global__ void __launch_bounds__(kClThreads, 1) vcycle_cluster(const __grid_con
     }
     xc = x;
   }
+  return xc;
 }
+
+template <class V>
+__global__ void __launch_bounds__(kClThreads, 1) vcycle_cluster(const __grid_constant__ ClArgs<V> A) {
+  extern __shared__ __align__(16) unsigned char cl_smem[];
+  __shared__ ClOffsets off[kClLevels];
+  __shared__ int4 dim[kClLevels];
+  const int t = threadIdx.x;
+  const ClCtx<V> X{cl_smem, off, dim, (int)cluster_rank(), A.nl - 1, A.sweeps, A.omega, A.alpha};
+  cl_stage(A, cl_smem, off, dim, X.rank);
+  {
+    // the right-hand side, and the first sweep from zero for every row
+    const ClView<V> Q = X.view(0);
+    if (X.last == 0) {
+      for (int i = t; i < Q.n; i += kClThreads) Q.b[i] = A.b[i];
+    } else {
+      const V *dinv = A.L[0].dinv;
+#pragma unroll 4
+      for (int i = t; i < Q.n; i += kClThreads) {
+        const V bi = A.b[i];
+        Q.xb[i] = X.om * dinv[i] * bi;
+        if ((unsigned)(i - Q.r0) < (unsigned)Q.rows) Q.b[i - Q.r0] = bi;
+      }
+    }
+  }
+  cl_staged();
+  cluster_barrier();  // every block runs: its shared memory may be written from here on
+  cl_vcycle<V>(X, A.x);
+}
+
+// ---- a whole solve on one cluster ----
+// Systems of up to 16 x 512 rows whose hierarchy fits one cluster's shared memory: the FP64
+// refinement loop, the (F)GMRES cycles and the V-cycles in one launch, with the same steps,
+// precisions and stopping tests as the graph of kernels, which such systems leave waiting for
+// launches (an iteration of 3,200 rows took 50 us in 5 dependent kernels and a loop node, and
+// each solve was captured and its executable updated by the host).  One thread per row of the block
+// holds the row's residual and basis entries; a vector that the next product gathers is stored
+// to every block's copy; sums go to every block, which adds them in block order, so all blocks
+// take the same branches.  Per iteration: the V-cycle's barriers and two more.  3,179 rows: 30 us
+// per potential iteration (50 as a graph); the 4k box's two solves 1.05 ms as graphs, 0.65 ms here.
+struct ClSolveShared {
+  double red[2][kClBlocks][kMaxM + 1];     // each block's sums, two reductions in turn
+  double wsum[kClThreads / 32][kMaxM + 1];
+  double h[kMaxM + 2];
+  double H[(kMaxM + 1) * kMaxM];           // column j at H[j * (M + 1)]
+  double cs[kMaxM], sn[kMaxM], g[kMaxM + 1], y[kMaxM];
+  double row[kClThreads];                  // products of the block's rows
+  double scale, beta;
+  int more;
+};
+
+// dynamic shared memory beside it, the levels' offsets and sizes
+constexpr unsigned kClSolveDyn = (unsigned)(kSmemMax - sizeof(ClSolveShared) - kClStatic) & ~15u;
+
+struct ClResult {
+  int outer, total_its, reason, pad;
+  double rn;
+};
+
+template <class T, class TV>
+struct ClSolveArgs {
+  int n, w;
+  size_t ld;
+  const int *col;
+  const T *valf;              // D^-1 A in the inner precision
+  const double *val, *b;      // FP64 operator (diagonal in slot 0) and right-hand side
+  double *x;                  // the initial guess, the solution
+  T *V, *Z;                   // basis, preconditioned vectors (own rows of each block)
+  size_t vn;
+  int M, max_it, max_outer, exact_inner, g;  // g: lanes per row of a product
+  double rtol, atol, dtol, rtol_in;
+  unsigned o_col, o_vec, total;  // without a V-cycle: columns and gathered vector after the values
+  ClResult *out;
+  ClArgs<TV> cl;              // with one
+};
+
+template <class T, class TV, bool MG, int NV>
+__global__ void __launch_bounds__(kClThreads, 1) solve_cluster(const __grid_constant__ ClSolveArgs<T, TV> A) {
+  extern __shared__ __align__(16) unsigned char cl_smem[];
+  __shared__ ClOffsets off[kClLevels];
+  __shared__ int4 dim[kClLevels];
+  __shared__ ClSolveShared S;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int rank = (int)cluster_rank(), n = A.n, M1 = A.M + 1;
+  const int R = cl_rows_per_block(n), r0 = rank * R, rows = max(0, min(R, n - r0)), ld = R | 1;
+  const bool own = t < rows;
+  const int row = r0 + t;
+  const ClCtx<TV> X{cl_smem, off, dim, rank, A.cl.nl - 1, A.cl.sweeps, A.cl.omega, A.cl.alpha};
+  // ---- stage the operator ----
+  const uint16_t *col;        // the block's rows of the columns, and of the values where
+  const T *vals = nullptr;    // they lie in shared memory in the inner precision
+  T *vec = nullptr;           // without a V-cycle: the gathered vector, all rows
+  if constexpr (MG) {
+    cl_stage(A.cl, cl_smem, off, dim, rank);
+    cl_staged();
+    if (X.last > 0) {
+      col = X.idx(off[0].col);
+      if constexpr (std::is_same_v<T, TV>) vals = X.ptr(off[0].val);  // level 0 is D^-1 A itself
+    }
+  } else {
+    T *v = reinterpret_cast<T *>(cl_smem);
+    uint16_t *cc = reinterpret_cast<uint16_t *>(cl_smem + A.o_col);
+    vec = reinterpret_cast<T *>(cl_smem + A.o_vec);
+    for (int s = warp; s < A.w; s += kClThreads / 32)
+#pragma unroll 4
+      for (int i = lane; i < rows; i += 32) {
+        const size_t at = (size_t)s * A.ld + r0 + i;
+        v[s * ld + i] = A.valf[at];
+        cc[s * ld + i] = (uint16_t)A.col[at];
+      }
+    vals = v;
+    col = cc;
+    __syncthreads();
+  }
+  const bool one_level = MG && X.last == 0;  // its columns are not staged: read from memory
+  double dii = 1.0, bi = 0.0, xi = 0.0;
+  TV od = TV(0);              // omega D^-1 of the row in the V-cycle's operator
+  if (own) {
+    const double d = A.val[row];
+    dii = d == 0.0 ? 1.0 : d;
+    bi = A.b[row];
+    xi = A.x[row];
+    if constexpr (MG)
+      if (!one_level) od = X.om * X.ptr(off[0].dinv)[t];
+  }
+  cluster_barrier();
+  int nred = 0;
+
+  // sums over all rows of the nv values f(j) of each thread, into S.h; a block barrier and a
+  // cluster barrier
+  auto reduce = [&](int nv, auto f) {
+    double (*red)[kMaxM + 1] = S.red[nred & 1];
+    ++nred;
+    if (nv == 1) {
+      const double v = warp_sum(f(0));
+      if (lane == 0) S.wsum[warp][0] = v;
+    } else {
+#pragma unroll
+      for (int j = 0; j < NV; ++j)
+        if (j < nv) {
+          const double v = warp_sum(f(j));
+          if (lane == 0) S.wsum[warp][j] = v;
+        }
+    }
+    __syncthreads();
+    if (t < nv * kClBlocks) {
+      // one store per (value, block): the lanes of a value form its sum alike
+      const int j = t / kClBlocks, d = t % kClBlocks;
+      double v = 0.0;
+#pragma unroll
+      for (int q = 0; q < kClThreads / 32; ++q) v += S.wsum[q][j];
+      remote_store(cluster_addr(&red[rank][j], d), v);
+    }
+    cluster_barrier();
+    if (t < nv) {
+      double v = 0.0;
+#pragma unroll
+      for (int q = 0; q < kClBlocks; ++q) v += red[q][t];
+      S.h[t] = v;
+    }
+    __syncthreads();
+  };
+  // the product of the block's rows with x, into S.row; ends with a block barrier
+  auto product = [&](auto x) {
+    const int g = A.g, sub = t & (g - 1), per = kClThreads / g;
+    for (int i0 = 0; i0 < rows; i0 += per) {
+      const int i = i0 + t / g;
+      T s = T(0);
+      if (i < rows) {
+#pragma unroll 4
+        for (int k = sub; k < A.w; k += g) {
+          const size_t at = (size_t)k * A.ld + r0 + i;
+          const T a = vals ? vals[k * ld + i] : A.valf[at];
+          s += a * x(one_level ? A.col[at] : (int)col[k * ld + i]);
+        }
+      }
+      for (int o = g >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (i < rows && sub == 0) S.row[i] = (double)s;
+    }
+    __syncthreads();
+  };
+  // v of the row, not yet normalised, to every block (for the next V-cycle or product)
+  auto publish = [&](T v) {
+    if (!own) return;
+    if constexpr (MG) {
+      const ClView<TV> Q = X.view(0);
+      if (one_level) cl_broadcast(Q.b + row, (TV)v, 0, 1);
+      else cl_broadcast(Q.xb + row, od * (TV)v, 0, 1);
+    } else {
+      cl_broadcast(vec + row, v, 0, 1);
+    }
+  };
+
+  // ---- ||D^-1 b||: the stopping test's scale ----
+  {
+    const double pb = own ? bi / dii : 0.0;
+    reduce(1, [&](int) { return pb * pb; });
+  }
+  const double bnorm = sqrt(S.h[0]);
+  const double ttol = fmax(A.rtol * bnorm, A.atol);
+  int outer = 0, total = 0, reason = 0;
+  double rn = 0.0, rtol_in = A.rtol_in;
+  for (;;) {
+    // ---- r = b - A x in FP64, ||D^-1 r||, the stopping test (as ir_residual) ----
+    double pr = 0.0;
+    if (own) {
+      double s = 0.0;
+#pragma unroll 6
+      for (int k = 0; k < A.w; ++k) {
+        const size_t at = (size_t)k * A.ld + row;
+        s += A.val[at] * __ldcg(A.x + A.col[at]);
+      }
+      pr = (bi - s) / dii;
+    }
+    reduce(1, [&](int) { return pr * pr; });
+    const double rnew = sqrt(S.h[0]);
+    bool stop = true;
+    if (outer == 0 && bnorm == 0.0) reason = kConvergedAtol;
+    else if (!(rnew == rnew)) reason = kDivergedNanOrInf;
+    else if (rnew <= ttol) reason = rnew < A.atol ? kConvergedAtol : kConvergedRtol;
+    else if (rnew >= A.dtol * bnorm) reason = kDivergedDtol;
+    else if (total >= A.max_it) reason = kDivergedIts;
+    else if (outer >= A.max_outer) reason = 0;
+    else stop = false;
+    if (A.exact_inner) {
+      if (rnew > 0.0) rtol_in = fmin(0.1, fmax(0.5 * ttol / rnew, 1e-15));
+    } else if (outer >= 1 && rn > 0.0) {
+      rtol_in = fmin(0.1, fmax(A.rtol_in, 0.5 * (rnew / rn)));
+    }
+    rn = rnew;
+    if (stop) break;
+    // ---- v_0 = D^-1 r / ||D^-1 r|| in the inner precision ----
+    T w = (T)(pr * (1.0 / rn));
+    publish(w);
+    reduce(1, [&](int) { return own ? (double)w * (double)w : 0.0; });
+    const double beta = sqrt(S.h[0]);
+    int it = 0;
+    const int inner_max = min(A.M, max(1, A.max_it - total));
+    double scale = beta > 0.0 ? 1.0 / beta : 0.0;
+    if (t == 0) S.g[0] = beta;
+    T vj[NV];                 // the row's entries of the basis
+    bool more = beta > 0.0;
+    while (more) {
+      {
+        const T u = w * (T)scale;
+#pragma unroll
+        for (int j = 0; j < NV; ++j)
+          if (j == it) vj[j] = u;
+      }
+      // ---- z = V-cycle(v_it) (or v_it itself), w = A z ----
+      if constexpr (MG) {
+        const ClView<TV> Q = X.view(0);
+        const TV sc = (TV)scale;
+        if (one_level) {
+          for (int i = t; i < n; i += kClThreads) Q.b[i] *= sc;
+        } else {
+          for (int i = t; i < n; i += kClThreads) Q.xb[i] *= sc;
+          if (own) Q.b[t] = (TV)(w * (T)scale);
+        }
+        __syncthreads();
+        const TV *z = cl_vcycle<TV>(X, nullptr);
+        if (own) A.Z[(size_t)it * A.vn + row] = (T)z[row];
+        product([&](int j) { return (T)z[j]; });
+        w = own ? (T)S.row[t] : T(0);
+      } else {
+        if (own) A.V[(size_t)it * A.vn + row] = w * (T)scale;
+        product([&](int j) { return vec[j]; });
+        w = own ? (T)(S.row[t] * scale) : T(0);
+      }
+      // ---- classical Gram-Schmidt ----
+      reduce(it + 1, [&](int j) { return own ? (double)w * (double)vj[j] : 0.0; });
+      double wi = (double)w;
+#pragma unroll
+      for (int j = 0; j < NV; ++j)
+        if (j <= it) wi -= S.h[j] * (double)vj[j];
+      w = own ? (T)wi : T(0);
+      publish(w);
+      // the column's earlier rotations run while the norm is summed: copy it first
+      double hc = 0.0;
+      if (t <= it) hc = S.h[t];
+      __syncthreads();
+      if (t <= it) S.H[(size_t)it * M1 + t] = hc;
+      reduce(1, [&](int) { return (double)w * (double)w; });
+      // ---- Arnoldi scalars (as arnoldi_step), by every block alike ----
+      if (t == 0) {
+        double *hs = S.H + (size_t)it * M1;
+        const double tt = sqrt(S.h[0]);
+        hs[it + 1] = tt;
+        for (int j = 1; j <= it; ++j) {
+          const double t0 = hs[j - 1];
+          hs[j - 1] = S.cs[j - 1] * t0 + S.sn[j - 1] * hs[j];
+          hs[j] = S.cs[j - 1] * hs[j] - S.sn[j - 1] * t0;
+        }
+        const double q = sqrt(hs[it] * hs[it] + hs[it + 1] * hs[it + 1]);
+        bool go = false;
+        if (q != 0.0 && q == q) {
+          const double cs = hs[it] / q, sn = hs[it + 1] / q;
+          S.cs[it] = cs;
+          S.sn[it] = sn;
+          const double gi = S.g[it];
+          S.g[it + 1] = -sn * gi;
+          S.g[it] = cs * gi;
+          hs[it] = cs * hs[it] + sn * hs[it + 1];
+          go = !(fabs(S.g[it + 1]) <= rtol_in * beta) && tt != 0.0;
+        }
+        S.more = go && it + 1 < inner_max;
+        S.scale = tt > 0.0 ? 1.0 / tt : 0.0;
+      }
+      __syncthreads();
+      ++it;
+      more = S.more != 0;
+      scale = S.scale;
+    }
+    // ---- y = H^-1 g, x += ||D^-1 r|| Z y ----
+    if (t == 0) {
+      for (int k = it - 1; k >= 0; --k) {
+        double s = S.g[k];
+        for (int j = k + 1; j < it; ++j) s -= S.H[(size_t)j * M1 + k] * S.y[j];
+        const double hkk = S.H[(size_t)k * M1 + k];
+        S.y[k] = hkk != 0.0 ? s / hkk : 0.0;
+      }
+    }
+    __syncthreads();
+    total += it;
+    if (own) {
+      const T *Z = (MG ? A.Z : A.V) + row;
+      double d = 0.0;
+#pragma unroll 4
+      for (int j = 0; j < it; ++j) d += S.y[j] * (double)Z[(size_t)j * A.vn];
+      xi += rn * (double)(T)d;
+      A.x[row] = xi;
+    }
+    ++outer;
+    cluster_barrier();  // x is complete
+  }
+  if (rank == 0 && t == 0) {
+    A.out->outer = outer;
+    A.out->total_its = total;
+    A.out->reason = reason;
+    A.out->rn = rn;
+  }
+}
+
 // ---------------------------------------------- the whole solve as one persistent kernel
 //
 // One cooperative launch runs a complete solve: the FP64 refinement loop, each
@@ -1427,10 +1771,7 @@ struct PLevel {
   T *x, *x2, *b, *r;
 };
 
-struct PResult {
-  int outer, total_its, reason, pad;
-  double rn;
-};
+using PResult = ClResult;
 
 template <class T>
 struct PSolveArgs {
@@ -2015,7 +2356,7 @@ struct MgWork {
   double *ppart = nullptr;
   GridBar *pbar = nullptr;
   PResult *pres = nullptr;
-  PResult *pres_host = nullptr;
+  PResult *pres_host = nullptr;  // in the context's pinned words
   // the device-side coarse inverse's outcome (0 or 1 = singular) and its pinned copy,
   // checked after the next solve's readback
   int *cstat = nullptr;
@@ -2094,7 +2435,6 @@ void apc_mg_free(apc_context *c) {
                m->cstat, m->wdev};
   for (void *q : p) apc_free(c, q);
   if (m->host) cudaFreeHost(m->host);
-  if (m->pres_host) cudaFreeHost(m->pres_host);
   if (m->cstat_host) cudaFreeHost(m->cstat_host);
   if (m->whost) cudaFreeHost(m->whost);
   for (int k = 0; k < 2; ++k) {
@@ -2426,6 +2766,28 @@ static int check_coarse(apc_context *c) {
   return APC_OK;
 }
 
+static int ensure_result(apc_context *c) {
+  MgWork *m = c->mg;
+  static_assert(sizeof(PResult) <= 8 * sizeof(int), "pinned words 40 .. 47");
+  if (!m->pres) APC_TRY(apc_alloc(c, (void **)&m->pres, sizeof(PResult)));
+  m->pres_host = reinterpret_cast<PResult *>(c->h_pinned + 40);
+  return APC_OK;
+}
+
+// one cluster of kClBlocks blocks
+static void cluster_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *at, size_t smem, cudaStream_t s) {
+  cfg.gridDim = dim3(kClBlocks);
+  cfg.blockDim = dim3(kClThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = kClBlocks;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+}
+
 // x = V-cycle(b) on level l, launched on stream s; b and x are that level's buffers
 template <class T>
 static void vcycle(apc_context *c, cudaStream_t s, int l, const T *b, T *x) {
@@ -2447,17 +2809,8 @@ static void vcycle(apc_context *c, cudaStream_t s, int l, const T *b, T *x) {
     A.b = b;
     A.x = x;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(kClBlocks);
-    cfg.blockDim = dim3(kClThreads);
-    cfg.dynamicSmemBytes = A.total;
-    cfg.stream = s;
     cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = kClBlocks;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cluster_config(cfg, at, A.total, s);
     cudaLaunchKernelEx(&cfg, vcycle_cluster<T>, A);  // an error is read after the capture
     apc_count_launch(c);
     return;
@@ -2773,9 +3126,8 @@ static int fill_psolve(apc_context *c, const IrSolveArgs<T> &a, PSolveArgs<T> &P
   if (!m->ppart) {
     APC_TRY(apc_alloc(c, (void **)&m->ppart, sizeof(double) * (size_t)kPSlots * kPMaxBlocks));
     APC_TRY(apc_alloc(c, (void **)&m->pbar, sizeof(GridBar)));
-    APC_TRY(apc_alloc(c, (void **)&m->pres, sizeof(PResult)));
   }
-  if (!m->pres_host) APC_CUDA_TRY(c, cudaMallocHost((void **)&m->pres_host, sizeof(PResult)));
+  APC_TRY(ensure_result(c));
   P = PSolveArgs<T>{};
   P.n = a.n;
   P.w = a.w;
@@ -2912,6 +3264,70 @@ static double solve_bytes(const MgHier<TV> &H, bool use_mg, int n, int w, int sw
   return outer * per_outer + total_its * per_it;
 }
 
+// A whole solve on one cluster (solve_cluster) where it fits: a row per thread and, for the
+// potential, the whole hierarchy in the cluster's shared memory; for the density, its operator
+// and one gathered vector.  *done says whether it was launched.
+template <class T, class TV>
+static int cluster_solve(apc_context *c, const IrSolveArgs<T> &a, bool *done) {
+  MgWork *m = c->mg;
+  MgHier<T> &H = hier<T>(m);
+  MgHier<TV> &HV = hier<TV>(m);
+  *done = false;
+  const int R = cl_rows_per_block(a.n);
+  if (R > kClThreads) return APC_OK;
+  ClSolveArgs<T, TV> A{};
+  A.n = a.n;
+  A.w = a.w;
+  A.ld = a.ld;
+  A.col = a.col;
+  A.valf = a.valf;
+  A.val = a.val;
+  A.b = a.b;
+  A.x = a.x;
+  A.V = H.V;
+  A.Z = H.Z;
+  A.vn = m->vn;
+  A.M = a.M;
+  A.max_it = a.max_it;
+  A.max_outer = a.max_outer;
+  A.exact_inner = sizeof(T) == sizeof(double) ? 1 : 0;
+  A.g = tail_lanes(R, a.w, kClThreads);
+  A.rtol = a.rtol;
+  A.atol = a.atol;
+  A.dtol = a.dtol;
+  A.rtol_in = a.rtol_in;
+  if (a.mg) {
+    if (HV.cl_first != 0) return APC_OK;
+    A.cl = HV.cl;
+    A.cl.sweeps = c->cfg.mg_sweeps > 0 ? c->cfg.mg_sweeps : 2;
+    A.cl.omega = (TV)(c->cfg.mg_omega > 0 ? c->cfg.mg_omega : 0.95);
+    A.cl.alpha = (TV)(c->cfg.mg_alpha > 0 ? c->cfg.mg_alpha : 1.8);
+    A.total = A.cl.total;
+  } else {
+    A.o_col = tail_align((size_t)a.w * (R | 1) * sizeof(T));
+    A.o_vec = A.o_col + tail_align((size_t)a.w * (R | 1) * sizeof(uint16_t));
+    A.total = A.o_vec + tail_align((size_t)a.n * sizeof(T));
+  }
+  if (A.total > kClSolveDyn) return APC_OK;
+  APC_TRY(ensure_result(c));
+  A.out = m->pres;
+  void (*kern)(ClSolveArgs<T, TV>);
+  if (a.mg)
+    kern = a.M <= 16 ? solve_cluster<T, TV, true, 16> : solve_cluster<T, TV, true, 32>;
+  else
+    kern = a.M <= 16 ? solve_cluster<T, TV, false, 16> : solve_cluster<T, TV, false, 32>;
+  APC_CUDA_TRY(c, cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)kClSolveDyn));
+  APC_CUDA_TRY(c, cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at[1];
+  cluster_config(cfg, at, A.total, c->s);
+  APC_CUDA_TRY(c, cudaLaunchKernelEx(&cfg, kern, A));
+  apc_count_launch(c);
+  *done = true;
+  return APC_OK;
+}
+
 template <class T>
 static int ir_solve(apc_context *c, int which, bool use_mg, const double *val, const T *valf, const double *b,
                     double *x, double *r, int restart, double rtol_in, int *its, double *rnorm, int *reason,
@@ -2934,18 +3350,7 @@ static int ir_solve(apc_context *c, int which, bool use_mg, const double *val, c
       APC_TRY(apc_ensure(c, &H.vout, vn));
     }
   }
-  APC_TRY(apc_ensure(c, &H.dvec, vn));
-  APC_TRY(apc_ensure(c, &m->partial, (size_t)kRedBlocks * 34));
-  APC_TRY(apc_ensure(c, &m->dots, (size_t)4 * 34));
   m->vn = vn;
-  if (!m->counter) {
-    APC_TRY(apc_alloc(c, (void **)&m->counter, 4 * sizeof(unsigned)));
-    APC_CUDA_TRY(c, cudaMemsetAsync(m->counter, 0, 4 * sizeof(unsigned), c->s));
-  }
-  if (!m->state) APC_TRY(apc_alloc(c, (void **)&m->state, sizeof(IrState)));
-  if (!m->host) APC_CUDA_TRY(c, cudaMallocHost((void **)&m->host, sizeof(IrState)));
-  for (int k = 0; k < 2; ++k)
-    if (!m->cap[k]) APC_CUDA_TRY(c, cudaStreamCreateWithFlags(&m->cap[k], cudaStreamNonBlocking));
   const apc_config &cfg = c->cfg;
   const auto t0 = std::chrono::steady_clock::now();
   const bool prebuilt = use_mg && m->prebuilt;  // built during the density solve
@@ -2987,6 +3392,22 @@ static int ir_solve(apc_context *c, int which, bool use_mg, const double *val, c
   // re-orthogonalising Gram-Schmidt and the FP32 V-cycle under FP64 vectors run only there)
   const bool can_persist = !cfg.mg_reorth && !mg32;
   bool persistent = can_persist && !cfg.mixed_solve_graphs;
+  // the outcome of a solve that ran as one kernel, read back
+  auto outcome = [&](const PResult &R) -> int {
+    float ms = 0.f;
+    APC_CUDA_TRY(c, cudaEventElapsedTime(&ms, c->kev[0], c->kev[1]));
+    *its = R.total_its;
+    *rnorm = R.rn;
+    *reason = R.reason;
+    *refinements = R.outer;
+    *levels = use_mg ? nlev : 0;
+    if (use_mg) {
+      c->prof.mg_solve_ms += ms;
+      c->prof.mg_iterations += R.total_its;
+      c->prof.mg_bytes += bytes(R.total_its, R.outer);
+    }
+    return APC_OK;
+  };
   if (can_persist && c->defer_solve) {
     // prepared for a batched launch with other boxes' solves (apc_mg_batched_solve);
     // apc_ir_finish reads the outcome
@@ -3028,22 +3449,36 @@ static int ir_solve(apc_context *c, int which, bool use_mg, const double *val, c
         return APC_ERR_TIMEOUT;
       }
       if (use_mg) APC_TRY(check_coarse(c));
-      const PResult &R = *m->pres_host;
-      float ms = 0.f;
-      APC_CUDA_TRY(c, cudaEventElapsedTime(&ms, c->kev[0], c->kev[1]));
-      *its = R.total_its;
-      *rnorm = R.rn;
-      *reason = R.reason;
-      *refinements = R.outer;
-      *levels = use_mg ? nlev : 0;
-      if (use_mg) {
-        c->prof.mg_solve_ms += ms;
-        c->prof.mg_iterations += R.total_its;
-        c->prof.mg_bytes += bytes(R.total_its, R.outer);
-      }
-      return APC_OK;
+      return outcome(*m->pres_host);
     }
   }
+  bool on_cluster = false;
+  if (!cfg.mg_reorth && cfg.mixed_solve_graphs) {
+    APC_CUDA_TRY(c, cudaEventRecord(c->kev[0], c->s));
+    APC_TRY((mg32 ? cluster_solve<T, float>(c, a, &on_cluster) : cluster_solve<T, T>(c, a, &on_cluster)));
+  }
+  if (on_cluster) {
+    if (use_mg)
+      c->prof.mg_build_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+    APC_CUDA_TRY(c, cudaEventRecord(c->kev[1], c->s));
+    APC_CUDA_TRY(c, cudaMemcpyAsync(m->pres_host, m->pres, sizeof(PResult), cudaMemcpyDeviceToHost, c->s));
+    if (during) APC_TRY(during(c));
+    APC_CUDA_TRY(c, apc_stream_wait(c));
+    APC_CUDA_TRY(c, cudaGetLastError());
+    if (use_mg) APC_TRY(check_coarse(c));
+    return outcome(*m->pres_host);
+  }
+  APC_TRY(apc_ensure(c, &H.dvec, vn));
+  APC_TRY(apc_ensure(c, &m->partial, (size_t)kRedBlocks * 34));
+  APC_TRY(apc_ensure(c, &m->dots, (size_t)4 * 34));
+  if (!m->counter) {
+    APC_TRY(apc_alloc(c, (void **)&m->counter, 4 * sizeof(unsigned)));
+    APC_CUDA_TRY(c, cudaMemsetAsync(m->counter, 0, 4 * sizeof(unsigned), c->s));
+  }
+  if (!m->state) APC_TRY(apc_alloc(c, (void **)&m->state, sizeof(IrState)));
+  if (!m->host) APC_CUDA_TRY(c, cudaMallocHost((void **)&m->host, sizeof(IrState)));
+  for (int k = 0; k < 2; ++k)
+    if (!m->cap[k]) APC_CUDA_TRY(c, cudaStreamCreateWithFlags(&m->cap[k], cudaStreamNonBlocking));
   APC_TRY(capture_solve(c, a));
   if (use_mg)
     c->prof.mg_build_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();

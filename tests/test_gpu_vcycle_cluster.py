@@ -84,3 +84,33 @@ def test_potential_residual(box, precision, sweeps):
     if bn > 1e-12 * C_POT / np.abs(d).max():  # equal densities: the right-hand side is rounding alone
         assert np.linalg.norm((b - ax) / d) <= 1.05e-10 * bn
         assert precision == "mixed" or abs(st["potential_its"] - its) <= 2
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64mg", "vcycle32"])
+@pytest.mark.parametrize("kw", [dict(mixed_restart=24), dict(mixed_restart=3), dict(precond=0), dict(warm_start=1),
+                                dict(max_it=5)], ids=lambda k: "-".join(k))
+def test_one_cluster_solve_options(gpu_lib, precision, kw):
+    """The whole solve on one cluster (ball1500: 700 rows) under the options that change its
+    loops: a long and a short restart, no V-cycle, a guess from the step before, max_it.  It
+    meets the stopping test or, cut at max_it, reports so; the potential agrees with the
+    persistent solve's to what two solves at rtol 1e-10 differ by (1e-7, as between the graph
+    and persistent forms elsewhere)."""
+    parts, c = _box(*BOXES["ball1500"])
+    prec = {"mixed": binding.APC_PREC_MIXED, "fp64mg": binding.APC_PREC_FP64_MULTIGRID,
+            "vcycle32": binding.APC_PREC_MIXED_VCYCLE}[precision]
+    out = []
+    for graphs in (1, 0):
+        g = binding.GpuPath(parts, 21, c, precision=prec, solve_graphs=graphs, **kw)
+        for _ in range(2 if "warm_start" in kw else 1):
+            g.select()
+            g.solve(1.0 / parts.n, C_POT, -1.0)
+        out.append((g.solve_stats(), g.fields()))
+        g.close()
+    (s1, f1), (s0, f0) = out
+    for k in ("density", "potential"):
+        a, b = getattr(f1, k), getattr(f0, k)
+        if "max_it" not in kw:
+            assert s1[k + "_reason"] in (2, 3) and s0[k + "_reason"] in (2, 3)
+            assert np.max(np.abs(a - b)) <= 1e-7 * np.max(np.abs(b)), k
+        else:
+            assert s1[k + "_reason"] == -3 and s1[k + "_its"] == 5
