@@ -326,6 +326,10 @@ __device__ __forceinline__ unsigned cluster_rank() {
 __device__ __forceinline__ void remote_store(unsigned addr, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
 }
+__device__ __forceinline__ void remote_store(unsigned addr, float4 v) {
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+               : "memory");
+}
 __device__ __forceinline__ void remote_store(unsigned addr, double v) {
   asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
 }
@@ -335,6 +339,27 @@ __device__ __forceinline__ unsigned cluster_addr(const void *p, unsigned rank) {
   const unsigned a = (unsigned)__cvta_generic_to_shared(p);
   asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(rank));
   return ra;
+}
+
+// xor-tree sums over the warp of eight values: on return the sum of value j is in the lanes
+// with (lane >> 2) == j, formed by the offsets 16, 8, 4, 2, 1 in turn
+__device__ __forceinline__ double warp_sum8(double (&v)[8], int lane) {
+  const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const double keep = b4 ? v[4 + i] : v[i], send = b4 ? v[i] : v[4 + i];
+    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const double keep = b3 ? v[2 + i] : v[i], send = b3 ? v[i] : v[2 + i];
+    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+  }
+  const double keep = b2 ? v[1] : v[0], send = b2 ? v[0] : v[1];
+  double s = keep + __shfl_xor_sync(0xffffffffu, send, 4);
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  s += __shfl_xor_sync(0xffffffffu, s, 1);
+  return s;
 }
 #endif
 

@@ -445,27 +445,6 @@ struct CgArgs {
   unsigned o_u, o_col, o_red, o_nrm, o_hh, o_small;  // byte offsets in shared memory (values at 0)
 };
 
-// xor-tree sums over the warp of eight values: on return the sum of value j is in the lanes
-// with (lane >> 2) == j, formed by the offsets 16, 8, 4, 2, 1 in turn
-__device__ __forceinline__ double warp_sum8(double (&v)[8], int lane) {
-  const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const double keep = b4 ? v[4 + i] : v[i], send = b4 ? v[i] : v[4 + i];
-    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-  }
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const double keep = b3 ? v[2 + i] : v[i], send = b3 ? v[i] : v[2 + i];
-    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
-  }
-  const double keep = b2 ? v[1] : v[0], send = b2 ? v[0] : v[1];
-  double s = keep + __shfl_xor_sync(0xffffffffu, send, 4);
-  s += __shfl_xor_sync(0xffffffffu, s, 2);
-  s += __shfl_xor_sync(0xffffffffu, s, 1);
-  return s;
-}
-
 __device__ __forceinline__ double xor_sum(double t) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);

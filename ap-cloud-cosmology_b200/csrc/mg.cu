@@ -1088,6 +1088,7 @@ constexpr int kClLevels = 16;
 template <class V>
 struct ClLevel {
   int n, w, g;                // rows, slots, lanes per row (power of two)
+  int rep;                    // every block holds and computes all rows
   size_t ld;
   const int *col;
   const V *val, *dinv;
@@ -1109,8 +1110,15 @@ __host__ __device__ inline unsigned tail_align(size_t b) { return (unsigned)((b 
 
 // a block's rows of a level of n rows, and the odd leading dimension of its staged slots (so
 // that lanes on neighbouring slots of a row fall in different banks)
-__host__ __device__ inline int cl_rows_per_block(int n) { return (n + kClBlocks - 1) / kClBlocks; }
-__host__ __device__ inline int cl_ld(int n) { return cl_rows_per_block(n) | 1; }
+__host__ __device__ inline int cl_rows_per_block(int n, int rep = 0) {
+  return rep ? n : ((n + kClBlocks - 1) / kClBlocks + 3) & ~3;  // whole 16-byte words of a vector
+}
+__host__ __device__ inline int cl_ld(int n, int rep) { return cl_rows_per_block(n, rep) | 1; }
+
+// Levels below the top one of at most this many entries are kept whole by every block, which
+// computes them redundantly between block barriers: 16 entries a thread take less than the
+// cluster barrier and the remote stores they save (per level 2-3 us).
+constexpr int kClRepEntries = 16 * kClThreads;
 
 // Byte offsets of level k in a block's shared memory; the same in every block.  The packed
 // share comes first (val .. mem of every level), the vectors after it.
@@ -1133,8 +1141,8 @@ __host__ __device__ inline void cl_layout(const ClArgs<V> &A, ClOffsets *off, un
   };
   for (int part = 0; part < 2; ++part) {
     for (int k = 0; k < A.nl; ++k) {
-      const size_t n = (size_t)A.L[k].n, rows = (size_t)cl_rows_per_block(A.L[k].n);
-      const size_t sl = (size_t)cl_ld(A.L[k].n) * A.L[k].w;
+      const size_t n = (size_t)A.L[k].n, rows = (size_t)cl_rows_per_block(A.L[k].n, A.L[k].rep);
+      const size_t sl = (size_t)cl_ld(A.L[k].n, A.L[k].rep) * A.L[k].w;
       const bool last = k + 1 == A.nl;
       if (part == 0) {
         const unsigned val = take((last ? rows * n : sl) * sizeof(V));
@@ -1152,9 +1160,11 @@ __host__ __device__ inline void cl_layout(const ClArgs<V> &A, ClOffsets *off, un
           off[k].mem = mem;
         }
       } else {
-        const unsigned xa = take(n * sizeof(V));
-        const unsigned xb = take(last ? 0 : n * sizeof(V));
-        const unsigned b = take((last ? n : rows) * sizeof(V));
+        // a vector of all rows, the blocks' shares whole
+        const size_t all = A.L[k].rep ? n : rows * kClBlocks;
+        const unsigned xa = take(all * sizeof(V));
+        const unsigned xb = take(last ? 0 : all * sizeof(V));
+        const unsigned b = take((last ? all : rows) * sizeof(V));
         if (off) {
           off[k].xa = xa;
           off[k].xb = xb;
@@ -1177,17 +1187,26 @@ static bool cl_fits(ClArgs<V> &A) {
   size_t big = 0;
   for (int k = 0; k < A.nl; ++k) {
     if (A.L[k].n > 65535) return false;
-    big += (size_t)cl_ld(A.L[k].n) * A.L[k].w + (size_t)A.L[k].n;
+    big += (size_t)cl_ld(A.L[k].n, A.L[k].rep) * A.L[k].w + (size_t)A.L[k].n;
   }
   if (big > (size_t)1 << 20) return false;  // far beyond shared memory: the sums stay small
   cl_layout<V>(A, nullptr, &A.share, &A.total);
   return A.total + kClStatic <= kSmemMax;
 }
 
-// v to *p of every block of the cluster, the g lanes of a group taking the blocks in turn
+// The block's rows [r0, r0 + R) of vector y, written in its own copy before a block barrier, to
+// the copies of the other blocks: warp w serves block w with 16-byte stores.  (One 4-byte store
+// per row and block, from the lanes that hold the row, took 2,800 clocks of a 3,179-row level's
+// phase, most of it the stores' issue.)
 template <class V>
-__device__ __forceinline__ void cl_broadcast(V *p, V v, int sub, int g) {
-  for (int d = sub; d < kClBlocks; d += g) remote_store(cluster_addr(p, d), v);
+__device__ __forceinline__ void cl_spread(V *y, int r0, int R, int rank) {
+  static_assert(kClThreads / 32 == kClBlocks, "a warp per block");
+  const int lane = threadIdx.x & 31, d = threadIdx.x >> 5;
+  if (d == rank) return;
+  const int words = R * (int)sizeof(V) / 16;
+  const float4 *src = reinterpret_cast<const float4 *>(y + r0);
+  const unsigned dst = cluster_addr(y + r0, d);
+  for (int c = lane; c < words; c += 32) remote_store(dst + 16u * c, src[c]);
 }
 
 // The block's share of every level, packed: block r of the grid writes block r's image.
@@ -1201,7 +1220,8 @@ __global__ void __launch_bounds__(kClThreads) cl_pack(const __grid_constant__ Cl
   const int last = A.nl - 1;
   for (int k = 0; k < A.nl; ++k) {
     const ClLevel<V> &L = A.L[k];
-    const int n = L.n, R = cl_rows_per_block(n), ld = cl_ld(n), r0 = rank * R, rows = max(0, min(R, n - r0));
+    const int n = L.n, R = cl_rows_per_block(n, L.rep), ld = cl_ld(n, L.rep), r0 = L.rep ? 0 : rank * R;
+    const int rows = max(0, min(R, n - r0));
     V *val = (V *)(img + off[k].val), *dinv = (V *)(img + off[k].dinv);
     uint16_t *col = (uint16_t *)(img + off[k].col), *agg = (uint16_t *)(img + off[k].agg);
     uint16_t *mptr = (uint16_t *)(img + off[k].mptr), *mem = (uint16_t *)(img + off[k].mem);
@@ -1233,16 +1253,26 @@ struct ClView {
   const V *val, *dinv;        // dinv: the block's rows
   const uint16_t *col;
   V *xa, *xb, *b;
-  int n, w, g, rows, r0, ld;
+  int n, w, lg, rows, r0, ld;  // lg: log2 of the lanes per row
+  bool rep;
+
+  // the end of a phase whose rows are in the block's own copy of y: on return every block has
+  // all rows of it
+  __device__ __forceinline__ void phase_end(V *y, int rank) const {
+    __syncthreads();
+    if (rep) return;
+    cl_spread(y, r0, cl_rows_per_block(n), rank);
+    cluster_barrier();
+  }
 };
 
 // v[i] = x[i] + om dinv_i (b_i - sum_k a_ik x(col_ik)) (RES: b_i - the sum) for the block's
-// rows of a level, g lanes per row, handed to out(row, value, lane of the group)
-template <bool RES, class V, class F>
-__device__ __forceinline__ void cl_rows(const ClView<V> &Q, const V *x, V om, F out) {
-  const int g = Q.g, sub = threadIdx.x & (g - 1), per = kClThreads / g, step = g * Q.ld;
+// rows of a level, g lanes per row, into y[i]
+template <bool RES, class V>
+__device__ __forceinline__ void cl_rows(const ClView<V> &Q, const V *x, V om, V *y) {
+  const int g = 1 << Q.lg, sub = threadIdx.x & (g - 1), per = kClThreads >> Q.lg, step = Q.ld << Q.lg;
   for (int i0 = 0; i0 < Q.rows; i0 += per) {  // the same count for the whole block (shuffles)
-    const int i = i0 + (int)threadIdx.x / g;
+    const int i = i0 + (int)(threadIdx.x >> Q.lg);
     const bool act = i < Q.rows;
     V s = V(0), bi = V(0), xi = V(0), di = V(0);
     if (act) {
@@ -1264,8 +1294,10 @@ __device__ __forceinline__ void cl_rows(const ClView<V> &Q, const V *x, V om, F 
       }
       for (; k < Q.w; k += g, vp += step, cp += step) s += *vp * x[*cp];
     }
-    for (int o = g >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (act) out(i, RES ? bi - s : xi + om * di * (bi - s), sub);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1)
+      if (o < g) s += __shfl_xor_sync(0xffffffffu, s, o);  // g <= 16
+    if (act && sub == 0) y[i] = RES ? bi - s : xi + om * di * (bi - s);
   }
 }
 
@@ -1274,7 +1306,7 @@ template <class V>
 struct ClCtx {
   unsigned char *smem;
   const ClOffsets *off;
-  const int4 *dim;            // n, w, g of each level
+  const int4 *dim;            // n, w, log2 g, rep of each level
   int rank, last, sweeps;
   V om, al;
 
@@ -1286,9 +1318,10 @@ struct ClCtx {
     ClView<V> Q;
     Q.n = q.x;
     Q.w = q.y;
-    Q.g = q.z;
-    const int R = cl_rows_per_block(Q.n);
-    Q.r0 = rank * R;
+    Q.lg = q.z;
+    Q.rep = q.w != 0;
+    const int R = cl_rows_per_block(Q.n, q.w);
+    Q.r0 = Q.rep ? 0 : rank * R;
     Q.rows = max(0, min(R, Q.n - Q.r0));
     Q.ld = R | 1;
     Q.val = ptr(o.val);
@@ -1312,7 +1345,7 @@ __device__ __forceinline__ void cl_stage(const ClArgs<V> &A, unsigned char *smem
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d + o), "l"(src + o) : "memory");
   asm volatile("cp.async.commit_group;\n" ::: "memory");
   if (t == 0) cl_layout<V>(A, off, nullptr, nullptr);
-  if (t >= 32 && t - 32 < A.nl) dim[t - 32] = make_int4(A.L[t - 32].n, A.L[t - 32].w, A.L[t - 32].g, 0);
+  if (t >= 32 && t - 32 < A.nl) dim[t - 32] = make_int4(A.L[t - 32].n, A.L[t - 32].w, 31 - __clz(A.L[t - 32].g), A.L[t - 32].rep);
   __syncthreads();
 }
 __device__ __forceinline__ void cl_staged() {
@@ -1336,12 +1369,12 @@ __device__ __forceinline__ V *cl_vcycle(const ClCtx<V> &X, V *out) {
     const ClView<V> Q = X.view(k);
     V *x = Q.xb, *y = Q.xa;
     for (int q = 1; q < sw; ++q) {
-      cl_rows<false>(Q, x, om, [&](int i, V v, int sub) { cl_broadcast(y + Q.r0 + i, v, sub, Q.g); });
-      cluster_barrier();
+      cl_rows<false>(Q, x, om, y + Q.r0);
+      Q.phase_end(y, X.rank);
       V *z = x; x = y; y = z;
     }
-    cl_rows<true>(Q, x, om, [&](int i, V v, int sub) { cl_broadcast(y + Q.r0 + i, v, sub, Q.g); });
-    cluster_barrier();
+    cl_rows<true>(Q, x, om, y + Q.r0);
+    Q.phase_end(y, X.rank);
     // the coarse right-hand side, in member order, and its first sweep
     const ClView<V> C = X.view(k + 1);
     const uint16_t *mptr = X.idx(X.off[k].mptr), *mem = X.idx(X.off[k].mem);
@@ -1366,30 +1399,28 @@ __device__ __forceinline__ V *cl_vcycle(const ClCtx<V> &X, V *out) {
     for (int j = lane; j < K.n; j += 32) s += K.val[i * K.n + j] * K.b[j];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (last == 0 && out) {
-      if (lane == 0) out[K.r0 + i] = s;
-    } else {
-      cl_broadcast(K.xa + K.r0 + i, s, lane, 32);
+    if (lane == 0) {
+      if (last > 0 || !out) K.xa[K.r0 + i] = s;
+      else if (!K.rep || X.rank == 0) out[K.r0 + i] = s;
     }
   }
   if (last == 0 && out) return nullptr;
-  cluster_barrier();
+  K.phase_end(K.xa, X.rank);
   // ---- up ----
   V *xc = K.xa;
   for (int k = last - 1; k >= 0; --k) {
     const ClView<V> Q = X.view(k);
     V *x = (sw & 1) ? Q.xb : Q.xa, *y = (sw & 1) ? Q.xa : Q.xb;
     const uint16_t *agg = X.idx(X.off[k].agg);
+#pragma unroll 4
     for (int i = t; i < Q.n; i += kClThreads) x[i] += al * xc[agg[i]];
     __syncthreads();
     for (int q = 0; q < sw; ++q) {
       if (out && k == 0 && q + 1 == sw) {
-        cl_rows<false>(Q, x, om, [&](int i, V v, int sub) {
-          if (sub == 0) out[Q.r0 + i] = v;
-        });
+        cl_rows<false>(Q, x, om, out + Q.r0);
       } else {
-        cl_rows<false>(Q, x, om, [&](int i, V v, int sub) { cl_broadcast(y + Q.r0 + i, v, sub, Q.g); });
-        cluster_barrier();
+        cl_rows<false>(Q, x, om, y + Q.r0);
+        Q.phase_end(y, X.rank);
       }
       V *z = x; x = y; y = z;
     }
@@ -1465,7 +1496,7 @@ struct ClSolveArgs {
   double *x;                  // the initial guess, the solution
   T *V, *Z;                   // basis, preconditioned vectors (own rows of each block)
   size_t vn;
-  int M, max_it, max_outer, exact_inner, g;  // g: lanes per row of a product
+  int M, max_it, max_outer, exact_inner, lg;  // lg: log2 of the lanes per row of a product
   double rtol, atol, dtol, rtol_in;
   unsigned o_col, o_vec, total;  // without a V-cycle: columns and gathered vector after the values
   ClResult *out;
@@ -1534,10 +1565,13 @@ __global__ void __launch_bounds__(kClThreads, 1) solve_cluster(const __grid_cons
       if (lane == 0) S.wsum[warp][0] = v;
     } else {
 #pragma unroll
-      for (int j = 0; j < NV; ++j)
-        if (j < nv) {
-          const double v = warp_sum(f(j));
-          if (lane == 0) S.wsum[warp][j] = v;
+      for (int j0 = 0; j0 < NV; j0 += 8)
+        if (j0 < nv) {
+          double v[8];
+#pragma unroll
+          for (int q = 0; q < 8; ++q) v[q] = j0 + q < nv ? f(j0 + q) : 0.0;
+          const double sum = warp_sum8(v, lane);
+          if ((lane & 3) == 0) S.wsum[warp][j0 + (lane >> 2)] = sum;
         }
     }
     __syncthreads();
@@ -1560,9 +1594,9 @@ __global__ void __launch_bounds__(kClThreads, 1) solve_cluster(const __grid_cons
   };
   // the product of the block's rows with x, into S.row; ends with a block barrier
   auto product = [&](auto x) {
-    const int g = A.g, sub = t & (g - 1), per = kClThreads / g;
+    const int g = 1 << A.lg, sub = t & (g - 1), per = kClThreads >> A.lg;
     for (int i0 = 0; i0 < rows; i0 += per) {
-      const int i = i0 + t / g;
+      const int i = i0 + (t >> A.lg);
       T s = T(0);
       if (i < rows) {
 #pragma unroll 4
@@ -1572,20 +1606,28 @@ __global__ void __launch_bounds__(kClThreads, 1) solve_cluster(const __grid_cons
           s += a * x(one_level ? A.col[at] : (int)col[k * ld + i]);
         }
       }
-      for (int o = g >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1)
+        if (o < g) s += __shfl_xor_sync(0xffffffffu, s, o);
       if (i < rows && sub == 0) S.row[i] = (double)s;
     }
     __syncthreads();
   };
-  // v of the row, not yet normalised, to every block (for the next V-cycle or product)
+  // v of the row, not yet normalised, to every block (for the next V-cycle or product); a
+  // reduction follows, whose cluster barrier completes it
   auto publish = [&](T v) {
-    if (!own) return;
     if constexpr (MG) {
       const ClView<TV> Q = X.view(0);
-      if (one_level) cl_broadcast(Q.b + row, (TV)v, 0, 1);
-      else cl_broadcast(Q.xb + row, od * (TV)v, 0, 1);
+      TV *y = one_level ? Q.b : Q.xb;
+      if (own) y[row] = one_level ? (TV)v : od * (TV)v;
+      __syncthreads();
+      if (!Q.rep) cl_spread(y, r0, R, rank);
+      else if (own)  // one small level, whole in every block
+        for (int d = 0; d < kClBlocks; ++d) remote_store(cluster_addr(y + row, d), y[row]);
     } else {
-      cl_broadcast(vec + row, v, 0, 1);
+      if (own) vec[row] = v;
+      __syncthreads();
+      cl_spread(vec, r0, R, rank);
     }
   };
 
@@ -1652,6 +1694,7 @@ __global__ void __launch_bounds__(kClThreads, 1) solve_cluster(const __grid_cons
         if (one_level) {
           for (int i = t; i < n; i += kClThreads) Q.b[i] *= sc;
         } else {
+#pragma unroll 4
           for (int i = t; i < n; i += kClThreads) Q.xb[i] *= sc;
           if (own) Q.b[t] = (TV)(w * (T)scale);
         }
@@ -2558,7 +2601,9 @@ static int cluster_levels(apc_context *c, MgHier<T> &H) {
       D.agg = Q.agg;
       D.mptr = k + 1 < A.nl ? H.lv[l + k + 1].mptr : nullptr;
       D.mem = k + 1 < A.nl ? H.lv[l + k + 1].mem : nullptr;
-      D.g = tail_lanes(cl_rows_per_block(Q.n), Q.w, kClThreads);
+      const bool last = k + 1 == A.nl;
+      D.rep = (last || k > 0) && (size_t)Q.n * (last ? Q.n : Q.w) <= (size_t)kClRepEntries ? 1 : 0;
+      D.g = tail_lanes(cl_rows_per_block(Q.n, D.rep), Q.w, kClThreads);
     }
     if (!cl_fits(A)) continue;
     APC_TRY(apc_ensure(c, &H.cl_img, (size_t)A.share * kClBlocks));
@@ -3291,7 +3336,7 @@ static int cluster_solve(apc_context *c, const IrSolveArgs<T> &a, bool *done) {
   A.max_it = a.max_it;
   A.max_outer = a.max_outer;
   A.exact_inner = sizeof(T) == sizeof(double) ? 1 : 0;
-  A.g = tail_lanes(R, a.w, kClThreads);
+  for (int g = tail_lanes(R, a.w, kClThreads); g > 1; g /= 2) ++A.lg;
   A.rtol = a.rtol;
   A.atol = a.atol;
   A.dtol = a.dtol;
@@ -3306,7 +3351,7 @@ static int cluster_solve(apc_context *c, const IrSolveArgs<T> &a, bool *done) {
   } else {
     A.o_col = tail_align((size_t)a.w * (R | 1) * sizeof(T));
     A.o_vec = A.o_col + tail_align((size_t)a.w * (R | 1) * sizeof(uint16_t));
-    A.total = A.o_vec + tail_align((size_t)a.n * sizeof(T));
+    A.total = A.o_vec + tail_align((size_t)R * kClBlocks * sizeof(T));
   }
   if (A.total > kClSolveDyn) return APC_OK;
   APC_TRY(ensure_result(c));
