@@ -247,7 +247,7 @@ int apc_reset_profile(apc_context *ctx);
  * synchronisation of cudaMalloc / cudaFree.  No counterpart in the reference: it has no
  * GPU code and no caller with this constraint.
  *
- * This call allocates nothing.  Its scratch (particle -> cell map, max-change
+ * This call allocates nothing.  Its scratch (a bit per particle, max-change
  * accumulator) is a fixed 4 MiB + 256 B array inside the library that every GPU loading
  * the library keeps until the process exits, so n_particles may not exceed
  * APC_NOALLOC_MAX_PARTICLES (larger sizes return APC_ERR_INVALID_ARG).  The first call
