@@ -158,6 +158,46 @@ __global__ void unpermute6(int n, const int *__restrict__ pid, Arrays6 a) {
   }
 }
 
+// the caller's six arrays into the context's, and the identity for the particle ids
+__global__ void load6(int n, Arrays6 a, int *__restrict__ pid) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    double v[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) v[k] = a.src[k][i];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) a.dst[k][i] = v[k];
+    pid[i] = i;
+  }
+}
+
+// Whether a kernel of the context may use the array of c->n doubles at p directly: at a whole
+// double, in the memory of its device, and inside one allocation.  A copy checks as much itself,
+// and also takes other devices' memory and odd addresses.
+bool kernel_array(const apc_context *c, const void *p) {
+  using RangeFn = int (*)(unsigned long long *, size_t *, unsigned long long);  // cuMemGetAddressRange
+  static const RangeFn range = [] {
+    void *f = nullptr;
+    cudaDriverEntryPointQueryResult q{};
+    if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      f = nullptr;
+    }
+    return (RangeFn)f;
+  }();
+  if (!range || ((uintptr_t)p & 7)) return false;
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (at.type != cudaMemoryTypeDevice || at.device != c->dev) return false;
+  unsigned long long base = 0;
+  size_t size = 0;
+  if (range(&base, &size, (unsigned long long)(uintptr_t)p) != 0) return false;
+  return (unsigned long long)(uintptr_t)p + sizeof(double) * (size_t)c->n <= base + size;
+}
+
 // dst_k[s] = src_k[pid[s]]: the caller-order velocities of a fresh upload, in sorted order
 __global__ void gather3(int n, const int *__restrict__ pid, const double *__restrict__ x, const double *__restrict__ y,
                         const double *__restrict__ z, double *__restrict__ ox, double *__restrict__ oy,
@@ -383,6 +423,17 @@ int apc_destroy(apc_context *c) {
   return APC_OK;
 }
 
+// the context holds a new particle set, the velocities in the caller's order
+static int particles_set(apc_context *c) {
+  c->vel_caller_order = true;
+  c->have_particles = true;
+  c->have_cells = false;
+  c->have_fields = false;
+  c->warm_cap = 0;  // a new particle set: no guess from the previous one
+  // levels_hint stays: a selection deeper than the hint redoes the sort over every bit
+  return APC_OK;
+}
+
 static int set_particles_impl(apc_context *c, const double *const *src, cudaMemcpyKind kind) {
   if (!c) return APC_ERR_INVALID_ARG;
   for (int k = 0; k < 6; ++k)
@@ -390,6 +441,22 @@ static int set_particles_impl(apc_context *c, const double *const *src, cudaMemc
   cudaSetDevice(c->dev);
   const size_t bytes = sizeof(double) * (size_t)c->n;
   double *dst[6] = {c->px, c->py, c->pz, c->pvx, c->pvy, c->pvz};
+  const int G = std::max(1, std::min((c->n + 255) / 256, apc_sm_count(c) * 8));
+  bool direct = kind == cudaMemcpyDeviceToDevice;
+  for (int k = 0; k < 6 && direct; ++k) direct = kernel_array(c, src[k]);
+  if (direct) {
+    // one kernel instead of six copies and the ids (an earlier upload may still write pvx ..)
+    APC_CUDA_TRY(c, cudaStreamWaitEvent(c->s, c->vel_ev, 0));
+    Arrays6 a{};
+    for (int k = 0; k < 6; ++k) {
+      a.src[k] = src[k];
+      a.dst[k] = dst[k];
+    }
+    load6<<<G, 256, 0, c->s>>>(c->n, a, c->pid);
+    apc_count_launch(c);
+    APC_CUDA_TRY(c, cudaGetLastError());
+    return particles_set(c);
+  }
   for (int k = 0; k < 3; ++k) APC_CUDA_TRY(c, cudaMemcpyAsync(dst[k], src[k], bytes, kind, c->s));
   // the velocities in the caller's order, on the copy stream after the work already queued
   // (which may still read them); the kick gathers them into the sorted order
@@ -397,16 +464,10 @@ static int set_particles_impl(apc_context *c, const double *const *src, cudaMemc
   APC_CUDA_TRY(c, cudaStreamWaitEvent(c->cs, c->cs_ev, 0));
   for (int k = 3; k < 6; ++k) APC_CUDA_TRY(c, cudaMemcpyAsync(dst[k], src[k], bytes, kind, c->cs));
   APC_CUDA_TRY(c, cudaEventRecord(c->vel_ev, c->cs));
-  c->vel_caller_order = true;
-  iota_int<<<std::max(1, std::min((c->n + 255) / 256, apc_sm_count(c) * 8)), 256, 0, c->s>>>(c->n, c->pid);
+  iota_int<<<G, 256, 0, c->s>>>(c->n, c->pid);
   apc_count_launch(c);
   APC_CUDA_TRY(c, cudaGetLastError());
-  c->have_particles = true;
-  c->have_cells = false;
-  c->have_fields = false;
-  c->warm_cap = 0;  // a new particle set: no guess from the previous one
-  // levels_hint stays: a selection deeper than the hint redoes the sort over every bit
-  return APC_OK;
+  return particles_set(c);
 }
 
 int apc_set_particles(apc_context *c, const double *x, const double *y, const double *z, const double *vx,
@@ -434,16 +495,20 @@ static int get_particles_impl(apc_context *c, double *const *dst, int count, cud
   for (int k0 = 0; k0 < count; k0 += 6) {
     Arrays6 a{};
     int which[6];
+    bool direct = kind == cudaMemcpyDeviceToDevice;
     for (int k = k0; k < count && k < k0 + 6; ++k) {
       if (!dst[k]) continue;
+      direct = direct && kernel_array(c, dst[k]);
       a.src[a.count] = src[k];
       a.dst[a.count] = spare[a.count];
       which[a.count++] = k;
     }
     if (a.count == 0) continue;
+    if (direct)  // straight into the caller's arrays
+      for (int j = 0; j < a.count; ++j) a.dst[j] = dst[which[j]];
     unpermute6<<<G, 256, 0, c->s>>>(c->n, c->pid, a);
     apc_count_launch(c);
-    for (int j = 0; j < a.count; ++j) APC_CUDA_TRY(c, cudaMemcpyAsync(dst[which[j]], a.dst[j], bytes, kind, c->s));
+    for (int j = 0; j < a.count && !direct; ++j) APC_CUDA_TRY(c, cudaMemcpyAsync(dst[which[j]], a.dst[j], bytes, kind, c->s));
   }
   APC_CUDA_TRY(c, apc_stream_wait(c));
   return APC_OK;
