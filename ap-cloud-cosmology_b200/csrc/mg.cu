@@ -85,15 +85,23 @@ __global__ void ell_dinv(int n, size_t ld, const V *__restrict__ val, V *__restr
   }
 }
 
-// Galerkin row I of A_c = P^T A P, one warp per coarse row.  The (J, a) contributions of
-// the members' rows are taken 32 at a time in member-then-slot order; lanes with equal J
-// are merged by their lowest lane, which adds the values in lane order into a shared-
-// memory hash table keyed by J (one writer per J per round, so every coarse entry is
-// summed in contribution order).  The distinct entries are then written sorted by J.
-// The result does not depend on scheduling, so the hierarchy is deterministic.
+// Galerkin row I of A_c = P^T A P, one warp per coarse row, written straight into the level's
+// slot-major ELL.  The (J, a) contributions of the members' rows are taken 32 at a time in
+// member-then-slot order; lanes with equal J are merged by their lowest lane, which adds the
+// values in lane order into a shared-memory hash table keyed by J (one writer per J per round, so
+// every coarse entry is summed in contribution order).  The distinct entries are then placed
+// sorted by J.  The result does not depend on scheduling, so the hierarchy is deterministic.
+// A row is a chain of dependent loads (member, column, aggregate) and table rounds: the loads
+// of kGalAhead rounds are issued together, and the table is as large as the row's
+// contributions need.  The ELL is padded to its wslots slots (own column, value zero), since
+// the level's width is known only when every row is done: it goes to *width (and *overflow when
+// a row has more distinct columns than slots; the build then runs again with room for it).
+// The products, their widths and transposes were 3 kernels a level; with one a 4k box's step
+// takes 1.04 ms instead of 1.10, a 48^3 box 1.79 instead of 1.86, the 262k ball 2.88 instead of 2.99.
 constexpr int kGalWarps = 4;
 constexpr int kGalTab = 512;   // hash slots per warp
 constexpr int kGalRows = 256;  // distinct coarse columns per row
+constexpr int kGalAhead = 5;   // 8 members of 18 slots are 144 contributions
 
 template <class V>
 __global__ void __launch_bounds__(32 * kGalWarps) galerkin_rows(int nc, const int *__restrict__ mptr, int nf,
@@ -101,9 +109,10 @@ __global__ void __launch_bounds__(32 * kGalWarps) galerkin_rows(int nc, const in
                                                               const int *__restrict__ wf_dev, int wf_cap, size_t ldf,
                                                               const int *__restrict__ colf,
                                                               const V *__restrict__ valf,
-                                                              const int *__restrict__ agg, int wcap,
-                                                              int *__restrict__ rowlen, int *__restrict__ tcol,
-                                                              V *__restrict__ tval, int *__restrict__ err) {
+                                                              const int *__restrict__ agg, int wslots, size_t ld,
+                                                              int *__restrict__ col, V *__restrict__ val,
+                                                              V *__restrict__ dinv, int *__restrict__ width,
+                                                              int *__restrict__ overflow, int *__restrict__ err) {
   __shared__ int tkey[kGalWarps][kGalTab];
   __shared__ double tsum[kGalWarps][kGalTab];
   __shared__ double stage[kGalWarps][32];
@@ -115,47 +124,63 @@ __global__ void __launch_bounds__(32 * kGalWarps) galerkin_rows(int nc, const in
   const int lane = threadIdx.x & 31, wv = threadIdx.x >> 5;
   int *K = tkey[wv];
   double *T = tsum[wv];
+  int widest = 0;
   for (int I = blockIdx.x * kGalWarps + wv; I < nc; I += gridDim.x * kGalWarps) {
     const int a = mptr[I], e = (I + 1 < nc) ? mptr[I + 1] : nf;
     const int cnt = (e - a) * wf;
-    for (int t = lane; t < kGalTab; t += 32) K[t] = -1;
+    // distinct columns are at most the contributions: a quarter of the slots stays free
+    const int bits = cnt <= 96 ? 7 : (cnt <= 192 ? 8 : 9), tab = 1 << bits;
+    for (int t = lane; t < tab; t += 32) K[t] = -1;
     __syncwarp();
     bool bad = false;
-    for (int t0 = 0; t0 < cnt; t0 += 32) {
-      const int t = t0 + lane;
-      int J = -1;
-      double v = 0.0;
-      if (t < cnt) {
-        const int i = mem[a + t / wf], sl = t % wf;
-        const size_t at = (size_t)sl * ldf + i;
-        J = agg[colf[at]];
-        v = (double)valf[at];
-      }
-      stage[wv][lane] = v;
-      __syncwarp();
-      const unsigned peers = __match_any_sync(0xffffffffu, J);
-      if (J >= 0 && lane == __ffs(peers) - 1) {
-        double sum = 0.0;
-        for (unsigned q = peers; q; q &= q - 1) sum += stage[wv][__ffs(q) - 1];
-        unsigned h = ((unsigned)J * 2654435761u) >> (32 - 9);
-        bool placed = false;
-        for (int probe = 0; probe < kGalTab && !placed; ++probe, h = (h + 1) & (kGalTab - 1)) {
-          const int cur = atomicCAS(&K[h], -1, J);
-          if (cur == -1) {
-            T[h] = sum;
-            placed = true;
-          } else if (cur == J) {
-            T[h] += sum;
-            placed = true;
-          }
+    for (int t0 = 0; t0 < cnt; t0 += 32 * kGalAhead) {
+      int Js[kGalAhead];
+      V vs[kGalAhead];
+#pragma unroll
+      for (int u = 0; u < kGalAhead; ++u) {
+        const int t = t0 + 32 * u + lane;
+        Js[u] = -1;
+        vs[u] = V(0);
+        if (t < cnt) {
+          const int q = t / wf;
+          const size_t at = (size_t)(t - q * wf) * ldf + mem[a + q];
+          Js[u] = colf[at];
+          vs[u] = valf[at];
         }
-        if (!placed) bad = true;
       }
-      __syncwarp();
+#pragma unroll
+      for (int u = 0; u < kGalAhead; ++u)
+        if (Js[u] >= 0) Js[u] = agg[Js[u]];
+#pragma unroll
+      for (int u = 0; u < kGalAhead; ++u) {
+        if (t0 + 32 * u >= cnt) break;
+        const int J = Js[u];
+        stage[wv][lane] = (double)vs[u];
+        __syncwarp();
+        const unsigned peers = __match_any_sync(0xffffffffu, J);
+        if (J >= 0 && lane == __ffs(peers) - 1) {
+          double sum = 0.0;
+          for (unsigned q = peers; q; q &= q - 1) sum += stage[wv][__ffs(q) - 1];
+          unsigned h = ((unsigned)J * 2654435761u) >> (32 - bits);
+          bool placed = false;
+          for (int probe = 0; probe < tab && !placed; ++probe, h = (h + 1) & (tab - 1)) {
+            const int cur = atomicCAS(&K[h], -1, J);
+            if (cur == -1) {
+              T[h] = sum;
+              placed = true;
+            } else if (cur == J) {
+              T[h] += sum;
+              placed = true;
+            }
+          }
+          if (!placed) bad = true;
+        }
+        __syncwarp();
+      }
     }
     // compact the occupied slots, then place each by its rank in J
     int nd = 0;
-    for (int t0 = 0; t0 < kGalTab; t0 += 32) {
+    for (int t0 = 0; t0 < tab; t0 += 32) {
       const int key = K[t0 + lane];
       const unsigned occ = __ballot_sync(0xffffffffu, key >= 0);
       const int pos = nd + __popc(occ & ((1u << lane) - 1u));
@@ -167,55 +192,36 @@ __global__ void __launch_bounds__(32 * kGalWarps) galerkin_rows(int nc, const in
     }
     __syncwarp();
     const int len = min(nd, kGalRows);
+    bool diag = false;
     for (int q = lane; q < len; q += 32) {
       const int key = dkey[wv][q];
+      const V v = (V)dval[wv][q];
       int rank = 0;
       for (int u = 0; u < len; ++u) rank += dkey[wv][u] < key ? 1 : 0;
-      if (rank < wcap) {
-        tcol[(size_t)I * wcap + rank] = key;
-        tval[(size_t)I * wcap + rank] = (V)dval[wv][q];
+      if (rank < wslots) {
+        col[(size_t)rank * ld + I] = key;
+        val[(size_t)rank * ld + I] = v;
+        if (key == I) {
+          diag = true;
+          dinv[I] = v != V(0) ? V(1) / v : V(1);
+        }
       }
     }
+    for (int q = len + lane; q < wslots; q += 32) {
+      col[(size_t)q * ld + I] = I;
+      val[(size_t)q * ld + I] = V(0);
+    }
+    diag = __any_sync(0xffffffffu, diag);
     bad = __any_sync(0xffffffffu, bad);
     if (lane == 0) {
-      rowlen[I] = nd;
-      if (bad || nd > wcap || nd > kGalRows) atomicOr(err, DERR_STENCIL_MANY);
+      if (!diag) dinv[I] = V(1);
+      if (bad || nd > kGalRows) atomicOr(err, DERR_STENCIL_MANY);
+      if (nd > wslots) atomicExch(overflow, 1);
     }
+    widest = max(widest, nd);
     __syncwarp();
   }
-}
-
-template <class V>
-__global__ void rows_to_ell(int n, const int *__restrict__ w_dev, int wslots, size_t ld, int wcap,
-                            const int *__restrict__ rowlen, const int *__restrict__ tcol,
-                            const V *__restrict__ tval, int *__restrict__ col, V *__restrict__ val,
-                            V *__restrict__ dinv, int *__restrict__ overflow) {
-  // the level's width (max_int, just before); the ELL holds wslots slots, and a wider level
-  // is flagged (the build then runs again with room for it)
-  const int wd = *w_dev;
-  const int w = min(wd, wslots);
-  if (wd > wslots && blockIdx.x == 0 && threadIdx.x == 0) atomicExch(overflow, 1);
-  for (int I = blockIdx.x * blockDim.x + threadIdx.x; I < n; I += gridDim.x * blockDim.x) {
-    const int len = rowlen[I];
-    V d = V(0);
-    for (int s = 0; s < w; ++s) {
-      const bool in = s < len;
-      const int c = in ? tcol[(size_t)I * wcap + s] : I;
-      const V v = in ? tval[(size_t)I * wcap + s] : V(0);
-      col[(size_t)s * ld + I] = c;
-      val[(size_t)s * ld + I] = v;
-      if (in && c == I) d += v;
-    }
-    dinv[I] = d != V(0) ? V(1) / d : V(1);
-  }
-}
-
-__global__ void max_int(int n, const int *__restrict__ a, int *out) {
-  int m = 0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) m = max(m, a[i]);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(out, m);
+  if (lane == 0 && widest > 0) atomicMax(width, widest);
 }
 
 // The coarsest level's explicit inverse: Gauss-Jordan elimination on [A | I] in FP64
@@ -1209,42 +1215,44 @@ __device__ __forceinline__ void cl_spread(V *y, int r0, int R, int rank) {
   for (int c = lane; c < words; c += 32) remote_store(dst + 16u * c, src[c]);
 }
 
-// The block's share of every level, packed: block r of the grid writes block r's image.
+// The block's share of every level, packed: grid (rank, level, part) writes the part of that
+// level in block `rank`'s image (kClPackParts parts of each array).
+constexpr int kClPackParts = 4;
 template <class V>
 __global__ void __launch_bounds__(kClThreads) cl_pack(const __grid_constant__ ClArgs<V> A) {
   __shared__ ClOffsets off[kClLevels];
-  const int t = threadIdx.x, rank = blockIdx.x;
+  const int t0 = blockIdx.z * kClThreads + threadIdx.x, step = kClPackParts * kClThreads;
+  const int t = threadIdx.x, rank = blockIdx.x, k = blockIdx.y;
   if (t == 0) cl_layout<V>(A, off, nullptr, nullptr);
   __syncthreads();
   unsigned char *img = A.img + (size_t)rank * A.share;
   const int last = A.nl - 1;
-  for (int k = 0; k < A.nl; ++k) {
-    const ClLevel<V> &L = A.L[k];
-    const int n = L.n, R = cl_rows_per_block(n, L.rep), ld = cl_ld(n, L.rep), r0 = L.rep ? 0 : rank * R;
-    const int rows = max(0, min(R, n - r0));
-    V *val = (V *)(img + off[k].val), *dinv = (V *)(img + off[k].dinv);
-    uint16_t *col = (uint16_t *)(img + off[k].col), *agg = (uint16_t *)(img + off[k].agg);
-    uint16_t *mptr = (uint16_t *)(img + off[k].mptr), *mem = (uint16_t *)(img + off[k].mem);
-    if (k == last) {
-      for (int e = t; e < rows * n; e += kClThreads) val[e] = A.inv[(size_t)r0 * n + e];
-      continue;
-    }
-    for (int e = t; e < ld * L.w; e += kClThreads) {
-      const int s = e / ld, i = e - s * ld;
-      const size_t at = (size_t)s * L.ld + r0 + i;
-      val[e] = i < rows ? L.val[at] : V(0);
-      col[e] = i < rows ? (uint16_t)L.col[at] : (uint16_t)0;
-    }
-    const int nc = A.L[k + 1].n;
-    for (int i = t; i < n; i += kClThreads) {
-      agg[i] = (uint16_t)L.agg[i];
-      mem[i] = (uint16_t)L.mem[i];
-      if (k > 0) dinv[i] = L.dinv[i];
-    }
-    if (k == 0)
-      for (int i = t; i < rows; i += kClThreads) dinv[i] = L.dinv[r0 + i];
-    for (int i = t; i <= nc; i += kClThreads) mptr[i] = (uint16_t)(i < nc ? L.mptr[i] : n);
+  const ClLevel<V> &L = A.L[k];
+  const int n = L.n, R = cl_rows_per_block(n, L.rep), ld = cl_ld(n, L.rep), r0 = L.rep ? 0 : rank * R;
+  const int rows = max(0, min(R, n - r0));
+  V *val = (V *)(img + off[k].val), *dinv = (V *)(img + off[k].dinv);
+  uint16_t *col = (uint16_t *)(img + off[k].col), *agg = (uint16_t *)(img + off[k].agg);
+  uint16_t *mptr = (uint16_t *)(img + off[k].mptr), *mem = (uint16_t *)(img + off[k].mem);
+  if (k == last) {
+    for (int e = t0; e < rows * n; e += step) val[e] = A.inv[(size_t)r0 * n + e];
+    return;
   }
+#pragma unroll 2
+  for (int e = t0; e < ld * L.w; e += step) {
+    const int s = e / ld, i = e - s * ld;
+    const size_t at = (size_t)s * L.ld + r0 + i;
+    val[e] = i < rows ? L.val[at] : V(0);
+    col[e] = i < rows ? (uint16_t)L.col[at] : (uint16_t)0;
+  }
+  const int nc = A.L[k + 1].n;
+  for (int i = t0; i < n; i += step) {
+    agg[i] = (uint16_t)L.agg[i];
+    mem[i] = (uint16_t)L.mem[i];
+    if (k > 0) dinv[i] = L.dinv[i];
+  }
+  if (k == 0)
+    for (int i = t0; i < rows; i += step) dinv[i] = L.dinv[r0 + i];
+  for (int i = t0; i <= nc; i += step) mptr[i] = (uint16_t)(i < nc ? L.mptr[i] : n);
 }
 
 // a level as the phases see it
@@ -2361,7 +2369,6 @@ struct MgHier {
   int nlev = 0;
   T *coarse_inv = nullptr;
   int coarse_n = 0;
-  T *uval = nullptr;  // coarse rows before the ELL transpose
   // the levels run by vcycle_cluster: from cl_first on (-1: none fit), their packed shares
   ClArgs<T> cl{};
   int cl_first = -1;
@@ -2377,7 +2384,7 @@ struct MgWork {
   // hierarchy temporaries: parent-code sort, flags, coarse rows before the ELL transpose
   uint64_t *pkey = nullptr, *pkey_alt = nullptr;
   uint32_t *pidx = nullptr, *pidx_alt = nullptr;
-  int *eflag = nullptr, *epos = nullptr, *ucol = nullptr, *rowstart = nullptr;
+  int *eflag = nullptr, *epos = nullptr;
   size_t vn = 0;
   double *partial = nullptr, *dots = nullptr;
   unsigned *counter = nullptr;
@@ -2458,7 +2465,7 @@ static void free_hier(apc_context *c, MgHier<T> &H) {
     apc_free(c, L.b);
     apc_free(c, L.r);
   }
-  void *p[] = {H.coarse_inv, H.uval, H.cl_img, H.V, H.Z, H.vin, H.vout, H.dvec};
+  void *p[] = {H.coarse_inv, H.cl_img, H.V, H.Z, H.vin, H.vout, H.dvec};
   for (void *q : p) apc_free(c, q);
 }
 
@@ -2473,8 +2480,8 @@ void apc_mg_free(apc_context *c) {
     apc_free(c, L.mptr);
     apc_free(c, L.mem);
   }
-  void *p[] = {m->pkey, m->pkey_alt, m->pidx, m->pidx_alt, m->eflag, m->epos, m->ucol,
-               m->rowstart, m->partial, m->dots, m->counter, m->state, m->total, m->ppart, m->pbar, m->pres,
+  void *p[] = {m->pkey, m->pkey_alt, m->pidx, m->pidx_alt, m->eflag, m->epos,
+               m->partial, m->dots, m->counter, m->state, m->total, m->ppart, m->pbar, m->pres,
                m->cstat, m->wdev};
   for (void *q : p) apc_free(c, q);
   if (m->host) cudaFreeHost(m->host);
@@ -2608,7 +2615,7 @@ static int cluster_levels(apc_context *c, MgHier<T> &H) {
     if (!cl_fits(A)) continue;
     APC_TRY(apc_ensure(c, &H.cl_img, (size_t)A.share * kClBlocks));
     A.img = H.cl_img;
-    cl_pack<T><<<kClBlocks, kClThreads, 0, c->s>>>(A);
+    cl_pack<T><<<dim3(kClBlocks, A.nl, kClPackParts), kClThreads, 0, c->s>>>(A);
     apc_count_launch(c);
     APC_CUDA_TRY(c, cudaGetLastError());
     H.cl = A;
@@ -2671,15 +2678,6 @@ static int mg_build(apc_context *c) {
     C.mptr = S.lv[lev + 1].mptr;
     C.mem = S.lv[lev + 1].mem;
     // ---- Galerkin product, one warp per coarse row ----
-    const int wcap = 256;
-    APC_TRY(apc_ensure(c, &m->rowstart, (size_t)nc + 1));
-    APC_TRY(apc_ensure(c, &m->ucol, (size_t)nc * wcap));
-    APC_TRY(apc_ensure(c, &H.uval, (size_t)nc * wcap));
-    galerkin_rows<<<std::max(1, std::min((nc + kGalWarps - 1) / kGalWarps, apc_sm_count(c) * 8)), 32 * kGalWarps, 0,
-                    c->s>>>(nc, C.mptr, nf, C.mem, F.w, lev == 0 ? nullptr : m->wdev + lev, F.w, F.ld, F.col,
-                            F.val, F.agg, wcap, m->rowstart, m->ucol, H.uval, c->d_err);
-    max_int<<<grid_for(nc, 256), kT, 0, c->s>>>(nc, m->rowstart, m->wdev + lev + 1);
-    apc_count_launch(c, 2);
     const int wslots = std::max(32, m->wslots[lev + 1]);
     C.w = wslots;  // until the readback below
     C.ld = (size_t)nc;
@@ -2690,8 +2688,9 @@ static int mg_build(apc_context *c) {
     APC_TRY(apc_ensure(c, &C.x2, (size_t)nc + 1));
     APC_TRY(apc_ensure(c, &C.b, (size_t)nc + 1));
     APC_TRY(apc_ensure(c, &C.r, (size_t)nc + 1));
-    rows_to_ell<T><<<grid_for(nc), kT, 0, c->s>>>(nc, m->wdev + lev + 1, wslots, C.ld, wcap, m->rowstart, m->ucol,
-                                                 H.uval, C.col, C.val, C.dinv, overflow);
+    galerkin_rows<<<std::max(1, std::min((nc + kGalWarps - 1) / kGalWarps, apc_sm_count(c) * 8)), 32 * kGalWarps, 0,
+                    c->s>>>(nc, C.mptr, nf, C.mem, F.w, lev == 0 ? nullptr : m->wdev + lev, F.w, F.ld, F.col,
+                            F.val, F.agg, wslots, C.ld, C.col, C.val, C.dinv, m->wdev + lev + 1, overflow, c->d_err);
     apc_count_launch(c);
     APC_CUDA_TRY(c, cudaGetLastError());
   }
