@@ -487,7 +487,9 @@ struct IrState {
   int max_it, max_outer, M, inner_max;
   int exact_inner;  // FP64 corrections: each cycle aims straight at the outer tolerance
   double beta;    // ||v_0|| of the current cycle
-  double scale;   // factor that normalises the newest basis vector
+  // basis vectors are kept un-normalised: v_j = scale[j] V_j.  (A pass that normalises the
+  // newest one cost a kernel of 4 us per iteration.)
+  double scale[kMaxM + 1];
   double H[(kMaxM + 1) * kMaxM];  // column j at H[j * (M + 1)]
   double cs[kMaxM], sn[kMaxM], g[kMaxM + 1], y[kMaxM];
 };
@@ -579,7 +581,8 @@ __device__ void arnoldi_step(IrState *S, const double *h1, const double *h2, dou
   __shared__ double hs[kMaxM + 2], css[kMaxM], sns[kMaxM];
   const int lane = threadIdx.x;
   const int it = S->it, M1 = S->M + 1;
-  if (lane <= it) hs[lane] = __ldcg(h1 + lane) + (h2 ? __ldcg(h2 + lane) : 0.0);
+  // the dots are with the un-normalised vectors
+  if (lane <= it) hs[lane] = (__ldcg(h1 + lane) + (h2 ? __ldcg(h2 + lane) : 0.0)) * S->scale[lane];
   if (lane < it) {
     css[lane] = S->cs[lane];
     sns[lane] = S->sn[lane];
@@ -607,7 +610,7 @@ __device__ void arnoldi_step(IrState *S, const double *h1, const double *h2, dou
     }
     S->it = it + 1;
     more = more && S->it < S->inner_max;
-    S->scale = tt > 0.0 ? 1.0 / tt : 0.0;
+    S->scale[it + 1] = tt > 0.0 ? 1.0 / tt : 0.0;
     cudaGraphSetConditional(cond, more ? 1u : 0u);
   }
   __syncwarp();
@@ -627,15 +630,18 @@ __device__ __forceinline__ T ld_krylov(const T *p) {
 // (one per lane); a row's basis values stay in registers for the update and the dots.
 //   MODE 1: w -= V h_in; h = V^T w.   MODE 2: w -= V h_in; out[0] = ||w||^2.
 // MODE 2 also finishes the Arnoldi step in its last block (h1, h2 as arnoldi_step).
-template <int MODE, class T, int NV>
+// vin: the V-cycle's input, the new vector in its type (the V-cycle runs on the un-normalised
+// vector; its result is scaled where it is used).
+template <int MODE, class T, int NV, class TV = T>
 __global__ void __launch_bounds__(kT) cgs_pass(int n, IrState *S, T *V, size_t vn,
                                                 const double *__restrict__ h_in, double *partial, unsigned *counter,
                                                 double *out, const double *h1, const double *h2,
-                                                cudaGraphConditionalHandle cond) {
+                                                cudaGraphConditionalHandle cond, TV *__restrict__ vin) {
   __shared__ double hsh[32];
   const int nv = S->it + 1;
   T *w = V + (size_t)nv * vn;
-  if ((int)threadIdx.x < nv) hsh[threadIdx.x] = h_in[threadIdx.x];
+  // <w, v_j> v_j = <w, V_j> scale_j^2 V_j
+  if ((int)threadIdx.x < nv) hsh[threadIdx.x] = h_in[threadIdx.x] * S->scale[threadIdx.x] * S->scale[threadIdx.x];
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   double acc[NV];
@@ -665,6 +671,7 @@ __global__ void __launch_bounds__(kT) cgs_pass(int n, IrState *S, T *V, size_t v
       for (int j = 0; j < NV; ++j)
         if (j < nv) wi -= hsh[j] * (double)ld_krylov(V + (size_t)j * vn + i);
       w[i] = (T)wi;
+      if (vin) vin[i] = (TV)wi;
       wi = (double)(T)wi;
       acc1 += wi * wi;
     }
@@ -701,7 +708,8 @@ __global__ void __launch_bounds__(kT, NV <= 16 ? 3 : 2) spmv_dots(int n, int ew,
                                                  T *V, size_t vn, const IrState *__restrict__ S, double *partial,
                                                  unsigned *counter, double *out) {
   const int it = S->it, nv = it + 1;
-  // the preconditioner's output (of type TZ), or the basis vector itself
+  // z = scale_it times the preconditioner's output (of type TZ), or the basis vector itself
+  const T sc = (T)S->scale[it];
   const TZ *zp = zin;
   const T *zv = V + (size_t)it * vn;
   T *zk = Z ? Z + (size_t)it * vn : nullptr;
@@ -718,11 +726,12 @@ __global__ void __launch_bounds__(kT, NV <= 16 ? 3 : 2) spmv_dots(int n, int ew,
     if (Z) {
       sacc = row_sum<T, kSpmvBatch<T>, kKrylovStream<T>>(ew, ld, i, 0, 1, col, val,
                                                           [&](int j) { return (T)zp[j]; });
-      zk[i] = (T)zp[i];
+      zk[i] = (T)zp[i] * sc;
     } else {
       sacc = row_sum<T, kSpmvBatch<T>, kKrylovStream<T>>(ew, ld, i, 0, 1, col, val,
                                                           [&](int j) { return zv[j]; });
     }
+    sacc *= sc;
     w[i] = sacc;
     const double wi = (double)sacc;
 #pragma unroll
@@ -731,19 +740,6 @@ __global__ void __launch_bounds__(kT, NV <= 16 ? 3 : 2) spmv_dots(int n, int ew,
   }
   block_partials(acc, nv, partial);
   if (last_block_arrived(counter)) finish_sums(nv, partial, counter, out);
-}
-
-// V_it *= scale (the newest basis vector), and the same into the V-cycle's input if any
-template <class T, class TV = T>
-__global__ void scale_next(int n, const IrState *__restrict__ S, T *__restrict__ V, size_t vn,
-                           TV *__restrict__ vin) {
-  const T f = (T)S->scale;
-  T *v = V + (size_t)S->it * vn;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const T u = v[i] * f;
-    v[i] = u;
-    if (vin) vin[i] = (TV)u;
-  }
 }
 
 // y = H^-1 g (upper triangular) for the cycle's iterations
@@ -762,20 +758,27 @@ __global__ void fg_finish(IrState *S) {
       ys[k] = hkk != 0.0 ? s / hkk : 0.0;
     }
     S->total_its += it;
+    S->outer += 1;
   }
   __syncthreads();
   for (int k = threadIdx.x; k < it; k += blockDim.x) S->y[k] = ys[k];
 }
 
-// d = Z y
+// x += ||D^-1 r|| Z y: the correction of the scaled system, d = Z y rounded to the inner
+// precision.  Without a preconditioner Z is the basis, whose scales go into y.
 template <class T>
-__global__ void combine(int n, const T *__restrict__ Z, size_t vn, const IrState *__restrict__ S,
-                        T *__restrict__ d) {
+__global__ void combine_apply(int n, const T *__restrict__ Z, size_t vn, const IrState *__restrict__ S, bool basis,
+                              double *__restrict__ x) {
   const int nv = S->it;
+  __shared__ double y[kMaxM];
+  if ((int)threadIdx.x < nv) y[threadIdx.x] = S->y[threadIdx.x] * (basis ? S->scale[threadIdx.x] : 1.0);
+  __syncthreads();
+  const double rn = S->rn;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     double t = 0.0;
-    for (int j = 0; j < nv; ++j) t += S->y[j] * (double)Z[(size_t)j * vn + i];
-    d[i] = (T)t;
+#pragma unroll 4
+    for (int j = 0; j < nv; ++j) t += y[j] * (double)Z[(size_t)j * vn + i];
+    x[i] += rn * (double)(T)t;
   }
 }
 
@@ -873,9 +876,9 @@ __global__ void __launch_bounds__(kT) ir_bnorm(int n, const double *__restrict__
 
 // v_0 = D^-1 r / ||D^-1 r|| rounded to the inner precision, and beta = ||v_0||; the last
 // block opens the (F)GMRES cycle (sets the inner loop's condition)
-template <class T>
+template <class T, class TV = T>
 __global__ void __launch_bounds__(kT) ir_to_inner(int n, const double *__restrict__ r, const double *__restrict__ diag,
-                                                   IrState *S, T *__restrict__ v0, double *partial,
+                                                   IrState *S, T *__restrict__ v0, TV *__restrict__ vin, double *partial,
                                                    unsigned *counter, double *tmp, cudaGraphConditionalHandle cond) {
   const double inv_s = 1.0 / S->rn;
   double nrm = 0.0;
@@ -883,6 +886,7 @@ __global__ void __launch_bounds__(kT) ir_to_inner(int n, const double *__restric
     const double d = diag[i];
     const T v = (T)((d == 0.0 ? r[i] : r[i] / d) * inv_s);
     v0[i] = v;
+    if (vin) vin[i] = (TV)v;
     nrm += (double)v * (double)v;
   }
   block_partial1(nrm, partial);
@@ -894,19 +898,10 @@ __global__ void __launch_bounds__(kT) ir_to_inner(int n, const double *__restric
   S->beta = beta;
   S->it = 0;
   S->g[0] = beta;
-  S->scale = beta > 0.0 ? 1.0 / beta : 0.0;
+  S->scale[0] = beta > 0.0 ? 1.0 / beta : 0.0;
   S->inner_max = min(S->M, max(1, S->max_it - S->total_its));
   cudaGraphSetConditional(cond, beta > 0.0 ? 1u : 0u);
 }
-
-// x += ||D^-1 r|| d: apply the correction of the scaled system
-template <class T>
-__global__ void ir_axpy(int n, IrState *S, const T *__restrict__ d, double *__restrict__ x) {
-  const double s = S->rn;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) x[i] += s * (double)d[i];
-  if (blockIdx.x == 0 && threadIdx.x == 0) S->outer += 1;
-}
-
 
 // ---- the coarse end of the V-cycle in one block: every level with <= kTail nodes,
 //      down (smooth, residual, restrict), the dense coarsest solve, and up (prolong,
@@ -2374,7 +2369,7 @@ struct MgHier {
   int cl_first = -1;
   unsigned char *cl_img = nullptr;
   // FGMRES: basis V, preconditioned vectors Z, V-cycle in/out, correction
-  T *V = nullptr, *Z = nullptr, *vin = nullptr, *vout = nullptr, *dvec = nullptr;
+  T *V = nullptr, *Z = nullptr, *vin = nullptr, *vout = nullptr;
 };
 
 struct MgWork {
@@ -2465,7 +2460,7 @@ static void free_hier(apc_context *c, MgHier<T> &H) {
     apc_free(c, L.b);
     apc_free(c, L.r);
   }
-  void *p[] = {H.coarse_inv, H.cl_img, H.V, H.Z, H.vin, H.vout, H.dvec};
+  void *p[] = {H.coarse_inv, H.cl_img, H.V, H.Z, H.vin, H.vout};
   for (void *q : p) apc_free(c, q);
 }
 
@@ -3011,10 +3006,9 @@ struct IrSolveArgs {
 // Capture one mixed solve:
 //   init; residual (sets cond_outer)
 //   while (cond_outer) {                       -- FP64 iterative refinement
-//     v0 = D^-1 r / ||D^-1 r|| (sets cond_inner); normalise v0
+//     v0 = D^-1 r / ||D^-1 r|| (sets cond_inner)
 //     while (cond_inner) {                     -- FP32 (F)GMRES cycle, right preconditioned
-//       z = V-cycle(v_it) or v_it; v_it+1 = A z; CGS; Arnoldi scalars (sets cond_inner);
-//       normalise
+//       z = V-cycle(v_it) or v_it; v_it+1 = A z; CGS; Arnoldi scalars (sets cond_inner)
 //     }
 //     y = H^-1 g; d = Z y; x += ||D^-1 r|| d; residual (sets cond_outer)
 //   }
@@ -3062,11 +3056,11 @@ static int capture_solve(apc_context *c, const IrSolveArgs<T> &a) {
         ok(cudaStreamBeginCaptureToGraph(s1, body_out, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal))) {
       cap1 = true;
       if (ok(cudaGraphConditionalHandleCreate(&cond_in, body_out, 0, 0))) {
-        ir_to_inner<T><<<G, kT, 0, s1>>>(n, a.r, a.val, m->state, H.V, m->partial, m->counter, tmp, cond_in);
         if (v32)
-          scale_next<T, float><<<Gs, kT, 0, s1>>>(n, m->state, H.V, vn, vin32);
+          ir_to_inner<T, float><<<G, kT, 0, s1>>>(n, a.r, a.val, m->state, H.V, vin32, m->partial, m->counter, tmp,
+                                                  cond_in);
         else
-          scale_next<T><<<Gs, kT, 0, s1>>>(n, m->state, H.V, vn, vin);
+          ir_to_inner<T><<<G, kT, 0, s1>>>(n, a.r, a.val, m->state, H.V, vin, m->partial, m->counter, tmp, cond_in);
         if (ok(cudaGetLastError()) && ok(add_while(s1, cond_in, &body_in)) &&
             ok(cudaStreamBeginCaptureToGraph(s2, body_in, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal))) {
           cap2 = true;
@@ -3086,24 +3080,26 @@ static int capture_solve(apc_context *c, const IrSolveArgs<T> &a) {
             else
               spmv_dots<T, T, NV><<<G, kT, 0, s2>>>(n, a.w, a.ld, a.col, a.valf, a.mg ? H.vout : nullptr, Z, H.V,
                                                     vn, m->state, m->partial, m->counter, h1);
+            auto cgs2 = [&](const double *h, const double *hb) {
+              if (v32)
+                cgs_pass<2, T, NV, float><<<G, kT, 0, s2>>>(n, m->state, H.V, vn, h, m->partial, m->counter, nr, h1, hb,
+                                                            cond_in, vin32);
+              else
+                cgs_pass<2, T, NV><<<G, kT, 0, s2>>>(n, m->state, H.V, vn, h, m->partial, m->counter, nr, h1, hb,
+                                                     cond_in, vin);
+            };
             if (reorth) {
               cgs_pass<1, T, NV><<<G, kT, 0, s2>>>(n, m->state, H.V, vn, h1, m->partial, m->counter, h2, nullptr,
-                                                   nullptr, cond_in);
-              cgs_pass<2, T, NV><<<G, kT, 0, s2>>>(n, m->state, H.V, vn, h2, m->partial, m->counter, nr, h1, h2,
-                                                   cond_in);
+                                                   nullptr, cond_in, (T *)nullptr);
+              cgs2(h2, h2);
             } else {
-              cgs_pass<2, T, NV><<<G, kT, 0, s2>>>(n, m->state, H.V, vn, h1, m->partial, m->counter, nr, h1,
-                                                   nullptr, cond_in);
+              cgs2(h1, nullptr);
             }
           };
           if (a.M <= 16)
             krylov(std::integral_constant<int, 16>{});
           else
             krylov(std::integral_constant<int, 32>{});
-          if (v32)
-            scale_next<T, float><<<Gs, kT, 0, s2>>>(n, m->state, H.V, vn, vin32);
-          else
-            scale_next<T><<<Gs, kT, 0, s2>>>(n, m->state, H.V, vn, vin);
           ok(cudaGetLastError());
         }
         if (cap2) {
@@ -3111,8 +3107,7 @@ static int capture_solve(apc_context *c, const IrSolveArgs<T> &a) {
           ok(cudaStreamEndCapture(s2, &g2));
         }
         fg_finish<<<1, 32, 0, s1>>>(m->state);
-        combine<T><<<Gs, kT, 0, s1>>>(n, a.mg ? H.Z : H.V, vn, m->state, H.dvec);
-        ir_axpy<T><<<Gs, kT, 0, s1>>>(n, m->state, H.dvec, a.x);
+        combine_apply<T><<<Gs, kT, 0, s1>>>(n, a.mg ? H.Z : H.V, vn, m->state, !a.mg, a.x);
         ir_residual<<<G, kT, 0, s1>>>(n, a.w, a.ld, a.col, a.val, a.b, a.x, a.r, m->state, m->partial, m->counter,
                                       tmp, cond_out);
         ok(cudaGetLastError());
@@ -3512,7 +3507,6 @@ static int ir_solve(apc_context *c, int which, bool use_mg, const double *val, c
     if (use_mg) APC_TRY(check_coarse(c));
     return outcome(*m->pres_host);
   }
-  APC_TRY(apc_ensure(c, &H.dvec, vn));
   APC_TRY(apc_ensure(c, &m->partial, (size_t)kRedBlocks * 34));
   APC_TRY(apc_ensure(c, &m->dots, (size_t)4 * 34));
   if (!m->counter) {
@@ -3542,8 +3536,8 @@ static int ir_solve(apc_context *c, int which, bool use_mg, const double *val, c
   *reason = S.reason;
   *refinements = S.outer;
   *levels = use_mg ? nlev : 0;
-  const int per_it = (int)m->vcycle_nodes[which] + 3 + (cfg.mg_reorth != 0 ? 1 : 0);
-  apc_count_launch(c, 3 + 6 * S.outer + per_it * S.total_its);
+  const int per_it = (int)m->vcycle_nodes[which] + 2 + (cfg.mg_reorth != 0 ? 1 : 0);
+  apc_count_launch(c, 3 + 4 * S.outer + per_it * S.total_its);
   if (use_mg) {
     c->prof.mg_solve_ms += ms;
     c->prof.mg_iterations += S.total_its;
