@@ -333,18 +333,6 @@ __global__ void prolong_add(int n, const int *__restrict__ agg, const V *__restr
 // than the extra pass (measured at 128^3 on levels of 262k and 33k rows)
 constexpr int kSplitProlongRows = 1 << 14;
 
-// b_c[I] = sum of r over the members of I, in member order
-template <class V>
-__global__ void restrict_sum(int nc, const int *__restrict__ mptr, int nf, const int *__restrict__ mem,
-                             const V *__restrict__ r, V *__restrict__ bc) {
-  for (int I = blockIdx.x * blockDim.x + threadIdx.x; I < nc; I += gridDim.x * blockDim.x) {
-    const int a = mptr[I], e = (I + 1 < nc) ? mptr[I + 1] : nf;
-    V s = V(0);
-    for (int k = a; k < e; ++k) s += r[mem[k]];
-    bc[I] = s;
-  }
-}
-
 // sum over this lane's slots k = sub, sub + g, ... < w of val[k][i] * xj(col[k][i]), added in
 // slot order.  The loads of up to kRowBatch slots are issued before the first product, so
 // a short row costs two dependent round trips to L2 (columns, then the gathered values)
@@ -387,7 +375,7 @@ __device__ __forceinline__ V row_sum(int w, size_t ld, long long i, int sub, int
 // slots sub, sub + G, ... (the slot-major ELL keeps each slot's rows adjacent, so a warp
 // still reads whole sectors) and add their sums by a fixed shuffle tree.  Levels with few
 // rows get more lanes per row (vcycle), so that each lane's loads fit one batch.
-enum RowOp { kOpFirst2, kOpSweep, kOpResidual, kOpProlongSweep };
+enum RowOp { kOpFirst2, kOpSweep, kOpProlongSweep };
 
 template <int G, int OP, class V>
 __global__ void __launch_bounds__(kT) row_op(int n, int w, size_t ld, const int *__restrict__ col,
@@ -419,8 +407,6 @@ __global__ void __launch_bounds__(kT) row_op(int n, int w, size_t ld, const int 
         out[i] = x1 + omega * dinv[i] * (b[i] - sacc);
       } else if (OP == kOpSweep) {
         out[i] = xin[i] + omega * dinv[i] * (b[i] - sacc);
-      } else if (OP == kOpResidual) {
-        out[i] = b[i] - sacc;
       } else {
         const V y = xin[i] + alpha * xc[agg[i]];
         out[i] = y + omega * dinv[i] * (b[i] - sacc);
@@ -431,8 +417,9 @@ __global__ void __launch_bounds__(kT) row_op(int n, int w, size_t ld, const int 
 
 // b_c[I] = sum over the members q of I (in member order) of r_q = b_q - (A x)_q: the
 // residual and the restriction in one pass, 8 lanes per coarse row, one member row each
-// (more members go round in turns).  For the coarse levels, whose rows are in code order,
-// so that a coarse row's members are adjacent rows and a warp's loads stay coalesced.
+// (more members go round in turns).  A coarse row's members are adjacent rows on every level:
+// the coarse levels are in code order, and the leaves of an octree node are numbered one after
+// the other; so a warp's loads stay coalesced.
 template <class V>
 __global__ void __launch_bounds__(kT) residual_restrict(int nc, const int *__restrict__ mptr,
                                                         const int *__restrict__ mem, int nf, int w, size_t ld,
@@ -2902,10 +2889,6 @@ static void vcycle(apc_context *c, cudaStream_t s, int l, const T *b, T *x) {
       row_op<GG, kOpSweep, T><<<G, kT, 0, s>>>(n, L.w, L.ld, L.col, L.val, L.dinv, b, xin, L.agg, C.x, alpha,        \
                                            omega, out);                                                          \
       break;                                                                                                      \
-    case kOpResidual:                                                                                             \
-      row_op<GG, kOpResidual, T><<<G, kT, 0, s>>>(n, L.w, L.ld, L.col, L.val, L.dinv, b, xin, L.agg, C.x, alpha,     \
-                                              omega, out);                                                       \
-      break;                                                                                                      \
     default:                                                                                                      \
       row_op<GG, kOpProlongSweep, T><<<G, kT, 0, s>>>(n, L.w, L.ld, L.col, L.val, L.dinv, b, xin, L.agg, C.x, alpha, \
                                                   omega, out);                                                   \
@@ -2941,16 +2924,9 @@ static void vcycle(apc_context *c, cudaStream_t s, int l, const T *b, T *x) {
     nxt = x;
     apc_count_launch(c);
   }
-  if (l > 0) {
-    // coarse levels are in code order: residual and restriction in one pass
-    residual_restrict<T><<<grid_for((long long)C.n * 8), kT, 0, s>>>(C.n, C.mptr, C.mem, n, L.w, L.ld, L.col,
-                                                                     L.val, b, cur, C.b);
-    apc_count_launch(c);
-  } else {
-    op(kOpResidual, cur, L.r);
-    restrict_sum<T><<<grid_for(C.n), kT, 0, s>>>(C.n, C.mptr, n, C.mem, L.r, C.b);
-    apc_count_launch(c);
-  }
+  residual_restrict<T><<<grid_for((long long)C.n * 8), kT, 0, s>>>(C.n, C.mptr, C.mem, n, L.w, L.ld, L.col, L.val, b,
+                                                                   cur, C.b);
+  apc_count_launch(c);
   vcycle<T>(c, s, l + 1, C.b, C.x);
   if (n > kSplitProlongRows) {
     prolong_add<T><<<grid_for(n), kT, 0, s>>>(n, L.agg, C.x, alpha, cur);
