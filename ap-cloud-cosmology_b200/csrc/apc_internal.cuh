@@ -312,6 +312,35 @@ __device__ __forceinline__ bool grid_sync(GridBar *bar, unsigned nblocks, unsign
   return s_go != 0;
 }
 
+// sum over the block of v, in every thread; sm: a word per warp
+template <int THREADS>
+__device__ __forceinline__ int block_sum_int(int v, int *sm) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  v = __reduce_add_sync(0xffffffffu, v);
+  __syncthreads();
+  if (lane == 0) sm[warp] = v;
+  __syncthreads();
+  return __reduce_add_sync(0xffffffffu, lane < THREADS / 32 ? sm[lane] : 0);
+}
+
+// exclusive sum over the block's threads; *total is the block's sum
+template <int THREADS>
+__device__ __forceinline__ int block_scan_int(int v, int *sm, int *total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int incl = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  __syncthreads();
+  if (lane == 31) sm[warp] = incl;
+  __syncthreads();
+  const int w = lane < THREADS / 32 ? sm[lane] : 0;
+  *total = __reduce_add_sync(0xffffffffu, w);
+  return incl - v + __reduce_add_sync(0xffffffffu, lane < warp ? w : 0);
+}
+
 // ------------------------------------------------------- thread-block clusters
 
 __device__ __forceinline__ void cluster_barrier() {

@@ -367,7 +367,7 @@ int apc_create(const apc_config *cfg, apc_context **out) {
   for (auto &e : c->sev)
     if (cudaEventCreate(&e) != cudaSuccess) return fail(APC_ERR_CUDA);
   if (cudaEventCreateWithFlags(&c->wait_ev, cudaEventDisableTiming) != cudaSuccess) return fail(APC_ERR_CUDA);
-  if (cudaMallocHost((void **)&c->h_pinned, 64 * sizeof(int)) != cudaSuccess) return fail(APC_ERR_CUDA);
+  if (cudaMallocHost((void **)&c->h_pinned, 128 * sizeof(int)) != cudaSuccess) return fail(APC_ERR_CUDA);
   const size_t n = (size_t)c->n;
   double **dbl[] = {&c->px, &c->py, &c->pz, &c->pvx, &c->pvy, &c->pvz, &c->pax, &c->pay, &c->paz,
                     &c->qx, &c->qy, &c->qz, &c->qvx, &c->qvy, &c->qvz};

@@ -57,23 +57,96 @@ __global__ void parent_codes(int n, const uint64_t *__restrict__ code, uint64_t 
   }
 }
 
-__global__ void change_flags_u64(int n, const uint64_t *__restrict__ key, int *__restrict__ flag) {
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
-    flag[k] = (k == 0 || key[k] != key[k - 1]) ? 1 : 0;
-}
+// The aggregation of every level in one cooperative kernel: level l + 1's nodes are the distinct
+// parents (code >> 3) of level l's nodes, taken in code order, down to kCoarsest nodes or until
+// nothing coarsens.  Level 0's parent codes come sorted (key, idx); the coarser levels are in
+// code order themselves.  Per level two grid barriers: the bits of the nodes whose parent
+// differs from the one before, then the numbering (a node's aggregate is the number of bits up
+// to it) and the member lists.  (Launches and a host read of each level's size took 25 us a
+// level.)
+constexpr int kStThreads = 512;
+struct StLevel {
+  int *agg;                   // node -> coarser node
+  uint64_t *ccode;            // of the coarser level: codes, members
+  int *mptr, *mem;
+};
+struct StArgs {
+  int n0, max_levels;
+  const uint64_t *key;
+  const uint32_t *idx;
+  uint32_t *words;
+  StLevel L[kMaxLevels];
+  int *sizes;                 // [level], sizes[kMaxLevels] the number of levels
+  GridBar *bar;
+  int *err;
+};
 
-// after the scan: aggregate map, coarse codes, member CSR of the coarse nodes
-__global__ void aggregate_map(int n, const uint64_t *__restrict__ key, const uint32_t *__restrict__ idx,
-                              const int *__restrict__ flag, const int *__restrict__ pos, int *__restrict__ agg,
-                              uint64_t *__restrict__ ccode, int *__restrict__ mptr, int *__restrict__ mem) {
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-    const int I = pos[k] + flag[k] - 1;  // inclusive count - 1
-    agg[idx[k]] = I;
-    mem[k] = (int)idx[k];
-    if (flag[k]) {
-      ccode[I] = key[k];
-      mptr[I] = k;
+__global__ void __launch_bounds__(kStThreads) mg_aggregate(const __grid_constant__ StArgs A) {
+  __shared__ int sm[kStThreads / 32], s_base[kStThreads];
+  __shared__ uint32_t s_word[kStThreads];
+  const int t = threadIdx.x, lane = t & 31, G = gridDim.x, b = blockIdx.x;
+  const int gwarps = G * (kStThreads / 32), gwarp = b * (kStThreads / 32) + (t >> 5);
+  unsigned epoch = 0;
+  int nf = A.n0, lev = 0;
+  while (nf > kCoarsest && lev + 1 < A.max_levels) {
+    const StLevel L = A.L[lev];
+    const uint64_t *code = lev > 0 ? A.L[lev - 1].ccode : nullptr;
+    auto parent = [&](int k) {
+      if (lev == 0) return A.key[k];
+      const uint64_t c = code[k];
+      return c > 1ull ? c >> 3 : (uint64_t)1;
+    };
+    const int nwords = (nf + 31) / 32;
+    for (int w = gwarp; w < nwords; w += gwarps) {
+      const int k = w * 32 + lane;
+      const bool f = k < nf && (k == 0 || parent(k) != parent(k - 1));
+      const unsigned bal = __ballot_sync(0xffffffffu, f);
+      if (lane == 0) A.words[w] = bal;
     }
+    if (!grid_sync(A.bar, G, epoch, A.err)) return;
+    // the block's share of the words, the bits before it and in all
+    const int per = (nwords + G - 1) / G, w0 = min(nwords, b * per), w1 = min(nwords, w0 + per);
+    int lo = 0, all = 0;
+    for (int w = t; w < nwords; w += kStThreads) {
+      const int p = __popc(__ldcg(A.words + w));
+      all += p;
+      if (w < w0) lo += p;
+    }
+    int before = block_sum_int<kStThreads>(lo, sm);
+    const int nc = block_sum_int<kStThreads>(all, sm);
+    if (nc >= nf) break;  // no coarsening left; the same in every block
+    for (int wb = w0; wb < w1; wb += kStThreads) {
+      const uint32_t word = wb + t < w1 ? __ldcg(A.words + wb + t) : 0u;
+      int sum;
+      const int ex = block_scan_int<kStThreads>(__popc(word), sm, &sum);
+      s_base[t] = before + ex;
+      s_word[t] = word;
+      __syncthreads();
+      const int items = min(kStThreads, w1 - wb) * 32;
+      for (int i = t; i < items; i += kStThreads) {
+        const int k = wb * 32 + i;
+        if (k >= nf) break;
+        const uint32_t wd = s_word[i >> 5];
+        const int I = s_base[i >> 5] + __popc(wd & ((2u << (i & 31)) - 1u)) - 1;
+        const int m = lev == 0 ? (int)A.idx[k] : k;
+        L.agg[m] = I;
+        L.mem[k] = m;
+        if ((wd >> (i & 31)) & 1u) {
+          L.ccode[I] = parent(k);
+          L.mptr[I] = k;
+        }
+      }
+      before += sum;
+      __syncthreads();
+    }
+    ++lev;
+    nf = nc;
+    if (b == 0 && t == 0) A.sizes[lev] = nc;
+    if (!grid_sync(A.bar, G, epoch, A.err)) return;
+  }
+  if (b == 0 && t == 0) {
+    A.sizes[0] = A.n0;
+    A.sizes[kMaxLevels] = lev + 1;
   }
 }
 
@@ -2366,13 +2439,13 @@ struct MgWork {
   // hierarchy temporaries: parent-code sort, flags, coarse rows before the ELL transpose
   uint64_t *pkey = nullptr, *pkey_alt = nullptr;
   uint32_t *pidx = nullptr, *pidx_alt = nullptr;
-  int *eflag = nullptr, *epos = nullptr;
+  uint32_t *words = nullptr;  // one bit per node of a level
+  int *sizes = nullptr;       // level sizes, grid barrier and error flag of mg_aggregate
   size_t vn = 0;
   double *partial = nullptr, *dots = nullptr;
   unsigned *counter = nullptr;
   IrState *state = nullptr;
   void *host = nullptr;  // pinned readback of the state
-  int *total = nullptr;
   // each mixed solve of the step as one graph, captured on c->s with the loop bodies on
   // two side streams
   cudaStream_t cap[2] = {nullptr, nullptr};
@@ -2462,8 +2535,7 @@ void apc_mg_free(apc_context *c) {
     apc_free(c, L.mptr);
     apc_free(c, L.mem);
   }
-  void *p[] = {m->pkey, m->pkey_alt, m->pidx, m->pidx_alt, m->eflag, m->epos,
-               m->partial, m->dots, m->counter, m->state, m->total, m->ppart, m->pbar, m->pres,
+  void *p[] = {m->pkey, m->pkey_alt, m->pidx, m->pidx_alt, m->words, m->sizes, m->partial, m->dots, m->counter, m->state, m->ppart, m->pbar, m->pres,
                m->cstat, m->wdev};
   for (void *q : p) apc_free(c, q);
   if (m->host) cudaFreeHost(m->host);
@@ -2482,14 +2554,6 @@ void apc_mg_free(apc_context *c) {
   c->mg = nullptr;
 }
 
-static int read_int(apc_context *c, const int *dev, int *host) {
-  // through the context's pinned word: a pageable destination would be staged
-  APC_CUDA_TRY(c, cudaMemcpyAsync(c->h_pinned + 10, dev, sizeof(int), cudaMemcpyDeviceToHost, c->s));
-  APC_CUDA_TRY(c, apc_stream_wait(c));
-  *host = c->h_pinned[10];
-  return APC_OK;
-}
-
 // Build the hierarchy over the current Jacobi-scaled potential operator in precision T
 // (c->a2f or c->a2d) and the cell codes.
 template <class T>
@@ -2503,59 +2567,68 @@ const double *scaled_potential<double>(const apc_context *c) {
   return c->a2d;
 }
 
-// The aggregation on c->s: level l + 1's nodes are the distinct parents (code >> 3) of
-// level l's, in code order, down to kCoarsest nodes or until nothing coarsens.
+// The aggregation on c->s (mg_aggregate), with one host read of the level sizes.
 static int mg_structure(apc_context *c) {
   MgWork *m = mg(c);
   MgStruct &S = m->st;
   S.gen = 0;
   S.on_side = false;
-  S.lv[0].n = c->nc + c->nv;
+  const int n0 = c->nc + c->nv;
+  S.lv[0].n = n0;
   S.lv[0].code = c->ccode;
-  if (!m->total) APC_TRY(apc_alloc(c, (void **)&m->total, 4 * sizeof(int)));
-  int lev = 0;
-  while (S.lv[lev].n > kCoarsest && lev + 1 < kMaxLevels) {
-    MgStructLevel &F = S.lv[lev];
-    MgStructLevel &C = S.lv[lev + 1];
-    const int nf = F.n;
-    APC_TRY(apc_ensure(c, &m->pkey, (size_t)nf));
-    APC_TRY(apc_ensure(c, &m->pkey_alt, (size_t)nf));
-    APC_TRY(apc_ensure(c, &m->pidx, (size_t)nf));
-    APC_TRY(apc_ensure(c, &m->pidx_alt, (size_t)nf));
-    APC_TRY(apc_ensure(c, &F.agg, (size_t)nf));
-    parent_codes<<<grid_for(nf), kT, 0, c->s>>>(nf, F.code, m->pkey, m->pidx);
-    apc_count_launch(c);
-    bool alt = false;
-    // level 0 is in the reference's cell order; coarser levels are already sorted by
-    // code, and so are their parents' codes
-    if (lev == 0) {
-      // parent codes of cells at level <= D have at most 3 D - 2 significant bits; the
-      // deepest cell level is one below the deepest top-down opened level
-      const int deepest = c->levels_hint + 2;
-      const int bits = std::min(64, 3 * deepest + 1);
-      APC_TRY(apc_radix_sort_u64(c, m->pkey, m->pidx, m->pkey_alt, m->pidx_alt, nf, 0, bits, &alt));
-    }
-    uint64_t *pk = alt ? m->pkey_alt : m->pkey;
-    uint32_t *pi = alt ? m->pidx_alt : m->pidx;
-    APC_TRY(apc_ensure(c, &m->eflag, (size_t)nf + 1));
-    APC_TRY(apc_ensure(c, &m->epos, (size_t)nf + 1));
-    change_flags_u64<<<grid_for(nf), kT, 0, c->s>>>(nf, pk, m->eflag);
-    apc_count_launch(c);
-    APC_TRY(apc_exclusive_scan(c, m->eflag, m->epos, nf, m->total));
-    int nc = 0;
-    APC_TRY(read_int(c, m->total, &nc));
-    if (nc >= nf) break;  // no coarsening left
-    C.n = nc;
-    APC_TRY(apc_ensure(c, &C.own_code, (size_t)nc + 1));
-    APC_TRY(apc_ensure(c, &C.mptr, (size_t)nc + 1));
-    APC_TRY(apc_ensure(c, &C.mem, (size_t)nf + 1));
+  // level 1's nodes are opened octree nodes, and every further level is at most as large; the
+  // cells lie at levels 1 .. levels_hint, so that many levels of parents
+  const int bound = c->n_open, nlev = std::min(kMaxLevels, c->levels_hint + 2);
+  APC_TRY(apc_ensure(c, &m->pkey, (size_t)n0));
+  APC_TRY(apc_ensure(c, &m->pkey_alt, (size_t)n0));
+  APC_TRY(apc_ensure(c, &m->pidx, (size_t)n0));
+  APC_TRY(apc_ensure(c, &m->pidx_alt, (size_t)n0));
+  APC_TRY(apc_ensure(c, &m->words, (size_t)n0 / 32 + 1));
+  if (!m->sizes) APC_TRY(apc_alloc(c, (void **)&m->sizes, (kMaxLevels + 1) * sizeof(int) + sizeof(GridBar) + sizeof(int)));
+  StArgs A{};
+  A.n0 = n0;
+  A.max_levels = nlev;
+  A.sizes = m->sizes;
+  A.bar = (GridBar *)(m->sizes + kMaxLevels + 1);
+  A.err = (int *)(A.bar + 1);
+  A.words = m->words;
+  for (int l = 0; l + 1 < nlev; ++l) {
+    MgStructLevel &F = S.lv[l];
+    MgStructLevel &C = S.lv[l + 1];
+    const size_t nf = (size_t)(l == 0 ? n0 : bound);
+    APC_TRY(apc_ensure(c, &F.agg, nf));
+    APC_TRY(apc_ensure(c, &C.own_code, (size_t)bound + 1));
+    APC_TRY(apc_ensure(c, &C.mptr, (size_t)bound + 1));
+    APC_TRY(apc_ensure(c, &C.mem, nf + 1));
     C.code = C.own_code;
-    aggregate_map<<<grid_for(nf), kT, 0, c->s>>>(nf, pk, pi, m->eflag, m->epos, F.agg, C.own_code, C.mptr, C.mem);
-    apc_count_launch(c);
-    APC_CUDA_TRY(c, cudaGetLastError());
-    ++lev;
+    A.L[l] = {F.agg, C.own_code, C.mptr, C.mem};
   }
-  S.nlev = lev + 1;
+  APC_CUDA_TRY(c, cudaMemsetAsync(m->sizes, 0, (kMaxLevels + 1) * sizeof(int) + sizeof(GridBar) + sizeof(int), c->s));
+  // level 0 is in the reference's cell order; the parents of cells at level <= levels_hint
+  // have at most 3 levels_hint - 2 significant bits
+  parent_codes<<<grid_for(n0), kT, 0, c->s>>>(n0, c->ccode, m->pkey, m->pidx);
+  apc_count_launch(c);
+  bool alt = false;
+  APC_TRY(apc_radix_sort_u64(c, m->pkey, m->pidx, m->pkey_alt, m->pidx_alt, n0, 0,
+                             std::min(64, std::max(1, 3 * c->levels_hint - 2)), &alt));
+  A.key = alt ? m->pkey_alt : m->pkey;
+  A.idx = alt ? m->pidx_alt : m->pidx;
+  const int blocks = std::max(1, std::min(apc_sm_count(c), n0 / 1024));
+  void *args[] = {&A};
+  APC_CUDA_TRY(c, cudaLaunchCooperativeKernel((const void *)mg_aggregate, dim3(blocks), dim3(kStThreads), args, 0,
+                                              c->s));
+  apc_count_launch(c);
+  int *host = c->h_pinned + 64;
+  static_assert(sizeof(GridBar) == 4 * sizeof(int) && kMaxLevels + 6 <= 64, "the pinned words from 64 on");
+  APC_CUDA_TRY(c, cudaMemcpyAsync(host, m->sizes, (kMaxLevels + 1 + 4 + 1) * sizeof(int), cudaMemcpyDeviceToHost,
+                                  c->s));
+  APC_CUDA_TRY(c, apc_stream_wait(c));
+  if (host[kMaxLevels + 5] != 0) {
+    c->err = "aggregation kernel grid barrier timed out";
+    return APC_ERR_TIMEOUT;
+  }
+  S.nlev = host[kMaxLevels];
+  for (int l = 1; l < S.nlev; ++l) S.lv[l].n = host[l];
   S.gen = c->select_gen;
   return APC_OK;
 }

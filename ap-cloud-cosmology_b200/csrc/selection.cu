@@ -160,33 +160,6 @@ __device__ __forceinline__ int warp_lower_digit(const uint64_t *keys, int lo, in
   return lo;
 }
 
-// sum over the block of v, in every thread
-__device__ __forceinline__ int tree_block_sum(int v, int *sm) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  v = __reduce_add_sync(0xffffffffu, v);
-  __syncthreads();
-  if (lane == 0) sm[warp] = v;
-  __syncthreads();
-  return __reduce_add_sync(0xffffffffu, lane < kTreeWarps ? sm[lane] : 0);
-}
-
-// exclusive sum over the block's threads; *total is the block's sum
-__device__ __forceinline__ int tree_block_scan(int v, int *sm, int *total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int incl = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int t = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += t;
-  }
-  __syncthreads();
-  if (lane == 31) sm[warp] = incl;
-  __syncthreads();
-  const int w = lane < kTreeWarps ? sm[lane] : 0;
-  *total = __reduce_add_sync(0xffffffffu, w);
-  return incl - v + __reduce_add_sync(0xffffffffu, lane < warp ? w : 0);
-}
-
 // One sweep ln's requests by one (opened node, child) pair: the child, a node of level ln,
 // requests the opening of the coarse cells that break 2:1 across its six faces.
 __device__ __forceinline__ void request_openings(const TreeArgs &A, int ln, int o, int ch, int tab) {
@@ -256,8 +229,8 @@ __global__ void __launch_bounds__(kTreeThreads) select_tree(const __grid_constan
       all += p;
       if (w < w0) lo += p;
     }
-    before = tree_block_sum(lo, sm);
-    total = tree_block_sum(all, sm);
+    before = block_sum_int<kTreeThreads>(lo, sm);
+    total = block_sum_int<kTreeThreads>(all, sm);
   };
   auto finish = [&](int maxlev, int n_open_td, int n_open) {
     if (b == 0 && t == 0) {
@@ -345,7 +318,7 @@ __global__ void __launch_bounds__(kTreeThreads) select_tree(const __grid_constan
     for (int wb = w0; wb < w1; wb += kTreeThreads) {
       const uint32_t word = wb + t < w1 ? __ldcg(words + wb + t) : 0u;
       int sum;
-      const int ex = tree_block_scan(__popc(word), sm, &sum);
+      const int ex = block_scan_int<kTreeThreads>(__popc(word), sm, &sum);
       s_base[t] = before + ex;
       s_word[t] = word;
       __syncthreads();
@@ -451,7 +424,7 @@ __global__ void __launch_bounds__(kTreeThreads) select_tree(const __grid_constan
   for (int wb = w0; wb < w1; wb += kTreeThreads) {
     const uint32_t word = wb + t < w1 ? __ldcg(A.leaf + wb + t) : 0u;
     int sum;
-    const int ex = tree_block_scan(__popc(word), sm, &sum);
+    const int ex = block_scan_int<kTreeThreads>(__popc(word), sm, &sum);
     if (wb + t < w1) {
       A.leaf_base[wb + t] = before + ex;
       if (wb + t == split >> 5) A.out->nc = before + ex + __popc(word & ((1u << (split & 31)) - 1u));
