@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 
 #include "apc_internal.cuh"
 
@@ -41,6 +42,25 @@ __global__ void morton_keys(const double *__restrict__ x, const double *__restri
     if (hz) lz = mz; else rz = mz;
   }
   keys[i] = key;
+  perm[i] = (uint32_t)i;
+}
+
+// The same keys for a box [0, 2^m): every midpoint of the bisection is a multiple of 2^(m - depth)
+// and exact, so a coordinate's bits are floor(x 2^(depth - m)), an exact scaling, limited to the
+// grid as the bisection leaves points outside the box in its end cells (and a NaN in the first).
+// Another lower bound takes the bisection: x - lo can round across a midpoint.  2.1M particles:
+// 60 us by bisection (issue-bound: 63 rounds of FP64 compare and halve), memory-bound here.
+__global__ void morton_keys_scaled(const double *__restrict__ x, const double *__restrict__ y,
+                                   const double *__restrict__ z, int n, int depth, double sx, double sy, double sz,
+                                   uint64_t *__restrict__ keys, uint32_t *__restrict__ perm, int *err) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double px = x[i], py = y[i], pz = z[i];
+  if (!(isfinite(px) && isfinite(py) && isfinite(pz))) atomicOr(err, DERR_NOT_FINITE);
+  const double top = (double)((1 << depth) - 1);
+  const uint64_t ix = (uint64_t)fmin(fmax(px * sx, 0.0), top), iy = (uint64_t)fmin(fmax(py * sy, 0.0), top),
+                 iz = (uint64_t)fmin(fmax(pz * sz, 0.0), top);
+  keys[i] = (spread3(ix) << 2) | (spread3(iy) << 1) | spread3(iz);
   perm[i] = (uint32_t)i;
 }
 
@@ -89,7 +109,20 @@ int apc_octree_build(apc_context *c) {
   const int n = c->n;
   if (n <= 0) return APC_OK;
   const int T = 256, G = (n + T - 1) / T;
-  morton_keys<<<G, T, 0, c->s>>>(c->px, c->py, c->pz, n, c->cfg.depth, c->cfg.box[0], c->cfg.box[1],
+  // box [0, 2^m) in every dimension, scales of ordinary size
+  double scale[3];
+  bool scaled = true;
+  for (int d = 0; d < 3; ++d) {
+    int e = 0;
+    const double lo = c->cfg.box[2 * d], hi = c->cfg.box[2 * d + 1];
+    scaled = scaled && lo == 0.0 && std::frexp(hi, &e) == 0.5 && e > -900 && e < 900;
+    scale[d] = scaled ? std::ldexp(1.0, c->cfg.depth + 1 - e) : 0.0;
+  }
+  if (scaled)
+    morton_keys_scaled<<<G, T, 0, c->s>>>(c->px, c->py, c->pz, n, c->cfg.depth, scale[0], scale[1], scale[2], c->keys,
+                                          c->perm, c->d_err);
+  else
+    morton_keys<<<G, T, 0, c->s>>>(c->px, c->py, c->pz, n, c->cfg.depth, c->cfg.box[0], c->cfg.box[1],
                                  c->cfg.box[2], c->cfg.box[3], c->cfg.box[4], c->cfg.box[5], c->keys,
                                  c->perm, c->d_err);
   apc_count_launch(c);
