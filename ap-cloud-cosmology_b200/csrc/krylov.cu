@@ -10,8 +10,9 @@
 //   - convergence on the preconditioned residual estimate against
 //     max(rtol ||D^-1 b||, atol), divergence at dtol * ||D^-1 b||, DIVERGED_ITS at max_it.
 //
-// Design (B200): one persistent cooperative kernel per solve.  Every block owns a
-// strided set of rows.
+// Design (B200): one persistent kernel per solve: thread-block clusters that exchange their
+// sums through distributed shared memory (gmres_cluster) up to the rows that fit, a
+// cooperative launch over all SMs (gmres_kernel) above.  Every block owns a set of rows.
 //   - Per Arnoldi step, one pass fuses SpMV + Jacobi + all dot products with the
 //     basis, and a second pass fuses the Gram-Schmidt update + norm.  That is two grid
 //     barriers per iteration.  With re-orthogonalisation (CGS2) it is three.

@@ -11,12 +11,13 @@
 //     conditional WHILE nodes of one graph; kernels hold every scalar (Hessenberg
 //     column, Givens rotations, stopping tests) in device memory and set the loop
 //     conditions, so a solve costs the host one launch and one readback.
+//     Small systems run whole on one thread-block cluster instead (solve_cluster).
 //   * Aggregation by the octree.  A node of the next coarser level is the parent cell
 //     (location code >> 3); its aggregate is the set of its children present on the
 //     finer level.  Coarse node order is sorted location code, so Morton order.
 //   * Galerkin coarse operators A_c = P^T A P, P piecewise constant, one warp per
-//     coarse row: the members' (J, a_ij) contributions are sorted in shared memory by a
-//     bitonic network and summed in sorted order, so the hierarchy is deterministic.
+//     coarse row: the members' (J, a_ij) contributions are merged in a per-warp hash table
+//     in contribution order and sorted by column, so the hierarchy is deterministic.
 //     Rows sum to zero except the Dirichlet pin's aggregate, so the constant mode is
 //     reproduced exactly on every level.
 //   * Damped Jacobi smoothing on ELL operators, over-scaled coarse corrections; the
