@@ -648,6 +648,10 @@ class ReferenceRun:
         self.r.close()
 
 
+REF_SO = os.path.join(ROOT, "oracle", "_ref", "libapcref.so")
+REF_MISSING = "oracle/_ref/libapcref.so not built (make -C oracle ref)"
+
+
 def ref_sample_text(cfg, threads: int, k: int, first_step: int, its) -> str:
     return (f"{k} whole 128^3 step(s) of the reference code (oracle/_ref), steps {first_step}-{first_step + k - 1} "
             f"of the run from its initial state: select, GFD assembly, density and potential GMRES({cfg.restart}) "
@@ -659,6 +663,8 @@ def ref_sample_text(cfg, threads: int, k: int, first_step: int, its) -> str:
 
 def cpu_baseline(cfg, args) -> dict:
     """The reference on the host, bounded: the first whole step of the run."""
+    if not os.path.exists(REF_SO):
+        return {"unavailable": REF_MISSING}
     th = reference_threads()
     rr = ReferenceRun(cfg, th)
     sec, its = rr.step()
@@ -672,9 +678,8 @@ def run_reference(args) -> dict | None:
     if rank != 0:
         return None
     cfg = ics.config(args.workload)
-    ref_so = os.path.join(ROOT, "oracle", "_ref", "libapcref.so")
-    if not os.path.exists(ref_so):
-        return {"impl": "reference", "unavailable": "oracle/_ref/libapcref.so not built (make -C oracle ref)"}
+    if not os.path.exists(REF_SO):
+        return {"impl": "reference", "unavailable": REF_MISSING}
     th = reference_threads()
     rr = ReferenceRun(cfg, th)
     for _ in range(args.warmup):
