@@ -469,7 +469,7 @@ def run_ours(args) -> dict:
                             "octree-multigrid V-cycles; one cooperative launch per step)"
                             if args.persistent and args.precision == "mixed" else
                             "potential solve: one CUDA graph per step (" + PRECISIONS[args.precision][1] +
-                            "; ~20 kernels per iteration), timed as a unit",
+                            "; 13 kernels per iteration at 128^3), timed as a unit",
                   "bound": "hbm", "achieved": mg_achieved, "peak": peak, "unit": "GB/s",
                   "frac": mg_achieved / peak, "peak_kind": peak_kind,
                   "traffic": (mg_traffic * mg_bytes) if mg_traffic else None,
