@@ -442,7 +442,6 @@ constexpr int kCgSmemMax = 225 * 1024;  // beside its few static words
 struct CgArgs {
   GmresArgs<double> g;
   int nvb, rpb;               // blocks of the persistent kernel, rows of each
-  int K;                      // blocks per cluster
   unsigned o_u, o_col, o_red, o_nrm, o_hh, o_small;  // byte offsets in shared memory (values at 0)
 };
 
@@ -457,13 +456,18 @@ __device__ __forceinline__ double xor_sum(double t) {
 template <int THREADS>
 constexpr int kCgBatch = THREADS == 256 ? 18 : (THREADS == 512 ? 9 : 6);
 
+// K: blocks per cluster, fixed in the kernel and not by the launch.  A profiler that replays
+// cooperative launches drops the launch's cluster attribute; every block was then a cluster of
+// its own, worked on its first rows alone and returned a wrong solution after max_it.
 // SMEM_U: the rows' slice of the basis lies in shared memory too; a basis too long for that
 // (restart 200 on 128 rows per block) is read from L2.
-template <int THREADS, bool SMEM_U>
-__global__ void __launch_bounds__(THREADS, 1) gmres_cluster(const __grid_constant__ CgArgs C) {
+template <int THREADS, int K, bool SMEM_U>
+__global__ void __cluster_dims__(K, 1, 1) __launch_bounds__(THREADS, 1)
+    gmres_cluster(const __grid_constant__ CgArgs C) {
   extern __shared__ __align__(16) unsigned char cg_smem[];
   const GmresArgs<double> &A = C.g;
-  const int K = C.K, m = A.restart, vw = 32 / K, R = 32 * vw;  // 32-row warps, row slots
+  constexpr int vw = 32 / K, R = 32 * vw;  // 32-row warps, row slots
+  const int m = A.restart;
   double *val = reinterpret_cast<double *>(cg_smem);           // [slot][row]
   int *col = reinterpret_cast<int *>(cg_smem + C.o_col);
   double *red = reinterpret_cast<double *>(cg_smem + C.o_red); // first block: [warp][vector]
@@ -810,6 +814,7 @@ struct KrylovWork {
   double *hh = nullptr;  // per-block Hessenberg slices of the large-restart kernel
   size_t hh_bytes = 0;
   bool cg_set = false;  // gmres_cluster may take kCgSmemMax and clusters of 16
+  bool last_on_clusters = false;  // the last solve ran as gmres_cluster
   int cap_n = 0;
   int occ64[2] = {0, 0}, occ32[2] = {0, 0};
 };
@@ -829,36 +834,46 @@ void apc_krylov_free(apc_context *c) {
   c->kw = nullptr;
 }
 
+// The forms of gmres_cluster, the preferred first: the largest cluster whose shared memory
+// and co-residency allow it, with the basis in shared memory if it fits for any size.
+struct CgForm {
+  void (*kern)(CgArgs);
+  int K, threads;
+  bool smem_u;
+};
+static const CgForm kCgForms[] = {
+    {gmres_cluster<256, 16, true>, 16, 256, true},   {gmres_cluster<512, 8, true>, 8, 512, true},
+    {gmres_cluster<1024, 4, true>, 4, 1024, true},   {gmres_cluster<256, 16, false>, 16, 256, false},
+    {gmres_cluster<512, 8, false>, 8, 512, false},   {gmres_cluster<1024, 4, false>, 4, 1024, false},
+    {gmres_cluster<1024, 2, false>, 2, 1024, false},
+};
+
 // The solve on clusters (gmres_cluster) where it applies: `blocks` blocks of the persistent
-// kernel of at most 1024 rows, each taken by a cluster of the largest K whose shared memory
-// and co-residency allow it, at least 2, with the basis in shared memory if it fits for any
-// K.  *done says whether it was launched.  More rows keep the persistent kernel, whose blocks
-// then fill the SMs.  Measured, us per iteration, persistent kernel (with the same grid barrier)
-// and clusters: 4,096 rows 16.1 and 8.0, 20,322 rows 19.4 and 11.5, 32,768 rows 16.3 and 11.2.
+// kernel of at most 1024 rows, each taken by a cluster.  *done says whether it was launched.
+// More rows keep the persistent kernel, whose blocks then fill the SMs.  Measured, us per
+// iteration, persistent kernel (with the same grid barrier) and clusters: 4,096 rows 16.1 and
+// 8.0, 20,322 rows 19.4 and 11.5, 32,768 rows 16.3 and 11.2.
 static int launch_gmres_cluster(apc_context *c, const GmresArgs<double> &g, int blocks, bool *done) {
   KrylovWork *k = c->kw;
   const int m = g.restart, rpb = (g.n + blocks - 1) / blocks;
   *done = false;
   if (rpb > 1024 || blocks > kCgMaxClusters) return APC_OK;
-  void (*const kern[2][3])(CgArgs) = {
-      {gmres_cluster<256, true>, gmres_cluster<512, true>, gmres_cluster<1024, true>},
-      {gmres_cluster<256, false>, gmres_cluster<512, false>, gmres_cluster<1024, false>}};
   if (!k->cg_set) {
-    for (auto &fs : kern)
-      for (auto f : fs) {
-        APC_CUDA_TRY(c, cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kCgSmemMax));
-        APC_CUDA_TRY(c, cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-      }
+    for (const CgForm &f : kCgForms) {
+      APC_CUDA_TRY(c, cudaFuncSetAttribute((const void *)f.kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           kCgSmemMax));
+      APC_CUDA_TRY(c, cudaFuncSetAttribute((const void *)f.kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    }
     k->cg_set = true;
   }
-  for (int q = 0; q < 7; ++q) {  // 16, 8, 4 with the basis in shared memory; 16, 8, 4, 2 without
-    const int in_l2 = q >= 3, K = 16 >> (in_l2 ? q - 3 : q), v = std::min(in_l2 ? q - 3 : q, 2);
+  for (const CgForm &f : kCgForms) {
+    if (c->gmres_form != 0 && c->gmres_form != (f.smem_u ? f.K : -f.K)) continue;
+    const int K = f.K;
     const size_t R = 1024 / (size_t)K, M = (size_t)m;
     CgArgs C{};
     C.g = g;
     C.nvb = blocks;
     C.rpb = rpb;
-    C.K = K;
     size_t o = 0;
     auto take = [&](size_t bytes) {
       const size_t p = o;
@@ -866,7 +881,7 @@ static int launch_gmres_cluster(apc_context *c, const GmresArgs<double> &g, int 
       return (unsigned)p;
     };
     take((size_t)g.w * R * sizeof(double));
-    C.o_u = take(in_l2 ? 0 : (M + 1) * R * sizeof(double));
+    C.o_u = take(f.smem_u ? (M + 1) * R * sizeof(double) : 0);
     C.o_col = take((size_t)g.w * R * sizeof(int));
     C.o_red = take(32 * (M + 1) * sizeof(double));
     C.o_nrm = take(1024 * sizeof(double));
@@ -875,20 +890,18 @@ static int launch_gmres_cluster(apc_context *c, const GmresArgs<double> &g, int 
     if (o > kCgSmemMax) continue;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(blocks * K);
-    cfg.blockDim = dim3(std::min(1024, 4096 / K));
+    cfg.blockDim = dim3(f.threads);
     cfg.dynamicSmemBytes = o;
     cfg.stream = c->s;
-    cudaLaunchAttribute at[2];
+    cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = K;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
-    at[1].id = cudaLaunchAttributeCooperative;
-    at[1].val.cooperative = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
     int ncl = 0;
-    if (cudaOccupancyMaxActiveClusters(&ncl, kern[in_l2][v], &cfg) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&ncl, f.kern, &cfg) != cudaSuccess) {
       cudaGetLastError();
       continue;
     }
@@ -903,8 +916,9 @@ static int launch_gmres_cluster(apc_context *c, const GmresArgs<double> &g, int 
       }
       C.g.hh = k->hh;
     }
-    cfg.numAttrs = 2;
-    APC_CUDA_TRY(c, cudaLaunchKernelEx(&cfg, kern[in_l2][v], C));
+    void *args[] = {&C};
+    APC_CUDA_TRY(c, cudaLaunchCooperativeKernel((const void *)f.kern, dim3(blocks * K), dim3(f.threads), args, o,
+                                                c->s));
     *done = true;
     return APC_OK;
   }
@@ -977,7 +991,9 @@ static int launch_gmres(apc_context *c, int n, const T *val, const T *b, T *x, i
   void *args[] = {&a};
   APC_CUDA_TRY(c, cudaEventRecord(c->kev[0], c->s));
   bool on_clusters = false;
-  if constexpr (std::is_same_v<T, double> && !RE) APC_TRY(launch_gmres_cluster(c, a, blocks, &on_clusters));
+  if constexpr (std::is_same_v<T, double> && !RE)
+    if (c->gmres_form != 1) APC_TRY(launch_gmres_cluster(c, a, blocks, &on_clusters));
+  k->last_on_clusters = on_clusters;
   if (!on_clusters)
     APC_CUDA_TRY(c, cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(kThreads), args, 0, c->s));
   APC_CUDA_TRY(c, cudaEventRecord(c->kev[1], c->s));
@@ -1112,6 +1128,28 @@ int apc_krylov_solve(apc_context *c, int which, const double *b, double *x, int 
                        during));
   if (use_mg) c->stats.mg_levels = levels;
   return APC_OK;
+}
+
+// For the tests: the form of the context's next FP64 GMRES solves - 0 by the rule, 1 the
+// persistent kernel, K or -K clusters of K blocks with the basis in shared memory or in L2,
+// where they fit (the persistent kernel elsewhere) - and whether the last one ran on clusters.
+extern "C" int apc_test_gmres_form(apc_context *c, int form) {
+  if (!c) return APC_ERR_INVALID_ARG;
+  c->gmres_form = form;
+  return c->kw && c->kw->last_on_clusters ? 1 : 0;
+}
+
+// For the tests: the cluster size that form (K or -K, as above) is compiled for, 0 where the
+// launch alone would set it, -1 for no such form.
+extern "C" int apc_test_gmres_cluster_width(int device, int form) {
+  if (cudaSetDevice(device) != cudaSuccess) return APC_ERR_CUDA;
+  for (const CgForm &f : kCgForms) {
+    if (form != (f.smem_u ? f.K : -f.K)) continue;
+    cudaFuncAttributes fa{};
+    if (cudaFuncGetAttributes(&fa, (const void *)f.kern) != cudaSuccess) return APC_ERR_CUDA;
+    return fa.requiredClusterWidth;
+  }
+  return -1;
 }
 
 extern "C" int apc_check_bounded_wait(int device, int spin_limit) {
