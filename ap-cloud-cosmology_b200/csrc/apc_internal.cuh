@@ -347,6 +347,9 @@ __device__ __forceinline__ int block_scan_int(int v, int *sm, int *total) {
 __device__ __forceinline__ void cluster_barrier() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// the two halves of it, for work in between that needs no other block
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ unsigned cluster_rank() {
   unsigned r;
   asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));

@@ -1137,7 +1137,8 @@ constexpr size_t kSmemMax = 227 * 1024;  // dynamic shared memory a block may op
 // dependent launch costs 4-5 us whatever the level's size).  The restriction, the coarse
 // level's first sweep and the prolongation need no phase of their own: every block does them
 // for all rows on its own copies.  Per level that leaves four barriers: two pre-smoothing
-// sweeps in one pass, the residual, and two post-smoothing sweeps.
+// sweeps in one pass, the residual, and two post-smoothing sweeps; and one more, split around
+// the levels that every block holds whole (cl_vcycle).
 // A block's share (matrix, maps, 16-bit indices) is packed once per hierarchy (cl_pack) into
 // one contiguous image, so that a launch stages it with 16-byte asynchronous copies.
 // What bounds it is the chain of phases, ~0.7 us each.  At 128^3 (levels of 4111, 527, 78 and 20
@@ -1426,6 +1427,15 @@ __device__ __forceinline__ V *cl_vcycle(const ClCtx<V> &X, V *out) {
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int sw = X.sweeps, last = X.last;
   const V om = X.om, al = X.al;
+  // The deepest level that is spread over the blocks, unless it is the coarsest, whose phase
+  // ends in a cluster barrier.  Below it no barrier is met, and on the way up its first sweep
+  // stores to the other blocks' copies of the residual (the same buffer), so every block must
+  // have restricted its copy first: the blocks arrive after the restriction and wait before
+  // those stores, with the levels below in between.
+  int kd = -1;
+  if (X.dim[last].w)
+    for (int k = 0; k < last; ++k)
+      if (!X.dim[k].w) kd = k;
   // ---- down ----
   // a level's iterate lies in xb after one sweep (from zero: no operator) and changes sides
   // with each further one
@@ -1454,6 +1464,7 @@ __device__ __forceinline__ V *cl_vcycle(const ClCtx<V> &X, V *out) {
       }
     }
     __syncthreads();
+    if (k == kd) cluster_arrive();
   }
   // ---- the coarsest level: x = K^-1 b, a warp per row ----
   const ClView<V> K = X.view(last);
@@ -1480,12 +1491,10 @@ __device__ __forceinline__ V *cl_vcycle(const ClCtx<V> &X, V *out) {
     for (int i = t; i < Q.n; i += kClThreads) x[i] += al * xc[agg[i]];
     __syncthreads();
     for (int q = 0; q < sw; ++q) {
-      if (out && k == 0 && q + 1 == sw) {
-        cl_rows<false>(Q, x, om, out + Q.r0);
-      } else {
-        cl_rows<false>(Q, x, om, y + Q.r0);
-        Q.phase_end(y, X.rank);
-      }
+      const bool done = out && k == 0 && q + 1 == sw;
+      cl_rows<false>(Q, x, om, (done ? out : y) + Q.r0);
+      if (k == kd && q == 0) cluster_wait();
+      if (!done) Q.phase_end(y, X.rank);
       V *z = x; x = y; y = z;
     }
     xc = x;
