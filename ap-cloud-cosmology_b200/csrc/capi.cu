@@ -72,6 +72,10 @@ static int pool_alloc(apc_context *c, void **p, size_t bytes) {
 constexpr size_t kSlabMax = 256 << 10, kSlabBytes = 4 << 20;
 
 int apc_alloc(apc_context *c, void **p, size_t bytes) {
+  if (c->fail_alloc > 0 && --c->fail_alloc == 0) {
+    *p = nullptr;
+    return APC_ERR_OUT_OF_MEMORY;
+  }
   bytes = (std::max<size_t>(bytes, 16) + 255) & ~(size_t)255;
   if (bytes > kSlabMax) return pool_alloc(c, p, bytes);
   if (c->slabs.empty() || c->slab_used + bytes > kSlabBytes) {
@@ -91,6 +95,15 @@ void apc_free(apc_context *c, void *p) {
   for (char *q : c->slabs)
     if ((char *)p >= q && (char *)p < q + kSlabBytes) return;  // released with its slab
   cudaFreeAsync(p, c->s);
+}
+
+// For the tests: the context's nth device allocation from now on fails as one out of memory
+// would (0: none does).  Returns how many were left to go of an earlier call, 0 if it failed.
+extern "C" int apc_test_fail_alloc(apc_context *c, int nth) {
+  if (!c) return APC_ERR_INVALID_ARG;
+  const int left = c->fail_alloc;
+  c->fail_alloc = nth;
+  return left;
 }
 
 template <class T>

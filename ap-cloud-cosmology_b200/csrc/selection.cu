@@ -539,6 +539,7 @@ int grid_for(long long n) { return (int)std::max<long long>(1, (n + kT - 1) / kT
 
 static int ensure_hash(apc_context *c, uint64_t **keys, void **vals, size_t val_size, int *cap, int want) {
   if (want > *cap) {
+    *cap = 0;  // until both are there
     apc_free(c, *keys);
     apc_free(c, *vals);
     *keys = nullptr;
@@ -556,7 +557,12 @@ static int ensure_tree(apc_context *c, int want) {
   if (!c->tree_out)
     APC_TRY(apc_alloc(c, (void **)&c->tree_out, sizeof(TreeOut) + sizeof(GridBar) + kTreeLevels * sizeof(int)));
   if (want <= c->hcap) return APC_OK;
-  APC_TRY(ensure_hash(c, &c->h_keys, (void **)&c->h_vals, sizeof(int), &c->hcap, want));
+  // hcap stands for every table below: none until the last of them is there, so that the call
+  // after a failed allocation allocates what is missing
+  int hash_cap = c->hcap;
+  c->hcap = 0;
+  c->r_dirty = true;
+  APC_TRY(ensure_hash(c, &c->h_keys, (void **)&c->h_vals, sizeof(int), &hash_cap, want));
   const size_t open = (size_t)want / 2, rcap = std::max<size_t>(1 << 16, (size_t)want / 4);
   APC_TRY(apc_ensure(c, &c->op_code, open));
   APC_TRY(apc_ensure(c, &c->op_base, open));
@@ -569,7 +575,7 @@ static int ensure_tree(apc_context *c, int want) {
   APC_TRY(apc_ensure(c, &c->leaf_base, open / 4));
   APC_TRY(apc_ensure(c, &c->child_range, 8 * open));
   c->rcap = (int)rcap;
-  c->r_dirty = true;
+  c->hcap = hash_cap;
   return APC_OK;
 }
 
