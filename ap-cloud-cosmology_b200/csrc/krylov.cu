@@ -834,6 +834,19 @@ void apc_krylov_free(apc_context *c) {
   c->kw = nullptr;
 }
 
+// *p of at least `need` bytes; no capacity is kept from before a failed allocation.  Small
+// buffers grow by a quarter, as those of apc_ensure (what they outgrow stays in its slab).
+static int grow(apc_context *c, void **p, size_t *cap, size_t need) {
+  if (*p && need <= *cap) return APC_OK;
+  *cap = 0;
+  apc_free(c, *p);
+  *p = nullptr;
+  const size_t want = need <= (256 << 10) ? need + need / 4 : need;
+  APC_TRY(apc_alloc(c, p, want));
+  *cap = want;
+  return APC_OK;
+}
+
 // The forms of gmres_cluster, the preferred first: the largest cluster whose shared memory
 // and co-residency allow it, with the basis in shared memory if it fits for any size.
 struct CgForm {
@@ -907,13 +920,7 @@ static int launch_gmres_cluster(apc_context *c, const GmresArgs<double> &g, int 
     }
     if (ncl < blocks) continue;
     if (m > 31) {
-      const size_t hb = sizeof(double) * (size_t)blocks * K * (M + 1) * M;
-      if (hb > k->hh_bytes) {
-        apc_free(c, k->hh);
-        k->hh = nullptr;
-        APC_TRY(apc_alloc(c, (void **)&k->hh, hb));
-        k->hh_bytes = hb;
-      }
+      APC_TRY(grow(c, (void **)&k->hh, &k->hh_bytes, sizeof(double) * (size_t)blocks * K * (M + 1) * M));
       C.g.hh = k->hh;
     }
     void *args[] = {&C};
@@ -938,13 +945,7 @@ static int launch_gmres(apc_context *c, int n, const T *val, const T *b, T *x, i
   const void *kern = large ? (const void *)gmres_kernel<T, RE, kMaxRestart + 1>
                            : (const void *)gmres_kernel<T, RE, 32>;
   const size_t un = ((size_t)n + 31) & ~(size_t)31;
-  const size_t need = un * (restart + 1) * sizeof(T);
-  if (need > k->u_bytes) {
-    apc_free(c, k->U);
-    k->U = nullptr;
-    APC_TRY(apc_alloc(c, &k->U, need));
-    k->u_bytes = need;
-  }
+  APC_TRY(grow(c, &k->U, &k->u_bytes, un * (restart + 1) * sizeof(T)));
   int occ = 0;
   APC_CUDA_TRY(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kThreads, 0));
   if (occ < 1) {
@@ -956,15 +957,8 @@ static int launch_gmres(apc_context *c, int n, const T *val, const T *b, T *x, i
     APC_TRY(apc_alloc(c, (void **)&k->part, sizeof(double) * 2 * kSlots * (size_t)kMaxBlocks));
     k->part_blocks = kMaxBlocks;
   }
-  if (large) {
-    const size_t hb = sizeof(double) * (size_t)blocks * (restart + 1) * restart;
-    if (hb > k->hh_bytes) {
-      apc_free(c, k->hh);
-      k->hh = nullptr;
-      APC_TRY(apc_alloc(c, (void **)&k->hh, hb));
-      k->hh_bytes = hb;
-    }
-  }
+  if (large)
+    APC_TRY(grow(c, (void **)&k->hh, &k->hh_bytes, sizeof(double) * (size_t)blocks * (restart + 1) * restart));
   APC_CUDA_TRY(c, cudaMemsetAsync(k->bar, 0, sizeof(GridBar), c->s));
   GmresArgs<T> a;
   a.n = n;
@@ -1035,14 +1029,13 @@ static int launch_gmres(apc_context *c, int n, const T *val, const T *b, T *x, i
 }
 
 static int ensure_work(apc_context *c, int n) {
-  if (!c->kw) {
-    c->kw = new KrylovWork();
-    APC_TRY(apc_alloc(c, (void **)&c->kw->bar, sizeof(GridBar)));
-    APC_TRY(apc_alloc(c, (void **)&c->kw->ires, 4 * sizeof(int)));
-    APC_TRY(apc_alloc(c, (void **)&c->kw->dres, 2 * sizeof(double)));
-  }
+  if (!c->kw) c->kw = new KrylovWork();
   KrylovWork *k = c->kw;
+  if (!k->bar) APC_TRY(apc_alloc(c, (void **)&k->bar, sizeof(GridBar)));
+  if (!k->ires) APC_TRY(apc_alloc(c, (void **)&k->ires, 4 * sizeof(int)));
+  if (!k->dres) APC_TRY(apc_alloc(c, (void **)&k->dres, 2 * sizeof(double)));
   if (n > k->cap_n) {
+    k->cap_n = 0;
     apc_free(c, k->r);
     k->r = nullptr;
     const int cap = n + n / 4 + 1024;

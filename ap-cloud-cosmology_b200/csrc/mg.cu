@@ -2723,10 +2723,8 @@ static int mg_build(apc_context *c) {
   // level is wider than its allocation, the build runs again with room for it (the levels
   // below it were built from its truncated rows, so each repeat settles at least one more
   // level).
-  if (!m->wdev) {
-    APC_TRY(apc_alloc(c, (void **)&m->wdev, (kMaxLevels + 2) * sizeof(int)));
-    APC_CUDA_TRY(c, cudaMallocHost((void **)&m->whost, (kMaxLevels + 2) * sizeof(int)));
-  }
+  if (!m->wdev) APC_TRY(apc_alloc(c, (void **)&m->wdev, (kMaxLevels + 2) * sizeof(int)));
+  if (!m->whost) APC_CUDA_TRY(c, cudaMallocHost((void **)&m->whost, (kMaxLevels + 2) * sizeof(int)));
   int lev = 0;
   for (int attempt = 0; attempt <= S.nlev; ++attempt) {
   APC_CUDA_TRY(c, cudaMemsetAsync(m->wdev, 0, (kMaxLevels + 2) * sizeof(int), c->s));
@@ -2802,9 +2800,10 @@ static int mg_build(apc_context *c) {
   if (n <= kCoarseInvMax) {
     // on the device, in stream order: no host round trip; a singular operator is reported
     // by the solve that follows (check_coarse)
-    if (!m->cstat) {
-      APC_TRY(apc_alloc(c, (void **)&m->cstat, sizeof(int)));
+    if (!m->cstat) APC_TRY(apc_alloc(c, (void **)&m->cstat, sizeof(int)));
+    if (!m->cstat_host) {
       APC_CUDA_TRY(c, cudaMallocHost((void **)&m->cstat_host, sizeof(int)));
+      *m->cstat_host = 0;
       APC_CUDA_TRY(c, cudaFuncSetAttribute(coarse_inverse<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            kCoarseInvMax * 2 * kCoarseInvMax * (int)sizeof(double)));
       APC_CUDA_TRY(c, cudaFuncSetAttribute(coarse_inverse<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -3221,10 +3220,8 @@ template <class T>
 static int fill_psolve(apc_context *c, const IrSolveArgs<T> &a, PSolveArgs<T> &P) {
   MgWork *m = c->mg;
   MgHier<T> &H = hier<T>(m);
-  if (!m->ppart) {
-    APC_TRY(apc_alloc(c, (void **)&m->ppart, sizeof(double) * (size_t)kPSlots * kPMaxBlocks));
-    APC_TRY(apc_alloc(c, (void **)&m->pbar, sizeof(GridBar)));
-  }
+  if (!m->ppart) APC_TRY(apc_alloc(c, (void **)&m->ppart, sizeof(double) * (size_t)kPSlots * kPMaxBlocks));
+  if (!m->pbar) APC_TRY(apc_alloc(c, (void **)&m->pbar, sizeof(GridBar)));
   APC_TRY(ensure_result(c));
   P = PSolveArgs<T>{};
   P.n = a.n;
@@ -3640,6 +3637,7 @@ int apc_mg_structure_during_assembly(apc_context *c) {
   int rc = mg_structure(c);
   if (rc == APC_OK && cudaEventRecord(m->side_ev[2], c->s) != cudaSuccess) rc = APC_ERR_CUDA;
   c->s = main;
+  if (rc != APC_OK) cudaStreamSynchronize(m->side);  // what was queued there is done before the caller goes on
   APC_TRY(rc);
   m->st.on_side = true;
   c->prof.mg_build_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
@@ -3671,6 +3669,7 @@ int apc_mg_prebuild(apc_context *c) {
   int rc = c->cfg.precision == APC_PREC_FP64_MULTIGRID ? mg_build<double>(c) : mg_build<float>(c);
   if (rc == APC_OK && cudaEventRecord(m->side_ev[1], c->s) != cudaSuccess) rc = APC_ERR_CUDA;
   c->s = main;
+  if (rc != APC_OK) cudaStreamSynchronize(m->side);
   APC_TRY(rc);
   APC_CUDA_TRY(c, cudaStreamWaitEvent(c->s, m->side_ev[1], 0));
   m->prebuilt = true;

@@ -56,6 +56,7 @@ int apc_warm_save(apc_context *c) {
   const int m = c->nc + c->nv;
   int cap = 1024;
   while (cap < 2 * m) cap <<= 1;
+  c->warm_cap = 0;  // until the three are there: no guess after a failure
   APC_TRY(apc_ensure(c, &c->warm_keys, (size_t)cap, nullptr));
   APC_TRY(apc_ensure(c, &c->warm_rho, (size_t)cap, nullptr));
   APC_TRY(apc_ensure(c, &c->warm_phi, (size_t)cap, nullptr));

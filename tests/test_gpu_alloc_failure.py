@@ -64,3 +64,35 @@ def test_select_after_a_failed_allocation(gpu_lib, gfd_c, grow):
 
     lib = binding.load_library(gpu_lib)
     _each_allocation_fails(lib, new, lambda g: g.set_particles(_parts(True)) or g.select(), _cells, want, 10)
+
+
+@pytest.mark.parametrize("kw", [dict(), dict(restart=200), dict(precision=binding.APC_PREC_MIXED),
+                                dict(precision=binding.APC_PREC_MIXED, solve_graphs=0),
+                                dict(precision=binding.APC_PREC_MIXED_VCYCLE, mg_reorth=1),
+                                dict(precision=binding.APC_PREC_FP64_MULTIGRID)], ids=lambda k: "-".join(map(str, k.values())))
+def test_solve_after_a_failed_allocation(gpu_lib, kw):
+    n = 6000
+    parts = ics.uniform_ball(n, 0.3, seed=3)
+    c = 8.0 ** (5.0 / 3.0) * (n / (4.0 / 3.0 * np.pi * 0.3 ** 3)) ** (-2.0 / 3.0)
+    few = ics.uniform_ball(n, 0.3, seed=3)  # another state of the box first, whose buffers then grow
+    for a in (few.x, few.y, few.z):
+        a[:] = 0.5 + 0.2 * (a - 0.5)
+    solve = lambda g: g.solve(1.0 / n, 30.0, -1.0)  # noqa: E731
+    got = lambda g: [g.fields().density, g.fields().potential, g.fields().deriv]  # noqa: E731
+
+    def new(grow):
+        g = binding.GpuPath(few if grow else parts, 21, c, **kw)
+        g.select()
+        if grow:
+            solve(g)
+            g.set_particles(parts)
+            g.select()
+        return g
+
+    g = new(False)
+    solve(g)
+    want = got(g)
+    g.close()
+    lib = binding.load_library(gpu_lib)
+    _each_allocation_fails(lib, lambda: new(False), solve, got, want, 15)
+    _each_allocation_fails(lib, lambda: new(True), solve, got, want, 1)
