@@ -86,11 +86,11 @@ __global__ void __launch_bounds__(kNoThreads) noalloc_kick(int n, int m, const i
   // ---- the ranges: a thread per cell; a cell of many words by its whole warp ----
   {
     unsigned long long mine = 0;
-    const int rounds = (m + threads - 1) / threads;
-    for (int r = 0; r < rounds; ++r) {  // the same count for every lane (ballots)
-      const int i = r * threads + g0;
+    const unsigned rounds = ((unsigned)m + (unsigned)threads - 1u) / (unsigned)threads;
+    for (unsigned r = 0; r < rounds; ++r) {  // the same count for every lane (ballots)
+      const unsigned i = r * (unsigned)threads + (unsigned)g0;  // past m, a multiple of the grid: no int
       long long f = 0, c = 0;
-      if (i < m) {
+      if (i < (unsigned)m) {
         f = first[i];
         c = count[i];
         if (c < 0 || (c > 0 && (f < 0 || f + c > n))) {
@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(kNoThreads) noalloc_kick(int n, int m, const i
         }
         if (c >= kNoBig) {  // more than kNoBigMax of them overlap
           const int q = atomicAdd(&acc->nbig, 1);
-          if (q < kNoBigMax) S->big[q] = i;
+          if (q < kNoBigMax) S->big[q] = (int)i;
         }
       }
       mine += (unsigned long long)c;
@@ -148,9 +148,10 @@ __global__ void __launch_bounds__(kNoThreads) noalloc_kick(int n, int m, const i
       mx = fmax(mx, __dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(sq, cv), cv), dt), dt));
     }
   };
-  for (int i = g0 / LANES; i < m && ok; i += threads / LANES) {
+  for (unsigned i = (unsigned)(g0 / LANES); i < (unsigned)m && ok; i += (unsigned)(threads / LANES)) {
     const int f = first[i], c = count[i];
-    if (c < kNoBig) kick_cell(i, f + g0 % LANES, f + c, LANES);
+    // nothing is formed from an empty cell's first: it may be any value
+    if (c > 0 && c < kNoBig) kick_cell((int)i, f + g0 % LANES, f + c, LANES);
   }
   const int nbig = ok ? min(*(volatile int *)&acc->nbig, kNoBigMax) : 0;
   for (int q = 0; q < nbig; ++q) {
