@@ -25,10 +25,14 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoallocScratch
 constexpr int kMaxDevices = 64;
 std::mutex g_setup_mutex;
 void *g_scratch_ptr[kMaxDevices] = {nullptr};
-void *g_result_ptr[kMaxDevices] = {nullptr};  // pinned host words, one set per device
+std::mutex g_call_mutex[kMaxDevices];  // held for a whole call: the scratch is one per device
 
 // The scratch array: one bit per particle, the cells of many particles, and the accumulators,
-// zero before the first call and left zero by every call.
+// which every call clears before its launch and copies to its own stack after it: nothing is
+// handed from one call to the next, and a device takes one call at a time.  (Accumulators left
+// clear by the kernel and results in pinned words saved the two stream operations, 8 us of
+// a call; but a call that broke off spoilt the next, threads read each other's results, and the
+// pinned words had to be allocated.)
 constexpr int kNoThreads = 512;
 constexpr int kNoBig = 2048;  // particles from which a cell is spread over the whole grid
 constexpr int kNoWords = APC_NOALLOC_MAX_PARTICLES / 32;
@@ -39,14 +43,7 @@ struct NoallocAcc {
   int bad;                     // ranges outside [0, n), or overlapping
   int err;                     // a grid barrier gave up
   int nbig;
-  int done;                    // blocks that have finished
   GridBar bar;
-};
-// what the host reads: written by the last block straight to pinned memory, so that a call is
-// one launch and one wait
-struct NoallocResult {
-  unsigned long long maxbits, total;
-  int bad, pending;            // pending: set by the host, cleared by the kernel
 };
 struct NoallocScratch {
   unsigned bits[kNoWords];
@@ -61,7 +58,7 @@ static_assert(sizeof(NoallocScratch) <= kNoallocScratchBytes, "fits the scratch 
 // kick, LANES lanes per cell, so that no particle -> cell map is written, checked and read
 // back.  The last phase is bound by memory: 96 B per particle beside its cell's row.
 // 1,000,003 particles in 111,111 cells: two memsets and three kernels took 52 us on the device,
-// this kernel 33 us (25 us of it the kick); a call from Python 99 -> 81 us.
+// this kernel 33 us (25 us of it the kick); a call from Python 99 -> 88 us.
 template <int LANES>
 __global__ void __launch_bounds__(kNoThreads) noalloc_kick(int n, int m, const int *__restrict__ first,
                                                            const int *__restrict__ count,
@@ -75,7 +72,7 @@ __global__ void __launch_bounds__(kNoThreads) noalloc_kick(int n, int m, const i
                                                            double *__restrict__ vy, double *__restrict__ vz,
                                                            double *__restrict__ ax, double *__restrict__ ay,
                                                            double *__restrict__ az, double cv, double dt,
-                                                           NoallocScratch *S, NoallocResult *result) {
+                                                           NoallocScratch *S) {
   __shared__ double sm[kNoThreads / 32];
   NoallocAcc *acc = &S->acc;
   const int t = threadIdx.x, lane = t & 31;
@@ -166,38 +163,26 @@ __global__ void __launch_bounds__(kNoThreads) noalloc_kick(int n, int m, const i
     double b = 0.0;
     for (int w = 0; w < kNoThreads / 32; ++w) b = fmax(b, sm[w]);
     atomicMax(&acc->maxbits, (unsigned long long)__double_as_longlong(b));
-    __threadfence();
-    if (atomicAdd(&acc->done, 1) == (int)gridDim.x - 1) {
-      result->maxbits = atomicExch(&acc->maxbits, 0ull);
-      result->total = atomicExch(&acc->total, 0ull);
-      result->bad = atomicExch(&acc->bad, 0);
-      atomicExch(&acc->nbig, 0);
-      atomicExch(&acc->done, 0);
-      atomicExch(&acc->bar.count, 0u);
-      __threadfence_system();
-      *(volatile int *)&result->pending = 0;
-    }
   }
 }
 
-// Device address of the scratch array for `dev` and its pinned result words, set up once per
-// device with that device current.  In host code the array's name is only a host-side
-// stand-in, so the kernels are always given this address.
-int scratch_for(int dev, void **out, void **result) {
+// Device address of the scratch array for `dev`, looked up once per device with that
+// device current.  In host code the array's name is only a host-side stand-in, so the
+// kernels are always given this address.
+int scratch_for(int dev, void **out) {
   std::lock_guard<std::mutex> lock(g_setup_mutex);
-  if (!g_scratch_ptr[dev]) {
-    void *p = nullptr, *r = nullptr;
-    cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
-    if (e == cudaSuccess && p) e = cudaHostAlloc(&r, sizeof(NoallocResult), cudaHostAllocPortable);
-    if (e != cudaSuccess || !p) {
-      cudaGetLastError();
-      return APC_ERR_CUDA;
-    }
-    g_result_ptr[dev] = r;
-    g_scratch_ptr[dev] = p;
+  if (g_scratch_ptr[dev]) {
+    *out = g_scratch_ptr[dev];
+    return APC_OK;
   }
-  *out = g_scratch_ptr[dev];
-  *result = g_result_ptr[dev];
+  void *p = nullptr;
+  cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
+  if (e != cudaSuccess || !p) {
+    cudaGetLastError();
+    return APC_ERR_CUDA;
+  }
+  g_scratch_ptr[dev] = p;
+  *out = p;
   return APC_OK;
 }
 
@@ -219,13 +204,11 @@ extern "C" int apc_move_velocity_noalloc(int n_particles, int n_cells, const int
     cudaGetLastError();
     return APC_ERR_CUDA;
   }
-  void *base = nullptr, *words = nullptr;
-  int rc = scratch_for(dev, &base, &words);
+  void *base = nullptr;
+  int rc = scratch_for(dev, &base);
   if (rc != APC_OK) return rc;
   cudaStream_t s = (cudaStream_t)stream;
   NoallocScratch *S = (NoallocScratch *)base;
-  NoallocResult *result = (NoallocResult *)words;
-  result->pending = 1;
   // lanes per cell: half the mean count or more, so that most cells take one or two rounds
   const double mean = (double)n_particles / n_cells;
   const void *kern = mean <= 8 ? (const void *)noalloc_kick<4>
@@ -244,26 +227,23 @@ extern "C" int apc_move_velocity_noalloc(int n_particles, int n_cells, const int
   const long long want = (std::max((long long)n_particles, (long long)n_cells * lanes) + kNoThreads - 1) / kNoThreads;
   const int blocks = (int)std::max(1ll, std::min(want, (long long)sms * occ));
   void *args[] = {&n_particles, &n_cells, &first, &count, &deriv9, &cx, &cy, &cz, &x, &y, &z, &vx, &vy, &vz,
-                  &ax, &ay, &az, &c_vel, &dt, &S, &result};
-  if (cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(kNoThreads), args, 0, s) != cudaSuccess) {
+                  &ax, &ay, &az, &c_vel, &dt, &S};
+  NoallocAcc got;
+  std::lock_guard<std::mutex> lock(g_call_mutex[dev]);
+  if (cudaMemsetAsync(&S->acc, 0, sizeof(NoallocAcc), s) != cudaSuccess ||
+      cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(kNoThreads), args, 0, s) != cudaSuccess ||
+      cudaMemcpyAsync(&got, &S->acc, sizeof(got), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+      cudaStreamSynchronize(s) != cudaSuccess) {
     cudaGetLastError();
     return APC_ERR_CUDA;
   }
-  if (cudaStreamSynchronize(s) != cudaSuccess) {
-    cudaGetLastError();
-    return APC_ERR_CUDA;
-  }
-  if (*(volatile int *)&result->pending) {  // a grid barrier gave up: nothing was written
-    cudaMemsetAsync(&S->acc, 0, sizeof(NoallocAcc), s);
-    cudaStreamSynchronize(s);
-    return APC_ERR_TIMEOUT;
-  }
+  if (got.err) return APC_ERR_TIMEOUT;  // a grid barrier gave up
   // cell ranges outside [0, n), overlapping, or leaving a particle uncovered: caller input,
   // so an invalid argument (the context path builds its ranges itself); nothing was written
-  if (result->bad || result->total != (unsigned long long)n_particles) return APC_ERR_INVALID_ARG;
+  if (got.bad || got.total != (unsigned long long)n_particles) return APC_ERR_INVALID_ARG;
   if (max_dv) {
     double v;
-    std::memcpy(&v, &result->maxbits, sizeof(v));
+    std::memcpy(&v, &got.maxbits, sizeof(v));
     *max_dv = std::sqrt(v);
   }
   return APC_OK;

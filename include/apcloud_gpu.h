@@ -254,9 +254,8 @@ int apc_reset_profile(apc_context *ctx);
  * on a device looks up the array's device address (once per device) and should come
  * before any stream capture; that address is kept for the life of the process, so the
  * call must not be used on a device again after cudaDeviceReset there.  All calls share
- * the one array: calls whose work overlaps on the GPU (other streams, other host
- * threads) race and must be serialised by the caller.  Each call resets the parts of the
- * scratch that must start cleared.
+ * the one array, so a device takes one call at a time: host threads wait for each other.
+ * Each call resets the parts of the scratch that must start cleared.
  *
  * Inputs, all device pointers on the current device: particles x, y, z in cell order
  * (cell i owns particles first[i] .. first[i]+count[i]-1); cell centres cx, cy, cz;
