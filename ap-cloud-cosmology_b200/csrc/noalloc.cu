@@ -42,9 +42,11 @@ struct NoallocAcc {
   unsigned long long total;    // particles in all ranges
   int bad;                     // ranges outside [0, n), or overlapping
   int err;                     // a grid barrier gave up
+  int outcome;                 // of the second barrier, the same for every block: kKick or kLeave
   int nbig;
   GridBar bar;
 };
+enum { kKick = 1, kLeave = 2 };
 struct NoallocScratch {
   unsigned bits[kNoWords];
   int big[kNoBigMax];
@@ -72,8 +74,9 @@ __global__ void __launch_bounds__(kNoThreads) noalloc_kick(int n, int m, const i
                                                            double *__restrict__ vy, double *__restrict__ vz,
                                                            double *__restrict__ ax, double *__restrict__ ay,
                                                            double *__restrict__ az, double cv, double dt,
-                                                           NoallocScratch *S) {
+                                                           NoallocScratch *S, long long limit0) {
   __shared__ double sm[kNoThreads / 32];
+  __shared__ int s_outcome;
   NoallocAcc *acc = &S->acc;
   const int t = threadIdx.x, lane = t & 31;
   const int threads = gridDim.x * kNoThreads, g0 = blockIdx.x * kNoThreads + t;
@@ -118,7 +121,15 @@ __global__ void __launch_bounds__(kNoThreads) noalloc_kick(int n, int m, const i
     for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
     if (lane == 0 && mine) atomicAdd(&acc->total, mine);
   }
-  if (!grid_sync(&acc->bar, gridDim.x, epoch, &acc->err)) return;
+  // A block whose wait runs out here leaves, and another may still find every block arrived.  All
+  // take the first claim, so that a call that gives up has written nothing.
+  const bool met = grid_sync(&acc->bar, gridDim.x, epoch, &acc->err, blockIdx.x == 0 ? limit0 : kSpinLimit);
+  if (t == 0) {
+    const int mine = met ? kKick : kLeave, first_claim = atomicCAS(&acc->outcome, 0, mine);
+    s_outcome = first_claim != 0 ? first_claim : mine;
+  }
+  __syncthreads();
+  if (s_outcome != kKick) return;
   // malformed cell ranges leave every output untouched
   const bool ok =
       *(volatile int *)&acc->bad == 0 && *(volatile unsigned long long *)&acc->total == (unsigned long long)n;
@@ -188,12 +199,11 @@ int scratch_for(int dev, void **out) {
 
 }  // namespace
 
-extern "C" int apc_move_velocity_noalloc(int n_particles, int n_cells, const int *first, const int *count,
-                                         const double *cx, const double *cy, const double *cz,
-                                         const double *deriv9, const double *x, const double *y,
-                                         const double *z, double *vx, double *vy, double *vz, double *ax,
-                                         double *ay, double *az, double dt, double c_vel, double *max_dv,
-                                         void *stream) {
+// limit0: polls of the first block at the second barrier
+static int noalloc_call(int n_particles, int n_cells, const int *first, const int *count, const double *cx,
+                        const double *cy, const double *cz, const double *deriv9, const double *x, const double *y,
+                        const double *z, double *vx, double *vy, double *vz, double *ax, double *ay, double *az,
+                        double dt, double c_vel, double *max_dv, void *stream, long long limit0) {
   if (n_particles < 1 || n_cells < 1) return APC_ERR_INVALID_ARG;
   if (n_particles > APC_NOALLOC_MAX_PARTICLES) return APC_ERR_INVALID_ARG;  // beyond the scratch array
   if (!first || !count || !cx || !cy || !cz || !deriv9 || !x || !y || !z || !vx || !vy || !vz || !ax || !ay ||
@@ -227,7 +237,7 @@ extern "C" int apc_move_velocity_noalloc(int n_particles, int n_cells, const int
   const long long want = (std::max((long long)n_particles, (long long)n_cells * lanes) + kNoThreads - 1) / kNoThreads;
   const int blocks = (int)std::max(1ll, std::min(want, (long long)sms * occ));
   void *args[] = {&n_particles, &n_cells, &first, &count, &deriv9, &cx, &cy, &cz, &x, &y, &z, &vx, &vy, &vz,
-                  &ax, &ay, &az, &c_vel, &dt, &S};
+                  &ax, &ay, &az, &c_vel, &dt, &S, &limit0};
   NoallocAcc got;
   std::lock_guard<std::mutex> lock(g_call_mutex[dev]);
   if (cudaMemsetAsync(&S->acc, 0, sizeof(NoallocAcc), s) != cudaSuccess ||
@@ -237,7 +247,7 @@ extern "C" int apc_move_velocity_noalloc(int n_particles, int n_cells, const int
     cudaGetLastError();
     return APC_ERR_CUDA;
   }
-  if (got.err) return APC_ERR_TIMEOUT;  // a grid barrier gave up
+  if (got.outcome != kKick) return APC_ERR_TIMEOUT;  // a grid barrier gave up: nothing was written
   // cell ranges outside [0, n), overlapping, or leaving a particle uncovered: caller input,
   // so an invalid argument (the context path builds its ranges itself); nothing was written
   if (got.bad || got.total != (unsigned long long)n_particles) return APC_ERR_INVALID_ARG;
@@ -247,4 +257,25 @@ extern "C" int apc_move_velocity_noalloc(int n_particles, int n_cells, const int
     *max_dv = std::sqrt(v);
   }
   return APC_OK;
+}
+
+extern "C" int apc_move_velocity_noalloc(int n_particles, int n_cells, const int *first, const int *count,
+                                         const double *cx, const double *cy, const double *cz,
+                                         const double *deriv9, const double *x, const double *y,
+                                         const double *z, double *vx, double *vy, double *vz, double *ax,
+                                         double *ay, double *az, double dt, double c_vel, double *max_dv,
+                                         void *stream) {
+  return noalloc_call(n_particles, n_cells, first, count, cx, cy, cz, deriv9, x, y, z, vx, vy, vz, ax, ay, az, dt,
+                      c_vel, max_dv, stream, kSpinLimit);
+}
+
+// For the tests: the same call, with a wait of the first block that gives up after spin_limit polls.
+extern "C" int apc_test_move_velocity_noalloc(int spin_limit, int n_particles, int n_cells, const int *first,
+                                              const int *count, const double *cx, const double *cy, const double *cz,
+                                              const double *deriv9, const double *x, const double *y, const double *z,
+                                              double *vx, double *vy, double *vz, double *ax, double *ay, double *az,
+                                              double dt, double c_vel, double *max_dv, void *stream) {
+  if (spin_limit < 1 || spin_limit > kSpinLimit) return APC_ERR_INVALID_ARG;
+  return noalloc_call(n_particles, n_cells, first, count, cx, cy, cz, deriv9, x, y, z, vx, vy, vz, ax, ay, az, dt,
+                      c_vel, max_dv, stream, spin_limit);
 }
