@@ -162,6 +162,7 @@ struct apc_context {
   bool step_open = false;    // a select has started a step that move_position will close
   unsigned select_gen = 0;   // completed selections (keys the multigrid aggregation to its cells)
   int fail_alloc = 0;        // for the tests: the allocation to fail, counted down (apc_alloc)
+  bool no_clusters = false;  // for the tests: as on a device without clusters of 16 blocks (mg.cu)
   int gmres_form = 0;        // FP64 GMRES: 0 by the rule, others for the tests (krylov.cu)
   bool kick_recorded = false;  // ev[4] holds the start of a move_velocity
 };

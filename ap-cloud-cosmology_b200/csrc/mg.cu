@@ -33,6 +33,7 @@
 #include <chrono>
 #include <cmath>
 #include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "apc_internal.cuh"
@@ -998,7 +999,7 @@ static inline int tail_lanes(int n, int w, int threads) {
 }
 
 // the graph path's tail kernel, for levels that do not fit the cluster kernel's shared
-// memory (rows of hundreds of slots): 512 threads leave 128 registers a thread for the batched
+// memory (rows of hundreds of slots) and devices without its clusters: 512 threads leave 128 registers a thread for the batched
 // row loads (a 1024-thread block has 64)
 constexpr int kTailThreads = 512;
 // sum_j a_ij xj(j) for every row of a tail level, L.g lanes per row; emit(i, sum) runs on
@@ -2476,7 +2477,8 @@ struct MgWork {
   // checked after the next solve's readback
   int *cstat = nullptr;
   int *cstat_host = nullptr;
-  bool cluster_set = false;  // vcycle_cluster may take kSmemMax and a 16-block cluster
+  // the cluster kernels asked about so far, and whether the device takes a cluster of them
+  std::vector<std::pair<const void *, bool>> cluster_kernels;
   // the numeric build's per-level widths (device, and its pinned readback; [kMaxLevels + 1]
   // is the ELL overflow flag) and the ELL slots allocated per level (host, the widest seen)
   int *wdev = nullptr;
@@ -2643,20 +2645,54 @@ static int mg_structure(apc_context *c) {
   return APC_OK;
 }
 
+// one cluster of kClBlocks blocks
+static void cluster_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *at, size_t smem, cudaStream_t s) {
+  cfg.gridDim = dim3(kClBlocks);
+  cfg.blockDim = dim3(kClThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = kClBlocks;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+}
+
+// Whether the device takes a cluster of kClBlocks blocks of `kern` with up to `smem` bytes of
+// dynamic shared memory each (asked once per context and kernel).  A part of a device may have
+// no 16 SMs that form a cluster; the solves then run in the forms without one.
+static bool cluster_ready(apc_context *c, const void *kern, size_t smem) {
+  if (c->no_clusters) return false;
+  auto &known = c->mg->cluster_kernels;
+  for (auto &k : known)
+    if (k.first == kern) return k.second;
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at[1];
+  cluster_config(cfg, at, smem, c->s);
+  int ncl = 0;
+  const bool ok =
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
+      cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+      cudaOccupancyMaxActiveClusters(&ncl, kern, &cfg) == cudaSuccess && ncl >= 1;
+  if (!ok) cudaGetLastError();
+  known.push_back({kern, ok});
+  return ok;
+}
+
+// For the tests: the context's next solves as on a device without clusters (on != 0).
+extern "C" int apc_test_no_clusters(apc_context *c, int on) {
+  if (!c) return APC_ERR_INVALID_ARG;
+  c->no_clusters = on != 0;
+  return APC_OK;
+}
+
 // The levels that vcycle_cluster runs (from the first that fits) and their packed shares,
 // on c->s after the hierarchy's operators and the coarsest inverse.
 template <class T>
 static int cluster_levels(apc_context *c, MgHier<T> &H) {
-  MgWork *m = c->mg;
   H.cl_first = -1;
-  if (!m->cluster_set) {
-    for (const void *f : {(const void *)vcycle_cluster<float>, (const void *)vcycle_cluster<double>}) {
-      APC_CUDA_TRY(c, cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)(kSmemMax - kClStatic)));
-      APC_CUDA_TRY(c, cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    }
-    m->cluster_set = true;
-  }
+  if (!cluster_ready(c, (const void *)vcycle_cluster<T>, kSmemMax - kClStatic)) return APC_OK;
   for (int l = std::max(0, H.nlev - kClLevels); l < H.nlev; ++l) {
     ClArgs<T> A{};
     A.nl = H.nlev - l;
@@ -2882,20 +2918,6 @@ static int ensure_result(apc_context *c) {
   return APC_OK;
 }
 
-// one cluster of kClBlocks blocks
-static void cluster_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *at, size_t smem, cudaStream_t s) {
-  cfg.gridDim = dim3(kClBlocks);
-  cfg.blockDim = dim3(kClThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = kClBlocks;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-}
-
 // x = V-cycle(b) on level l, launched on stream s; b and x are that level's buffers
 template <class T>
 static void vcycle(apc_context *c, cudaStream_t s, int l, const T *b, T *x) {
@@ -2924,7 +2946,7 @@ static void vcycle(apc_context *c, cudaStream_t s, int l, const T *b, T *x) {
     return;
   }
   if (n <= kTail || l == H.nlev - 1) {
-    // levels that do not fit a cluster (rows of hundreds of slots): a single block
+    // levels that do not fit a cluster (rows of hundreds of slots), or no cluster: a single block
     TailArgs<T> A{};
     A.nl = std::min(H.nlev - l, kTailLevels);
     A.inv = H.coarse_inv;
@@ -3359,8 +3381,8 @@ static double solve_bytes(const MgHier<TV> &H, bool use_mg, int n, int w, int sw
   return outer * per_outer + total_its * per_it;
 }
 
-// A whole solve on one cluster (solve_cluster) where it fits: a row per thread and, for the
-// potential, the whole hierarchy in the cluster's shared memory; for the density, its operator
+// A whole solve on one cluster (solve_cluster) where the device has one and it fits: a row per thread
+// and, for the potential, the whole hierarchy in the cluster's shared memory; for the density, its operator
 // and one gathered vector.  *done says whether it was launched.
 template <class T, class TV>
 static int cluster_solve(apc_context *c, const IrSolveArgs<T> &a, bool *done) {
@@ -3411,9 +3433,7 @@ static int cluster_solve(apc_context *c, const IrSolveArgs<T> &a, bool *done) {
     kern = a.M <= 16 ? solve_cluster<T, TV, true, 16> : solve_cluster<T, TV, true, 32>;
   else
     kern = a.M <= 16 ? solve_cluster<T, TV, false, 16> : solve_cluster<T, TV, false, 32>;
-  APC_CUDA_TRY(c, cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)kClSolveDyn));
-  APC_CUDA_TRY(c, cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  if (!cluster_ready(c, (const void *)kern, kClSolveDyn)) return APC_OK;
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute at[1];
   cluster_config(cfg, at, A.total, c->s);
