@@ -2687,11 +2687,18 @@ extern "C" int apc_test_no_clusters(apc_context *c, int on) {
   return APC_OK;
 }
 
+// One persistent kernel per solve can run: the re-orthogonalising Gram-Schmidt and the FP32
+// V-cycle under FP64 vectors are only in the other forms.
+static bool can_persist(const apc_context *c, bool mg32) { return !c->cfg.mg_reorth && !mg32; }
+
 // The levels that vcycle_cluster runs (from the first that fits) and their packed shares,
 // on c->s after the hierarchy's operators and the coarsest inverse.
 template <class T>
 static int cluster_levels(apc_context *c, MgHier<T> &H) {
   H.cl_first = -1;
+  // the persistent solves, queued for a batch or not, read the levels themselves
+  if (can_persist(c, c->cfg.precision == APC_PREC_MIXED_VCYCLE) && (c->defer_solve || !c->cfg.mixed_solve_graphs))
+    return APC_OK;
   if (!cluster_ready(c, (const void *)vcycle_cluster<T>, kSmemMax - kClStatic)) return APC_OK;
   for (int l = std::max(0, H.nlev - kClLevels); l < H.nlev; ++l) {
     ClArgs<T> A{};
@@ -3503,10 +3510,9 @@ static int ir_solve(apc_context *c, int which, bool use_mg, const double *val, c
   // bounds the loop in every case
   a.max_outer = use_mg && sizeof(T) == sizeof(float) ? 40 : std::max(40, cfg.gmres_max_it);
   a.M = M;
-  // one persistent kernel per solve unless the graph path is asked for (or needed: the
-  // re-orthogonalising Gram-Schmidt and the FP32 V-cycle under FP64 vectors run only there)
-  const bool can_persist = !cfg.mg_reorth && !mg32;
-  bool persistent = can_persist && !cfg.mixed_solve_graphs;
+  // one persistent kernel per solve unless the graph path is asked for (or needed)
+  const bool persists = can_persist(c, mg32);
+  bool persistent = persists && !cfg.mixed_solve_graphs;
   // the outcome of a solve that ran as one kernel, read back
   auto outcome = [&](const PResult &R) -> int {
     float ms = 0.f;
@@ -3523,7 +3529,7 @@ static int ir_solve(apc_context *c, int which, bool use_mg, const double *val, c
     }
     return APC_OK;
   };
-  if (can_persist && c->defer_solve) {
+  if (persists && c->defer_solve) {
     // prepared for a batched launch with other boxes' solves (apc_mg_batched_solve);
     // apc_ir_finish reads the outcome
     if (use_mg)
