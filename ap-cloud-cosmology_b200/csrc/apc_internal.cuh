@@ -95,6 +95,7 @@ struct apc_context {
   int *op_base = nullptr;        // temp index of the node's first child
   int *op_first = nullptr, *op_count = nullptr;  // particle range (all opened nodes)
   int n_open_td = 0, n_open = 0;
+  int open_hint = 0;             // nodes that the last attempt at a selection opened: sizes the next one's grid
   int *r_list = nullptr;         // used slots of the two request tables
   bool r_dirty = true;           // the request tables may hold entries
   uint32_t *child_words = nullptr;  // one bit per child: two levels in turn, the leaves

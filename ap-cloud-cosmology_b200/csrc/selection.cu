@@ -112,6 +112,9 @@ constexpr int kTreeThreads = 512;
 constexpr int kTreeWarps = kTreeThreads / 32;
 constexpr int kTreeLevels = 24;
 constexpr int kReqChunk = 4096;  // requests of a sweep that are ordered together (a power of two)
+constexpr int kReqKeys = 4;      // and keys that a thread looks up in each chunk at a time
+constexpr int kTreeBlocks = 2;   // blocks per SM, for trees of more than kTreeTwo opened nodes
+constexpr int kTreeTwo = 1 << 20;
 
 // what the host reads back: the sizes, and why the kernel stopped early
 enum : int { TREE_FULL = 1, TREE_DEEPER = 2 };
@@ -237,29 +240,48 @@ __device__ __noinline__ void sort_requests(const int *list, const unsigned long 
   for (int i = t; i < cn; i += kTreeThreads) sorted[c0 + i] = s_key[i];
 }
 
-// By the block: the number of requests below each thread's key, chunk by chunk
-__device__ __noinline__ int rank_requests(const unsigned long long *sorted, int nreq, unsigned long long key,
-                                          unsigned long long *s_key) {
-  int rank = 0;
+// By the block: the number of requests below each of a thread's keys, chunk by chunk.  The
+// thread's key q is key i + q stride, the block's first i0 + q stride.
+__device__ __noinline__ void rank_requests(const unsigned long long *sorted, int nreq, int i0, int stride,
+                                           unsigned long long *s_key, unsigned long long (&key)[kReqKeys],
+                                           int (&rank)[kReqKeys]) {
+  const int t = threadIdx.x;
+#pragma unroll
+  for (int q = 0; q < kReqKeys; ++q) {
+    const long long i = i0 + t + (long long)q * stride;
+    key[q] = i < nreq ? __ldcg(sorted + i) : 0ull;
+    rank[q] = 0;
+  }
   for (int c0 = 0; c0 < nreq; c0 += kReqChunk) {
     __syncthreads();
-    for (int j = threadIdx.x; j < kReqChunk; j += kTreeThreads)
-      s_key[j] = c0 + j < nreq ? __ldcg(sorted + c0 + j) : ~0ull;
+    for (int j = t; j < kReqChunk; j += kTreeThreads) s_key[j] = c0 + j < nreq ? __ldcg(sorted + c0 + j) : ~0ull;
     __syncthreads();
-    int at = 0;
+    int at[kReqKeys];
+#pragma unroll
+    for (int q = 0; q < kReqKeys; ++q) at[q] = 0;
+    const int keys = i0 + (long long)stride < nreq ? kReqKeys : 1;  // the same for the whole block
+    if (keys == 1) {
+#pragma unroll
+      for (int step = kReqChunk / 2; step > 0; step >>= 1)
+        if (s_key[at[0] + step - 1] < key[0]) at[0] += step;
+      rank[0] += at[0] + (s_key[at[0]] < key[0] ? 1 : 0);
+      continue;
+    }
 #pragma unroll
     for (int step = kReqChunk / 2; step > 0; step >>= 1)
-      if (s_key[at + step - 1] < key) at += step;
-    rank += at + (s_key[at] < key ? 1 : 0);
+#pragma unroll
+      for (int q = 0; q < kReqKeys; ++q)
+        if (s_key[at[q] + step - 1] < key[q]) at[q] += step;
+#pragma unroll
+    for (int q = 0; q < kReqKeys; ++q) rank[q] += at[q] + (s_key[at[q]] < key[q] ? 1 : 0);
   }
-  return rank;
 }
 
 // The opened nodes of the octree (top-down refinement, then the 2:1 balance) in the
 // reference's temp-node order, and the numbering of their leaves.  The root is open (the host
 // tests it).  Every block takes the same branches: the counts it branches on are read after a
 // barrier.  What bounds it is the chain of ~4 barriers and dependent key probes per level.
-__global__ void __launch_bounds__(kTreeThreads) select_tree(const __grid_constant__ TreeArgs A) {
+__global__ void __launch_bounds__(kTreeThreads, kTreeBlocks) select_tree(const __grid_constant__ TreeArgs A) {
   __shared__ int sm[kTreeWarps], off_s[kTreeLevels + 1], s_base[kTreeThreads];
   __shared__ uint32_t s_word[kTreeThreads];
   __shared__ unsigned long long s_key[kReqChunk];
@@ -401,9 +423,27 @@ __global__ void __launch_bounds__(kTreeThreads) select_tree(const __grid_constan
   int tab = 0, dirty[2] = {0, 0};
   for (int ln = maxlev; ln > 1 && !stop; --ln) {
     const int td_a = off_s[ln - 1], ntd = off_s[ln] - td_a, nbal = n_open - n_open_td;
-    for (int q = gt; q < 8 * (ntd + nbal); q += gthreads) {
+    // the nodes opened by the balance are of all levels: as many as one round holds are taken as
+    // they come; beyond it a warp picks those of level ln - 1 among its share, up to 32 of them,
+    // and its lanes take four of these at a time (6.6 -> 4.1 ms for 2,000 groups in empty space)
+    const bool pick = 8ll * nbal > gthreads;
+    const int share_bal = min(32, (nbal + gwarps - 1) / gwarps);
+    for (int q = gt; q < 8 * (pick ? ntd : ntd + nbal); q += gthreads) {
       const int r = q >> 3;
       request_openings(A, ln, r < ntd ? td_a + r : n_open_td + (r - ntd), q & 7, tab);
+    }
+    for (int o0 = share_bal * gwarp; o0 < nbal && pick; o0 += share_bal * gwarps) {
+      const bool of_level = lane < share_bal && o0 + lane < nbal && code_level(A.op_code[n_open_td + o0 + lane]) == ln - 1;
+      for (unsigned todo = __ballot_sync(0xffffffffu, of_level); todo;) {
+        unsigned rest = todo;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (k < (lane >> 3)) rest &= rest - 1u;
+          todo &= todo - 1u;
+        }
+        if (rest) request_openings(A, ln, n_open_td + o0 + __ffs(rest) - 1, lane & 7, tab);
+        __syncwarp();
+      }
     }
     if (!grid_sync(A.bar, G, epoch, A.err)) return;
     const int nreq = __ldcg(A.nreq + ln);
@@ -446,11 +486,12 @@ __global__ void __launch_bounds__(kTreeThreads) select_tree(const __grid_constan
       unsigned long long *sorted = reinterpret_cast<unsigned long long *>(A.crange);  // not used past the levels
       for (int c0 = b * kReqChunk; c0 < nreq; c0 += G * kReqChunk) sort_requests(list, vals, nreq, c0, s_key, sorted);
       if (!grid_sync(A.bar, G, epoch, A.err)) return;
-      for (int i0 = b * kTreeThreads; i0 < nreq; i0 += gthreads) {
-        const int i = i0 + t;
-        const unsigned long long key = i < nreq ? __ldcg(sorted + i) : 0ull;
-        const int rank = rank_requests(sorted, nreq, key, s_key);
-        if (i < nreq) open_request(rank, requested_cell(A, ln, key));
+      for (long long i0 = b * kTreeThreads; i0 < nreq; i0 += (long long)kReqKeys * gthreads) {
+        unsigned long long key[kReqKeys];
+        int rank[kReqKeys];
+        rank_requests(sorted, nreq, (int)i0, gthreads, s_key, key, rank);
+        for (int q = 0; q < kReqKeys; ++q)
+          if (i0 + t + (long long)q * gthreads < nreq) open_request(rank[q], requested_cell(A, ln, key[q]));
       }
     }
     n_open += nreq;
@@ -707,8 +748,15 @@ static int select_once(apc_context *c, int *hash_full) {
   }
   APC_CUDA_TRY(c, cudaMemsetAsync(c->tree_out, 0, sizeof(TreeOut) + sizeof(GridBar) + kTreeLevels * sizeof(int), c->s));
   APC_CUDA_TRY(c, cudaMemsetAsync(c->h_keys, 0, sizeof(uint64_t) * c->hcap, c->s));
-  // a block for every 2048 particles (about as many children of opened nodes as threads)
-  const int blocks = std::max(1, std::min(apc_sm_count(c), n / 2048));
+  // a block for every 2048 particles (about as many children of opened nodes as threads), or for
+  // every 256 nodes that the last selection or attempt opened: groups in empty space open more
+  // nodes than they have particles (2,000 groups of 64: 4.1 ms by particles, 3.3 ms by nodes).
+  // Two blocks per SM where the probes miss L2 anyway: at 2.5M nodes 16.8 and 15.7 ms, at 0.3M
+  // 3.3 and 3.5.
+  const int sms = apc_sm_count(c);
+  const int blocks = c->open_hint > kTreeTwo
+                         ? kTreeBlocks * sms
+                         : std::max(1, std::min(sms, std::max(n / 2048, c->open_hint / 256)));
   void *args[] = {&A};
   APC_CUDA_TRY(c, cudaLaunchCooperativeKernel((const void *)select_tree, dim3(blocks), dim3(kTreeThreads), args, 0,
                                               c->s));
@@ -734,6 +782,7 @@ static int select_once(apc_context *c, int *hash_full) {
     c->err = "selection kernel grid barrier timed out";
     return APC_ERR_TIMEOUT;
   }
+  c->open_hint = T.n_open;
   if (T.stop & TREE_DEEPER) return APC_RETRY_FULL_SORT;
   if ((T.stop & TREE_FULL) || (derr & DERR_HASH_FULL)) {
     *hash_full = 1;
