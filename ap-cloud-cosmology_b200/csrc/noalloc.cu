@@ -60,7 +60,7 @@ static_assert(sizeof(NoallocScratch) <= kNoallocScratchBytes, "fits the scratch 
 // kick, LANES lanes per cell, so that no particle -> cell map is written, checked and read
 // back.  The last phase is bound by memory: 96 B per particle beside its cell's row.
 // 1,000,003 particles in 111,111 cells: two memsets and three kernels took 52 us on the device,
-// this kernel 33 us (25 us of it the kick); a call from Python 99 -> 88 us.
+// this kernel 33 us (25 us of it the kick); a call from Python 99 -> 86 us.
 template <int LANES>
 __global__ void __launch_bounds__(kNoThreads) noalloc_kick(int n, int m, const int *__restrict__ first,
                                                            const int *__restrict__ count,
