@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <cstddef>
 #include <cstring>
 #include <mutex>
 
@@ -34,13 +35,15 @@ std::mutex g_call_mutex[kMaxDevices];  // held for a whole call: the scratch is 
 // a call; but a call that broke off spoilt the next, threads read each other's results, and the
 // pinned words had to be allocated.)
 constexpr int kNoThreads = 512;
-constexpr int kNoBig = 2048;  // particles from which a cell is spread over the whole grid
+constexpr int kNoBig = 256;   // particles from which a cell is spread over the whole grid
+constexpr int kNoUnit = 128;  // in pieces of this many, a warp each
 constexpr int kNoWords = APC_NOALLOC_MAX_PARTICLES / 32;
 constexpr int kNoBigMax = APC_NOALLOC_MAX_PARTICLES / kNoBig;
 struct NoallocAcc {
   unsigned long long maxbits;  // IEEE bits of max |a|^2 c_vel^2 dt^2
   unsigned long long total;    // particles in all ranges
-  int bad;                     // ranges outside [0, n), or overlapping
+  int covered;                 // bits set
+  int bad;                     // ranges outside [0, n)
   int err;                     // a grid barrier gave up
   int outcome;                 // of the second barrier, the same for every block: kKick or kLeave
   int nbig;
@@ -48,19 +51,20 @@ struct NoallocAcc {
 };
 enum { kKick = 1, kLeave = 2 };
 struct NoallocScratch {
+  NoallocAcc acc;           // cleared before each launch, with the words of the bits that it uses
   unsigned bits[kNoWords];
-  int big[kNoBigMax];
-  NoallocAcc acc;
+  int4 big[kNoBigMax];      // a cell of many particles: its index, first and count
 };
 static_assert(sizeof(NoallocScratch) <= kNoallocScratchBytes, "fits the scratch array");
 
-// The whole call in one cooperative launch, its phases a grid barrier apart: clear the bits,
-// mark every range's particles (a bit already set is an overlap; ranges without overlaps
-// that hold n particles in all cover every particle), and - when all is well - interpolate and
-// kick, LANES lanes per cell, so that no particle -> cell map is written, checked and read
-// back.  The last phase is bound by memory: 96 B per particle beside its cell's row.
-// 1,000,003 particles in 111,111 cells: two memsets and three kernels took 52 us on the device,
-// this kernel 33 us (25 us of it the kick); a call from Python 99 -> 86 us.
+// The whole call in one cooperative launch, its phases a grid barrier apart: mark every range's
+// particles in the bits and add up the ranges; count the bits (ranges that hold n particles in
+// all and cover n of them cover each once); and - when all is well - interpolate and kick, LANES
+// lanes per cell and a warp per piece of a cell of many, so that no particle -> cell map is
+// written, checked and read back.  The marks return nothing, so nobody waits for them.  The last
+// phase is bound by memory: 96 B per particle beside its cell's row.  A call for 1,000,000
+// particles from the host, in us, by the particles of a cell, as two memsets and three kernels
+// and now: 9: 60, 57; 20: 51, 57; 50: 51, 52; 200: 51, 57; 2,500: 78, 57; 50,000: 607, 57.
 template <int LANES>
 __global__ void __launch_bounds__(kNoThreads) noalloc_kick(int n, int m, const int *__restrict__ first,
                                                            const int *__restrict__ count,
@@ -76,19 +80,19 @@ __global__ void __launch_bounds__(kNoThreads) noalloc_kick(int n, int m, const i
                                                            double *__restrict__ az, double cv, double dt,
                                                            NoallocScratch *S, long long limit0) {
   __shared__ double sm[kNoThreads / 32];
-  __shared__ int s_outcome;
+  __shared__ int s_outcome, s_scan[kNoThreads / 32], s_piece[kNoBigMax];
   NoallocAcc *acc = &S->acc;
   const int t = threadIdx.x, lane = t & 31;
   const int threads = gridDim.x * kNoThreads, g0 = blockIdx.x * kNoThreads + t;
   unsigned epoch = 0;
-  for (int w = g0; w < (n + 31) / 32; w += threads) S->bits[w] = 0u;
-  if (!grid_sync(&acc->bar, gridDim.x, epoch, &acc->err)) return;
-  // ---- the ranges: a thread per cell; a cell of many words by its whole warp ----
+  // ---- the ranges: a lane for about every word of a cell; a cell of many by its whole warp ----
   {
+    constexpr int kMark = LANES > 8 ? LANES / 8 : 1;
+    const int sub = g0 % kMark;
+    const unsigned cells = (unsigned)threads / kMark, rounds = ((unsigned)m + cells - 1u) / cells;
     unsigned long long mine = 0;
-    const unsigned rounds = ((unsigned)m + (unsigned)threads - 1u) / (unsigned)threads;
     for (unsigned r = 0; r < rounds; ++r) {  // the same count for every lane (ballots)
-      const unsigned i = r * (unsigned)threads + (unsigned)g0;  // past m, a multiple of the grid: no int
+      const unsigned i = r * cells + (unsigned)(g0 / kMark);  // past m, a multiple of the grid: no int
       long long f = 0, c = 0;
       if (i < (unsigned)m) {
         f = first[i];
@@ -97,21 +101,21 @@ __global__ void __launch_bounds__(kNoThreads) noalloc_kick(int n, int m, const i
           atomicOr(&acc->bad, 1);
           c = 0;
         }
-        if (c >= kNoBig) {  // more than kNoBigMax of them overlap
+        if (c >= kNoBig && sub == 0) {  // more than kNoBigMax of them overlap
           const int q = atomicAdd(&acc->nbig, 1);
-          if (q < kNoBigMax) S->big[q] = (int)i;
+          if (q < kNoBigMax) S->big[q] = make_int4((int)i, (int)f, (int)c, 0);
         }
       }
-      mine += (unsigned long long)c;
+      if (sub == 0) mine += (unsigned long long)c;
       auto mark = [&](long long lo, long long hi, int w) {  // bits [lo, hi) of word w
         const int a = (int)max(lo - 32ll * w, 0ll), b = (int)min(hi - 32ll * w, 32ll);
         const unsigned mask = (b == 32 ? ~0u : (1u << b) - 1u) & ~((1u << a) - 1u);
-        if (atomicOr(&S->bits[w], mask) & mask) atomicOr(&acc->bad, 1);
+        atomicOr(&S->bits[w], mask);
       };
-      const bool wide = c > 256;
+      const bool wide = c >= kNoBig;
       if (c > 0 && !wide)
-        for (int w = (int)(f >> 5); w <= (int)((f + c - 1) >> 5); ++w) mark(f, f + c, w);
-      for (unsigned todo = __ballot_sync(0xffffffffu, wide); todo; todo &= todo - 1) {
+        for (int w = (int)(f >> 5) + sub; w <= (int)((f + c - 1) >> 5); w += kMark) mark(f, f + c, w);
+      for (unsigned todo = __ballot_sync(0xffffffffu, wide && sub == 0); todo; todo &= todo - 1) {
         const int src = __ffs(todo) - 1;
         const long long bf = __shfl_sync(0xffffffffu, f, src), bc = __shfl_sync(0xffffffffu, c, src);
         for (int w = (int)(bf >> 5) + lane; w <= (int)((bf + bc - 1) >> 5); w += 32) mark(bf, bf + bc, w);
@@ -120,6 +124,13 @@ __global__ void __launch_bounds__(kNoThreads) noalloc_kick(int n, int m, const i
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
     if (lane == 0 && mine) atomicAdd(&acc->total, mine);
+  }
+  if (!grid_sync(&acc->bar, gridDim.x, epoch, &acc->err)) return;
+  {
+    int mine = 0;
+    for (int w = g0; w < (n + 31) / 32; w += threads) mine += __popc(__ldcg(&S->bits[w]));
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if (lane == 0 && mine) atomicAdd(&acc->covered, mine);
   }
   // A block whose wait runs out here leaves, and another may still find every block arrived.  All
   // take the first claim, so that a call that gives up has written nothing.
@@ -131,8 +142,8 @@ __global__ void __launch_bounds__(kNoThreads) noalloc_kick(int n, int m, const i
   __syncthreads();
   if (s_outcome != kKick) return;
   // malformed cell ranges leave every output untouched
-  const bool ok =
-      *(volatile int *)&acc->bad == 0 && *(volatile unsigned long long *)&acc->total == (unsigned long long)n;
+  const bool ok = *(volatile int *)&acc->bad == 0 && *(volatile int *)&acc->covered == n &&
+                  *(volatile unsigned long long *)&acc->total == (unsigned long long)n;
   // ---- same arithmetic, operand order and rounding as the kick of apc_move_velocity ----
   double mx = 0.0;
   auto kick_cell = [&](int i, int s0, int s1, int step) {  // particles s0, s0 + step, ... < s1 of cell i
@@ -161,10 +172,32 @@ __global__ void __launch_bounds__(kNoThreads) noalloc_kick(int n, int m, const i
     // nothing is formed from an empty cell's first: it may be any value
     if (c > 0 && c < kNoBig) kick_cell((int)i, f + g0 % LANES, f + c, LANES);
   }
+  // the cells of many particles, piece by piece: every block numbers the pieces of all of them,
+  // and a warp finds the cell of its piece.  (Cell after cell, each over the whole grid, took
+  // 606 us for 1,000,000 particles in 400 cells, 57 now.)
   const int nbig = ok ? min(*(volatile int *)&acc->nbig, kNoBigMax) : 0;
-  for (int q = 0; q < nbig; ++q) {
-    const int i = S->big[q], f = first[i];
-    kick_cell(i, f + g0, f + count[i], threads);
+  if (nbig > 0) {
+    constexpr int kEach = kNoBigMax / kNoThreads;
+    int mine[kEach], sum = 0, total;
+#pragma unroll
+    for (int k = 0; k < kEach; ++k) {
+      const int q = t * kEach + k;
+      mine[k] = sum;
+      if (q < nbig) sum += (__ldcg(&S->big[q]).z + kNoUnit - 1) / kNoUnit;
+    }
+    const int before = block_scan_int<kNoThreads>(sum, s_scan, &total);
+#pragma unroll
+    for (int k = 0; k < kEach; ++k) s_piece[t * kEach + k] = before + mine[k];
+    __syncthreads();
+    for (int u = g0 >> 5; u < total; u += threads >> 5) {
+      int q = 0;  // the last cell whose pieces begin at or before u
+#pragma unroll
+      for (int step = kNoBigMax / 2; step > 0; step >>= 1)
+        if (q + step < nbig && s_piece[q + step] <= u) q += step;
+      const int4 cell = __ldcg(&S->big[q]);
+      const int at = cell.y + (u - s_piece[q]) * kNoUnit;
+      kick_cell(cell.x, at + lane, min(at + kNoUnit, cell.y + cell.z), 32);
+    }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
@@ -219,28 +252,40 @@ static int noalloc_call(int n_particles, int n_cells, const int *first, const in
   if (rc != APC_OK) return rc;
   cudaStream_t s = (cudaStream_t)stream;
   NoallocScratch *S = (NoallocScratch *)base;
-  // lanes per cell: half the mean count or more, so that most cells take one or two rounds
+  // lanes per cell: half the mean count or more, so that most cells take one or two rounds and
+  // a last wave of blocks that is nearly empty stays short
   const double mean = (double)n_particles / n_cells;
-  const void *kern = mean <= 8 ? (const void *)noalloc_kick<4>
-                               : (mean <= 16 ? (const void *)noalloc_kick<8>
-                                             : (mean <= 32 ? (const void *)noalloc_kick<16>
-                                                           : (const void *)noalloc_kick<32>));
-  const int lanes = mean <= 8 ? 4 : (mean <= 16 ? 8 : (mean <= 32 ? 16 : 32));
-  // as many blocks as are resident together (the phases are grid barriers), no more than the
-  // cells' lane groups or the particles need
-  int sms = 1, occ = 0;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kNoThreads, 0) != cudaSuccess || occ < 1) {
-    cudaGetLastError();
-    return APC_ERR_CUDA;
+  const struct {
+    double mean;
+    int lanes;
+    const void *kern;
+  } forms[] = {{8, 4, (const void *)noalloc_kick<4>},     {16, 8, (const void *)noalloc_kick<8>},
+               {32, 16, (const void *)noalloc_kick<16>},  {64, 32, (const void *)noalloc_kick<32>},
+               {1e300, 64, (const void *)noalloc_kick<64>}};
+  int form = 0;
+  while (mean > forms[form].mean) ++form;
+  const int lanes = forms[form].lanes;
+  const void *kern = forms[form].kern;
+  std::lock_guard<std::mutex> lock(g_call_mutex[dev]);
+  // as many blocks as are resident together (the phases are grid barriers; asked once per device
+  // and form), no more than the cells' lane groups or the particles need
+  static int resident[kMaxDevices][sizeof(forms) / sizeof(forms[0])] = {};
+  if (resident[dev][form] == 0) {
+    int sms = 0, occ = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kNoThreads, 0) != cudaSuccess || occ < 1) {
+      cudaGetLastError();
+      return APC_ERR_CUDA;
+    }
+    resident[dev][form] = sms * occ;
   }
   const long long want = (std::max((long long)n_particles, (long long)n_cells * lanes) + kNoThreads - 1) / kNoThreads;
-  const int blocks = (int)std::max(1ll, std::min(want, (long long)sms * occ));
+  const int blocks = (int)std::max(1ll, std::min(want, (long long)resident[dev][form]));
   void *args[] = {&n_particles, &n_cells, &first, &count, &deriv9, &cx, &cy, &cz, &x, &y, &z, &vx, &vy, &vz,
                   &ax, &ay, &az, &c_vel, &dt, &S, &limit0};
   NoallocAcc got;
-  std::lock_guard<std::mutex> lock(g_call_mutex[dev]);
-  if (cudaMemsetAsync(&S->acc, 0, sizeof(NoallocAcc), s) != cudaSuccess ||
+  const size_t clear = offsetof(NoallocScratch, bits) + sizeof(unsigned) * (size_t)((n_particles + 31) / 32);
+  if (cudaMemsetAsync(S, 0, clear, s) != cudaSuccess ||
       cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(kNoThreads), args, 0, s) != cudaSuccess ||
       cudaMemcpyAsync(&got, &S->acc, sizeof(got), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess) {
@@ -250,7 +295,7 @@ static int noalloc_call(int n_particles, int n_cells, const int *first, const in
   if (got.outcome != kKick) return APC_ERR_TIMEOUT;  // a grid barrier gave up: nothing was written
   // cell ranges outside [0, n), overlapping, or leaving a particle uncovered: caller input,
   // so an invalid argument (the context path builds its ranges itself); nothing was written
-  if (got.bad || got.total != (unsigned long long)n_particles) return APC_ERR_INVALID_ARG;
+  if (got.bad || got.covered != n_particles || got.total != (unsigned long long)n_particles) return APC_ERR_INVALID_ARG;
   if (max_dv) {
     double v;
     std::memcpy(&v, &got.maxbits, sizeof(v));
