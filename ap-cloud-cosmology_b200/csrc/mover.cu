@@ -17,30 +17,48 @@
 
 namespace {
 
-// each cell writes its particle range: a warp takes 32 cells (their ranges in one coalesced
-// load), 8 lanes a cell; cells of more than 64 particles follow, the whole warp on each.
-// (One warp per cell spent a dependent load per ~8 particles: 31 us at 128^3.)
-__global__ void cell_of_particles(int m, const int *__restrict__ first, const int *__restrict__ count,
-                                  int *__restrict__ cell_of) {
-  const int lane = threadIdx.x & 31, sub = lane & 7;
-  const int wpb = blockDim.x >> 5, nb = (m + 31) / 32;
-  for (int b = blockIdx.x * wpb + (threadIdx.x >> 5); b < nb; b += gridDim.x * wpb) {
-    const int i = b * 32 + lane;
-    const int f = i < m ? first[i] : 0, c = i < m ? count[i] : 0;
+// each cell writes its particle range: a warp takes `per` cells (their ranges in one coalesced
+// load), 8 lanes a cell; cells of more than 64 particles follow, the whole warp on each, and of
+// more than 1024 the block.
+// One cell per warp spent a dependent load per ~8 particles (31 us at 128^3), 32 cells with many
+// particles left most SMs idle, so per follows the mean count, about 256 particles a warp: kick
+// and drift of 2.1M particles in 512 cells 191 us with 32, 118 with one; in 32,768 cells with
+// nearly all particles in a few of them 369 us with 32, 309 with 4 without the block, 248
+// with it.
+constexpr int kMapWarps = 8, kMapBlock = 1024;
+__global__ void __launch_bounds__(32 * kMapWarps) cell_of_particles(int m, int per, const int *__restrict__ first,
+                                                                    const int *__restrict__ count,
+                                                                    int *__restrict__ cell_of) {
+  __shared__ int s_cell[32 * kMapWarps], s_n;
+  const int lane = threadIdx.x & 31, sub = lane & 7, w = threadIdx.x >> 5;
+  const int nb = (m + per - 1) / per;
+  for (int b0 = blockIdx.x * kMapWarps; b0 < nb; b0 += gridDim.x * kMapWarps) {
+    if (threadIdx.x == 0) s_n = 0;
+    __syncthreads();
+    const int i = (b0 + w) * per + lane;
+    const bool in = lane < per && i < m;
+    const int f = in ? first[i] : 0, c = in ? count[i] : 0;
 #pragma unroll
     for (int q = 0; q < 32; q += 4) {
       const int src = q + (lane >> 3);
       const int fq = __shfl_sync(0xffffffffu, f, src), cq = __shfl_sync(0xffffffffu, c, src);
       if (cq <= 64)
-        for (int k = sub; k < cq; k += 8) cell_of[fq + k] = b * 32 + src;
+        for (int k = sub; k < cq; k += 8) cell_of[fq + k] = i - lane + src;
     }
-    unsigned big = __ballot_sync(0xffffffffu, c > 64);
+    if (c > kMapBlock) s_cell[atomicAdd(&s_n, 1)] = i;
+    unsigned big = __ballot_sync(0xffffffffu, c > 64 && c <= kMapBlock);
     while (big) {
       const int src = __ffs(big) - 1;
       big &= big - 1;
       const int fq = __shfl_sync(0xffffffffu, f, src), cq = __shfl_sync(0xffffffffu, c, src);
-      for (int k = lane; k < cq; k += 32) cell_of[fq + k] = b * 32 + src;
+      for (int k = lane; k < cq; k += 32) cell_of[fq + k] = i - lane + src;
     }
+    __syncthreads();
+    for (int q = 0, n = s_n; q < n; ++q) {
+      const int cell = s_cell[q], fq = first[cell], cq = count[cell];
+      for (int k = threadIdx.x; k < cq; k += 32 * kMapWarps) cell_of[fq + k] = cell;
+    }
+    __syncthreads();
   }
 }
 
@@ -195,6 +213,15 @@ __global__ void max_cell_density(int m, const int *__restrict__ count, const dou
   if (threadIdx.x == 0) atomic_max_nonneg(maxbits, mx);
 }
 
+// cell_of for the context's m cells
+void map_particles(apc_context *c, int m, int sms) {
+  int per = 32;
+  while (per > 1 && (long long)c->n * per > 256ll * m) per >>= 1;
+  const int cells = kMapWarps * per;  // of a block
+  cell_of_particles<<<std::max(1, std::min((m + cells - 1) / cells, sms * 16)), 32 * kMapWarps, 0, c->s>>>(
+      m, per, c->cfirst, c->ccount, c->cell_of);
+}
+
 }  // namespace
 
 int apc_mover_max_density(apc_context *c, double *out) {
@@ -219,8 +246,7 @@ int apc_mover_velocity(apc_context *c, double dt, double c_vel, double *max_dv) 
   APC_CUDA_TRY(c, cudaMemsetAsync(c->cell_of, 0xff, sizeof(int) * (size_t)n, c->s));
   APC_CUDA_TRY(c, cudaMemsetAsync(c->d_err, 0, sizeof(int), c->s));
   const int sms = apc_sm_count(c);
-  cell_of_particles<<<std::max(1, std::min((M + 255) / 256, sms * 16)), 256, 0, c->s>>>(M, c->cfirst, c->ccount,
-                                                                                   c->cell_of);
+  map_particles(c, M, sms);
   unsigned long long *mb = (unsigned long long *)(c->counters + 96);
   APC_CUDA_TRY(c, cudaMemsetAsync(mb, 0, sizeof(unsigned long long), c->s));
   const int G = std::max(1, std::min((n + 255) / 256, sms * 8));
@@ -276,8 +302,7 @@ int apc_mover_kick_drift(apc_context *c, double dt, double c_vel, double c_pos, 
   APC_CUDA_TRY(c, cudaMemsetAsync(c->cell_of, 0xff, sizeof(int) * (size_t)n, c->s));
   APC_CUDA_TRY(c, cudaMemsetAsync(c->d_err, 0, sizeof(int), c->s));
   const int sms = apc_sm_count(c);
-  cell_of_particles<<<std::max(1, std::min((M + 255) / 256, sms * 16)), 256, 0, c->s>>>(M, c->cfirst, c->ccount,
-                                                                                   c->cell_of);
+  map_particles(c, M, sms);
   // counters + 96 .. + 99: the two maxima (8 bytes each)
   unsigned long long *mb = (unsigned long long *)(c->counters + 96);
   APC_CUDA_TRY(c, cudaMemsetAsync(mb, 0, 2 * sizeof(unsigned long long), c->s));
