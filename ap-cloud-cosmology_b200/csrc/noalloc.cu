@@ -138,6 +138,7 @@ __global__ void __launch_bounds__(kNoThreads) noalloc_kick(int n, int m, const i
   if (t == 0) {
     const int mine = met ? kKick : kLeave, first_claim = atomicCAS(&acc->outcome, 0, mine);
     s_outcome = first_claim != 0 ? first_claim : mine;
+    if (!met) __threadfence();  // the claim of a block that did see all arrive: its view, in place of the barrier's
   }
   __syncthreads();
   if (s_outcome != kKick) return;
